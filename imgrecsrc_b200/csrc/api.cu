@@ -146,26 +146,10 @@ void fill_det_table(const Geo &g, DetEntry *de)
     }
 }
 
-template <class T>
-static int upload(T **dst, const std::vector<T> &src)
-{
-    int st = cuda_error(cudaMalloc((void **)dst, sizeof(T) * (src.empty() ? 1 : src.size())),
-                        "table allocation");
-    if (st) return st;
-    if (!src.empty())
-        st = cuda_error(cudaMemcpy(*dst, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice),
-                        "table upload");
-    return st;
-}
-
 static void free_plan(ctprj_plan *p)
 {
     if (!p) return;
-    cudaFree(p->d_fview);
-    cudaFree(p->d_bview);
-    cudaFree(p->d_det);
-    cudaFree(p->d_quad);
-    cudaFree(p->d_count);
+    cudaFree(p->d_arena);
     cudaFree(p->d_ramp);
     cudaFree(p->d_fsino);
     cudaFree(p->d_mimg);
@@ -236,26 +220,57 @@ static int build_plan(const ctprj_geometry *geom, int device, ctprj_plan **out)
 
     DeviceGuard dg(device);
     if ((st = dg.status)) { delete p; return st; }
-    if ((st = upload(&p->d_fview, fv)) || (st = upload(&p->d_bview, bv)) ||
-        (st = upload(&p->d_det, de)) ||
-        (st = cuda_error(cudaMalloc((void **)&p->d_quad, sizeof(float4) * quad_elems(g.n)),
-                         "scratch allocation")) ||
-        (st = cuda_error(cudaMalloc((void **)&p->d_count, sizeof(unsigned long long)),
-                         "counter allocation"))) {
-        free_plan(p);
-        return st;
+    // One allocation and one upload for the plan: the host-built tables and the
+    // counter, then the quad image and the staged backprojection's tables (an
+    // allocation of its own for each took most of a plan's creation).
+    struct Part {
+        size_t at, bytes;
+    };
+    size_t total = 0;
+    auto part = [&](size_t bytes) {
+        const Part r = {total, bytes};
+        total += (bytes + 255) / 256 * 256;
+        return r;
+    };
+    const Part pf = part(sizeof(FwdView) * fv.size()), pb = part(sizeof(BwdView) * bv.size()),
+               pd = part(sizeof(DetEntry) * de.size()), pc = part(sizeof(unsigned long long));
+    const size_t uploaded = total;
+    const Part pq = part(sizeof(float4) * quad_elems(g.n));
+    const size_t without = total;
+    const Part pt = part(backward_table_bytes(g));
+    std::vector<char> host(uploaded, 0);
+    memcpy(&host[pf.at], fv.data(), pf.bytes);
+    memcpy(&host[pb.at], bv.data(), pb.bytes);
+    memcpy(&host[pd.at], de.data(), pd.bytes);
+    bool tables = true;
+    if (cudaMalloc((void **)&p->d_arena, total) != cudaSuccess) {
+        // no room for the tables: the unstaged backprojection needs none
+        cudaGetLastError();
+        p->d_arena = nullptr;
+        tables = false;
+        if ((st = cuda_error(cudaMalloc((void **)&p->d_arena, without), "plan allocation"))) {
+            free_plan(p);
+            return st;
+        }
     }
+    p->d_fview = (FwdView *)(p->d_arena + pf.at);
+    p->d_bview = (BwdView *)(p->d_arena + pb.at);
+    p->d_det = (DetEntry *)(p->d_arena + pd.at);
+    p->d_count = (unsigned long long *)(p->d_arena + pc.at);
+    p->d_quad = (float4 *)(p->d_arena + pq.at);
     // backprojection kernel: staged tiles sized to the widest tile shadow of
     // this geometry, or the unstaged kernel when a shadow exceeds 64 detectors
     // or CTPRJ_BWD_KERNEL=direct asks for it (kept for comparison)
+    const char *bk = getenv("CTPRJ_BWD_KERNEL");
+    if (bk && strcmp(bk, "direct") == 0) tables = false;
     int span = 0;
-    if ((st = backward_max_span(p, &span))) {
+    if ((st = cuda_error(cudaMemcpy(p->d_arena, host.data(), uploaded, cudaMemcpyHostToDevice), "table upload")) ||
+        (tables && ((st = backward_tables(p, (float4 *)(p->d_arena + pt.at))) || (st = backward_max_span(p, &span))))) {
         free_plan(p);
         return st;
     }
-    const char *bk = getenv("CTPRJ_BWD_KERNEL");
-    p->bwd_seg = span <= 32 ? 32 : (span <= 64 ? 64 : 0);
-    if (bk && strcmp(bk, "direct") == 0) p->bwd_seg = 0;
+    p->bwd_seg = !tables ? 0 : (span <= 32 ? 32 : (span <= 64 ? 64 : 0));
+    p->bwd_split = backward_split(p);
     *out = p;
     return CTPRJ_OK;
 }

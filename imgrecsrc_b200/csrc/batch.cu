@@ -8,8 +8,8 @@
 // own ctprj_forward / ctprj_backward: the block bodies are the same.
 //
 // The tuner times the candidate launch shapes on the bound buffers -- forward
-// block of 2, 4 or 8 views x 32 rays, backprojection batches of 8 or 16 views
-// per staged tile, full or half residency, slices handed out largest first or
+// block of 2, 4 or 8 views x 32 rays, backprojection staging buffers of 8 or 16
+// views in all, full or half residency, slices handed out largest first or
 // in order -- and keeps the fastest; results are cached in a text file keyed by
 // the device and the batch's geometries.
 #include <algorithm>
@@ -28,7 +28,7 @@ struct BatchConfig {
     int fwd_views = 4;     // 2, 4, 8
     int fwd_occ = 1;       // 1 full residency, 2 half
     int fwd_order = 1;     // 1 largest slice first, 0 as given
-    int bwd_vb = 8;        // views per staged batch (16 only with 32-detector staging)
+    int bwd_vb = 16;       // views in a tile's two staging buffers (16 only with 32-detector staging)
     int bwd_occ = 1;
     int bwd_order = 1;
 };
@@ -42,9 +42,10 @@ struct ctprj_batch {
     BatchSlice *d_slices = nullptr;
     int *d_order_f = nullptr, *d_order_b = nullptr;
     long long *d_fprefix = nullptr, *d_bprefix = nullptr, *d_tprefix = nullptr;
+    long long *d_sprefix = nullptr, *d_oprefix = nullptr;   // sample rows, natural and in backward order
     unsigned long long *d_counter = nullptr;   // [0] forward, [1] backward
-    int *d_status = nullptr;                   // streaming: per slice, 1 = timed out
-    long long ftotal = 0, btotal = 0, ttotal = 0;
+    int *d_status = nullptr;                   // streaming: per slice, 1 = timed out; then sample rows done
+    long long ftotal = 0, btotal = 0, ttotal = 0, stotal = 0;
     int seg = 0;                  // staging capacity used by the batched backprojection
     int bound = 0;                // buffers bound
     BatchConfig cfg;
@@ -78,6 +79,9 @@ long long bwd_items(const ctprj_plan *p)
     return (long long)T * (T + 1) / 2;
 }
 
+// rows of a slice's sample image (none: unstaged)
+long long samp_rows(const ctprj_batch *b, int i) { return b->hs[i].tiled ? b->geoms[i].prjFull / 4 : 0; }
+
 // slice work estimate for ordering: updates ~ n^2 * views
 double slice_cost(const ctprj_geometry &g) { return (double)g.n * g.n * g.np; }
 
@@ -100,20 +104,25 @@ int upload_lists(ctprj_batch *b)
     auto bigger = [&](int a, int c) { return slice_cost(b->geoms[a]) > slice_cost(b->geoms[c]); };
     if (b->cfg.fwd_order) std::stable_sort(of.begin(), of.end(), bigger);
     if (b->cfg.bwd_order) std::stable_sort(ob.begin(), ob.end(), bigger);
-    std::vector<long long> fp(n + 1, 0), bp(n + 1, 0), tp(n + 1, 0);
+    std::vector<long long> fp(n + 1, 0), bp(n + 1, 0), tp(n + 1, 0), sp(n + 1, 0), op(n + 1, 0);
     for (int i = 0; i < n; ++i) {
         fp[i + 1] = fp[i] + fwd_items(b->plans[of[i]], b->cfg.fwd_views);
         bp[i + 1] = bp[i] + bwd_items(b->plans[ob[i]]);
         tp[i + 1] = tp[i] + quad_tiles(b->geoms[i].n);
+        sp[i + 1] = sp[i] + samp_rows(b, i);
+        op[i + 1] = op[i] + samp_rows(b, ob[i]);
     }
     b->ftotal = fp[n];
     b->btotal = bp[n];
     b->ttotal = tp[n];
+    b->stotal = sp[n];
     int st;
     if ((st = cuda_error(cudaMemcpy(b->d_order_f, of.data(), sizeof(int) * n, cudaMemcpyHostToDevice), "batch lists")) ||
         (st = cuda_error(cudaMemcpy(b->d_order_b, ob.data(), sizeof(int) * n, cudaMemcpyHostToDevice), "batch lists")) ||
         (st = cuda_error(cudaMemcpy(b->d_fprefix, fp.data(), sizeof(long long) * (n + 1), cudaMemcpyHostToDevice), "batch lists")) ||
         (st = cuda_error(cudaMemcpy(b->d_bprefix, bp.data(), sizeof(long long) * (n + 1), cudaMemcpyHostToDevice), "batch lists")) ||
+        (st = cuda_error(cudaMemcpy(b->d_sprefix, sp.data(), sizeof(long long) * (n + 1), cudaMemcpyHostToDevice), "batch lists")) ||
+        (st = cuda_error(cudaMemcpy(b->d_oprefix, op.data(), sizeof(long long) * (n + 1), cudaMemcpyHostToDevice), "batch lists")) ||
         (st = cuda_error(cudaMemcpy(b->d_tprefix, tp.data(), sizeof(long long) * (n + 1), cudaMemcpyHostToDevice), "batch lists")))
         return st;
     free_graphs(b);
@@ -130,6 +139,9 @@ BatchArgs fwd_args(const ctprj_batch *b)
     a.total = b->ftotal;
     a.tprefix = b->d_tprefix;
     a.ttotal = b->ttotal;
+    a.sprefix = b->d_sprefix;
+    a.stotal = b->stotal;
+    a.oprefix = b->d_oprefix;
     a.counter = b->d_counter;
     return a;
 }
@@ -231,8 +243,10 @@ extern "C" int ctprj_batch_create(const ctprj_geometry *geoms, int nslices, int 
             !(st = cuda_error(cudaMalloc((void **)&b->d_fprefix, sizeof(long long) * (n + 1)), "batch tables")) &&
             !(st = cuda_error(cudaMalloc((void **)&b->d_bprefix, sizeof(long long) * (n + 1)), "batch tables")) &&
             !(st = cuda_error(cudaMalloc((void **)&b->d_tprefix, sizeof(long long) * (n + 1)), "batch tables")) &&
+            !(st = cuda_error(cudaMalloc((void **)&b->d_sprefix, sizeof(long long) * (n + 1)), "batch tables")) &&
+            !(st = cuda_error(cudaMalloc((void **)&b->d_oprefix, sizeof(long long) * (n + 1)), "batch tables")) &&
             !(st = cuda_error(cudaMalloc((void **)&b->d_counter, 2 * sizeof(unsigned long long)), "batch tables")) &&
-            !(st = cuda_error(cudaMalloc((void **)&b->d_status, sizeof(int) * n), "batch tables")))
+            !(st = cuda_error(cudaMalloc((void **)&b->d_status, 2 * sizeof(int) * n), "batch tables")))
             st = upload_lists(b);
     }
     if (st) {
@@ -255,6 +269,8 @@ extern "C" void ctprj_batch_destroy(ctprj_batch *b)
     cudaFree(b->d_fprefix);
     cudaFree(b->d_bprefix);
     cudaFree(b->d_tprefix);
+    cudaFree(b->d_sprefix);
+    cudaFree(b->d_oprefix);
     cudaFree(b->d_counter);
     cudaFree(b->d_status);
     delete b;
@@ -456,12 +472,12 @@ extern "C" int ctprj_batch_stream_backward(ctprj_batch *b, const int *dev_flags,
     cudaStream_t s = (cudaStream_t)stream;
     int st;
     if ((st = cuda_error(cudaMemsetAsync(b->d_counter + 1, 0, sizeof(unsigned long long), s), "batch counter")) ||
-        (st = cuda_error(cudaMemsetAsync(b->d_status, 0, sizeof(int) * b->n, s), "stream status")))
+        (st = cuda_error(cudaMemsetAsync(b->d_status, 0, 2 * sizeof(int) * b->n, s), "stream status")))
         return st;
     const int seg = b->seg <= 32 ? 32 : 64;
     const int vb = seg == 32 ? b->cfg.bwd_vb : 8;
     if ((st = launch_backward_stream(bwd_args(b), seg, vb, ctas(b, 1, bwd_param(b), b->cfg.bwd_occ),
-                                     dev_flags, b->d_status,
+                                     dev_flags, b->d_status + b->n, b->d_status,
                                      (unsigned long long)(timeout_s * 1e9), s)))
         return st;
     std::vector<int> h(b->n, 0);

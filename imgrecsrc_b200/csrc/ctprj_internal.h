@@ -86,8 +86,13 @@ struct BwdParams {
     int tiles_side;
     int zero_axes;            // even n: row 0 and column 0 written as zero
     float scale;              // output scale: FBP PI_f/np/dSize^2, BHC gradient Ts, else 1
-    int fast_shadow;          // fan: pixel shadows from the first-order expansion (staged kernel)
-    int win;                  // staged kernel: 3 detectors per pixel and view hold every shadow; 0: range
+    double invd;              // fan: 1 / d
+    float cG, invG;           // fan: dSize / d and d / dSize; parallel beam: 0 and 1 / dSize
+    int mode;                 // staged kernel: kBwdUnit, kBwdNarrow or kBwdRange
+    int split;                // staged kernel: parts the base views are summed in
+    int Wp;                   // entries of a table row
+    float4 *samp;             // sample image of the staged kernel, 2 x Wp per base view < prjFull/4
+    const float4 *foot;       // fan: its footprint table, Wp per base view < prjFull/4
     const BwdView *view;
     const DetEntry *det;
 };
@@ -113,6 +118,9 @@ struct BatchArgs {
     long long total;
     const long long *tprefix;      // quad-image tiles (natural order)
     long long ttotal;
+    const long long *sprefix;      // sample-image rows (natural order)
+    long long stotal;
+    const long long *oprefix;      // sample-image rows in `order`
     unsigned long long *counter;   // work counter, zero before each launch
 };
 
@@ -125,6 +133,9 @@ struct ctprj_plan {
     int nb, k0, nk;           // forward ray set (prj/cpuPrj.c:326-332, :469-475)
     int nv;                   // backward view count
     int bwd_seg;              // staged detectors per view and tile (32, 64), 0: unstaged
+    int bwd_split;            // parts the staged backprojection sums the base views in
+    float4 *d_samp, *d_foot;  // staged backprojection: sample image (scratch) and footprint table
+    char *d_arena;            // the plan's one allocation, which the next pointers lead into
     ctprj::FwdView *d_fview;
     ctprj::BwdView *d_bview;
     ctprj::DetEntry *d_det;
@@ -282,6 +293,9 @@ int bhc_forward_keep_projection(ctprj_bhc *m, const float *d_x, const double *d_
                                 double *d_f, float *proj, cudaStream_t s);
 int forward_blocks(const ctprj_plan *p);
 int backward_max_span(const ctprj_plan *p, int *max_span);
+int backward_split(const ctprj_plan *p);
+size_t backward_table_bytes(const Geo &g);
+int backward_tables(ctprj_plan *p, float4 *mem);
 FwdParams make_fwd_params(const ctprj_plan *p);
 BwdParams make_bwd_params(const ctprj_plan *p);
 // persistent batch launches (projector.cu)
@@ -289,7 +303,7 @@ int launch_quad_batch(const BatchArgs &a, cudaStream_t s);
 int launch_forward_batch(const BatchArgs &a, int views, int ctas, cudaStream_t s);
 int launch_backward_batch(const BatchArgs &a, int seg, int vb, int ctas, cudaStream_t s);
 int batch_max_ctas(int kind, int param, int *per_sm);
-int launch_backward_stream(const BatchArgs &a, int seg, int vb, int ctas, const int *ready,
+int launch_backward_stream(const BatchArgs &a, int seg, int vb, int ctas, const int *ready, int *rows_done,
                            int *status, unsigned long long timeout_ns, cudaStream_t s);
 int launch_backward(const ctprj_plan *p, const float *sino, float *img, int fbp,
                     unsigned long long *counter, cudaStream_t s, float scale = 1.0f);

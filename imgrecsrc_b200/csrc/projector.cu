@@ -13,10 +13,10 @@
 //            mirrored pixels of a pixel come from the plan's quad image (two
 //            float4 per pixel, built at the start of each call), so that every
 //            gather is a 16-byte load coalesced along x.
-//  backward  one thread per octant pixel 0 <= y <= x (pixel-driven,
+//  backward  one thread per pair of octant pixels 0 <= y <= x (pixel-driven,
 //            prj/cpuPrj.c:46-317), looping over the base views and the
-//            detectors under the pixel's shadow; each thread owns its eight
-//            output pixels, so no atomics are needed.
+//            detectors under the pair's shadow, staged in shared memory; each
+//            thread owns its sixteen output pixels, so no atomics are needed.
 //
 // Precision: the weights are FP32 but each distance from a ray is evaluated in
 // FP64 before rounding (x cos R + y sin R - offset cancels to O(1) from terms
@@ -26,6 +26,8 @@
 #include <climits>
 #include <cstdio>
 #include <type_traits>
+
+#include <cooperative_groups.h>
 
 #include "ctprj_internal.h"
 #include "footprint.cuh"
@@ -46,24 +48,14 @@ namespace ctprj {
 #define CTPRJ_FWD_MINBLOCKS 5
 #endif
 #ifndef CTPRJ_BWD_MINBLOCKS
-#define CTPRJ_BWD_MINBLOCKS 4
-#endif
-// CTPRJ_BWD_DERIVE = 1: the staged fan backprojection keeps one coefficient
-// plane per detector and derives the footprint's hw and w / (2 b1) from its
-// b2 / w (two reciprocals) instead of reading them from a second plane
-#ifndef CTPRJ_BWD_DERIVE
-#define CTPRJ_BWD_DERIVE 0
-#endif
-constexpr bool kBwdDerive = CTPRJ_BWD_DERIVE != 0;
-// CTPRJ_BWD_ASYNC = 1: the staged backprojection copies its mirrored sinogram
-// samples into shared memory by 4-byte cp.async (no register round trip; the
-// lane computes the ray coefficients while they are in flight)
-#ifndef CTPRJ_BWD_ASYNC
-#define CTPRJ_BWD_ASYNC 0
+#define CTPRJ_BWD_MINBLOCKS 5
 #endif
 constexpr int kFwdViews = CTPRJ_FWD_VIEWS;
 constexpr int kFwdThreads = 32 * kFwdViews;
 constexpr int kBwdTile = 16;   // 16 x 16 octant pixels per block
+// detectors of the staged backprojection (below): effectiveRate 1, below, above
+enum { kBwdUnit = 0, kBwdNarrow = 1, kBwdRange = 2 };
+constexpr int kBwdTablePad = 80;   // zero entries beyond the detectors at each end of a table row
 
 // --------------------------------------------------------------- quad image
 
@@ -1061,16 +1053,17 @@ __device__ __forceinline__ void backward_tile_direct(const BwdParams &p, int til
         }
     int tx, ty;
     decode_tile(tile, tx, ty);
-    const int x = tx * kBwdTile + (int)(threadIdx.x % kBwdTile);
-    const int y = ty * kBwdTile + (int)(threadIdx.x / kBwdTile);
-    if (x > g.half || y > x) return;
-    const int nimg = (y == 0 || y == x) ? 4 : 8;
-    float S[8];
+    for (int e = threadIdx.x; e < kBwdTile * kBwdTile; e += blockDim.x) {
+        const int x = tx * kBwdTile + e % kBwdTile, y = ty * kBwdTile + e / kBwdTile;
+        if (x > g.half || y > x) continue;
+        const int nimg = (y == 0 || y == x) ? 4 : 8;
+        float S[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) S[j] = 0.0f;
-    unsigned long long nz = 0;
-    for (int i = 0; i < p.nv; ++i) bwd_view_direct<FAN, false, false>(p, sino, i, x, y, nimg, S, nz);
-    write_octant(p, img, x, y, nimg, S);
+        for (int j = 0; j < 8; ++j) S[j] = 0.0f;
+        unsigned long long nz = 0;
+        for (int i = 0; i < p.nv; ++i) bwd_view_direct<FAN, false, false>(p, sino, i, x, y, nimg, S, nz);
+        write_octant(p, img, x, y, nimg, S);
+    }
 }
 
 template <bool FAN, bool COUNT, bool FBP>
@@ -1105,44 +1098,78 @@ k_backward(const BwdParams p, const float *__restrict__ sino, float *__restrict_
 // ------------------------------------------------------ backward, staged tiles
 //
 // The same backprojection with the per-(view, detector) work hoisted out of the
-// per-pixel loop.  A block owns a 16 x 16 tile of octant pixels; for a batch of
-// VB base views it first stages, for every detector under the tile's shadow,
-// (a) the ray's footprint coefficients and its distance from the tile centre,
-// computed in FP64 and rounded, and (b) the eight mirrored sinogram samples the
-// weight will multiply.  Each pixel then needs only its offset from the tile
-// centre: dist = D_k + cos B_k du + sin B_k dv, a saturating-FMA footprint and
-// eight shared-memory reads per detector.  The staging capacity SEG (detectors
-// per view and tile) is chosen per plan from the exact maximum shadow width,
-// found once by k_tile_span_max; geometries whose shadows exceed 64 detectors
-// use the unstaged kernel.
+// per-pixel loop.  Its operands come from two tables.  The sample image holds,
+// for base view i < prjFull/4 and detector k, the eight mirrored sinogram
+// samples one weight multiplies (two float4 planes, built by k_samples at the
+// start of each call; parallel beam: a sample plus its point-reflected partner
+// of the opposite view, which takes the same weight).  Base view i + a prjFull/4
+// reads the same samples, rotated among the images, so the accumulators are
+// rotated instead at each quarter.  The footprint table (fan beam) holds each
+// ray's trapezoid; a quarter turn leaves it as it is.
+//
+// A block owns a 16 x 16 tile of octant pixels.  For a batch of VB base views
+// it copies the detectors under the tile's shadow into shared memory by 16-byte
+// cp.async, double-buffered: the next batch is in flight while this one is
+// summed, at one barrier per batch.  A thread owns two pixels side by side and
+// reads each staged detector of the union of their windows once for both.
+//
+// What bounds it: the shared-memory data path (a warp's 16-byte load takes four
+// wavefronts whatever its lanes read) and instruction issue, about equally.
+// Samples and footprint of a fan detector are 48 bytes, twelve wavefronts; a
+// pixel on its own needs three detectors per view, a pair four (or three), so a
+// view costs 26 (20) wavefronts per 32 pixels instead of 38.  Packed
+// fma.rn.f32x2 gains nothing here: it takes two turns of the FP32 pipe.
+// Against one pixel per thread with samples gathered by each tile: 4.60 -> 3.01
+// ms at the 2048^2 fan workload, 149 -> 70 us at 512^2 (1024 detectors, 360
+// views), parallel 1001^2 (720 views) 814 -> 386 us and 256^2 78 -> 19 us.  At
+// 1024^2 (fan, 720 views): 116 warp instructions per 32 pixels and view, issue
+// 77 % active, shared-memory wavefronts 59 %, FP32 pipe 55 % (ncu).
+//
+// Geometry, in units of (distance from the ray) / cos B: with T = t / d the
+// tangent of detector k's fan angle, a pixel at (u, v) along / across the
+// detector lies at E_k = u - t_k + T_k v from ray k, the ray spacing there is
+// G = (d - v) dSize / d exactly, the half beam width G effectiveRate / 2, and
+// the pixel's trapezoid has lo = min(|c - T s|, |s + T c|) and hi = max(.).  So
+// E_k = E_r - (k - r) G from any reference detector r, the beam edges of
+// neighbouring detectors coincide (effectiveRate = 1), and cos B drops out.
+// The reference detector is the one nearest the centre of a warp's 8 x 8
+// pixels, with E_r formed in FP64 there: everything a pixel then adds is at
+// most a few units in size, so its rounding stays below 3e-7.  Parallel beam:
+// T = 0, G = dSize.
+//
+// Window: the beams that meet a pixel's footprint lie within rho = (shadow
+// width + effectiveRate) / 2 detectors of its projected centre.  The two pixels
+// project Delta = |c - T s| / G apart; if the right one's window starts o
+// detectors after the left one's, n detectors each hold both as soon as
+// n >= 2 rho + |Delta - o|.  The smallest n (and its smallest o) is chosen per
+// view and warp, so every lane takes the same straight code.  A beam wider than
+// the pitch (effectiveRate > 1) also meets pixels whose shadow its detector
+// lies outside of, which the reference's range rule (prj/cpuPrj.c:81-105,
+// :218-244) leaves out: such plans (RANGE) also test each detector against the
+// pixel's own corner shadow.
 
 struct TileSpan {
     int klo, nseg;
 };
 
 // Detectors any pixel of tile (tx, ty) can reach in base view bv, as the first
-// one (relative to the centre bin) and a count, with one spare on each side
-// (the pixels' own shadows are rounded to the nearest bin from FP32 corners).
+// one (relative to the centre bin) and a count, with one spare on each side;
+// `past` entries beyond the first and last detector may belong to it.
 // nseg = 1 << 20 flags a tile the source sees from behind or edge-on.
-__device__ __forceinline__ TileSpan tile_span(const Geo &g, const BwdView &bv, int tx, int ty)
+__device__ __forceinline__ float tile_corner(const Geo &g, float cf, float sf, int tx, int ty, int q, int &bad)
 {
-    const int dmax = (g.W - 1) / 2;
-    const float X0 = tx * kBwdTile - 0.5f, X1 = X0 + kBwdTile;
-    const float Y0 = ty * kBwdTile - 0.5f, Y1 = Y0 + kBwdTile;
-    const float cx[4] = {X0, X1, X1, X0}, cy[4] = {Y0, Y0, Y1, Y1};
-    float lo = 0.0f, hi = 0.0f;
-    bool bad = false;
-    for (int q = 0; q < 4; ++q) {
-        const float oc = fmaf(cx[q], bv.cf, cy[q] * bv.sf);
-        float tq = oc;
-        if (g.fan) {
-            const float qe = fmaf(cx[q], bv.sf, -cy[q] * bv.cf) + g.dF;
-            bad |= !(qe > 1e-3f * g.dF);
-            tq = g.dF * oc / qe;
-        }
-        lo = q == 0 ? tq : fminf(lo, tq);
-        hi = q == 0 ? tq : fmaxf(hi, tq);
-    }
+    const float X0 = tx * kBwdTile - 0.5f, Y0 = ty * kBwdTile - 0.5f;
+    const float cx = (q == 1 || q == 2) ? X0 + kBwdTile : X0, cy = q >= 2 ? Y0 + kBwdTile : Y0;
+    const float oc = fmaf(cx, cf, cy * sf);
+    if (!g.fan) return oc;
+    const float qe = fmaf(cx, sf, -cy * cf) + g.dF;
+    bad |= !(qe > 1e-3f * g.dF);
+    return g.dF * oc / qe;
+}
+
+__device__ __forceinline__ TileSpan span_of(const Geo &g, float lo, float hi, int bad, int past)
+{
+    const int dmax = (g.W - 1) / 2 + past;
     TileSpan sp;
     const float inv = (float)(1.0 / g.dSize), lim = (float)dmax + 2.0f;
     const int klo = max(__float2int_rd(fminf(fmaxf(lo * inv, -lim), lim)) - 1, -dmax);
@@ -1152,36 +1179,16 @@ __device__ __forceinline__ TileSpan tile_span(const Geo &g, const BwdView &bv, i
     return sp;
 }
 
-// The same span from a full warp: lane l takes corner l % 4, the four
-// corners' projections are reduced over aligned groups of four lanes (min and
-// max are exact, so every lane gets tile_span's result)
-__device__ __forceinline__ TileSpan tile_span_lanes(const Geo &g, const BwdView &bv, int tx, int ty, int lane)
+__device__ __forceinline__ TileSpan tile_span(const Geo &g, const BwdView &bv, int tx, int ty)
 {
-    const int dmax = (g.W - 1) / 2, q = lane & 3;
-    const float X0 = tx * kBwdTile - 0.5f, Y0 = ty * kBwdTile - 0.5f;
-    const float cx = (q == 1 || q == 2) ? X0 + kBwdTile : X0, cy = q >= 2 ? Y0 + kBwdTile : Y0;
-    const float oc = fmaf(cx, bv.cf, cy * bv.sf);
-    float tq = oc;
     int bad = 0;
-    if (g.fan) {
-        const float qe = fmaf(cx, bv.sf, -cy * bv.cf) + g.dF;
-        bad = !(qe > 1e-3f * g.dF);
-        tq = g.dF * oc / qe;
+    float lo = 0.0f, hi = 0.0f;
+    for (int q = 0; q < 4; ++q) {
+        const float tq = tile_corner(g, bv.cf, bv.sf, tx, ty, q, bad);
+        lo = q == 0 ? tq : fminf(lo, tq);
+        hi = q == 0 ? tq : fmaxf(hi, tq);
     }
-    float lo = tq, hi = tq;
-#pragma unroll
-    for (int o = 1; o <= 2; o <<= 1) {
-        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-        bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-    }
-    TileSpan sp;
-    const float inv = (float)(1.0 / g.dSize), lim = (float)dmax + 2.0f;
-    const int klo = max(__float2int_rd(fminf(fmaxf(lo * inv, -lim), lim)) - 1, -dmax);
-    const int khi = min(__float2int_ru(fminf(fmaxf(hi * inv, -lim), lim)) + 1, dmax);
-    sp.klo = klo;
-    sp.nseg = bad ? (1 << 20) : khi - klo + 1;
-    return sp;
+    return span_of(g, lo, hi, bad, 0);
 }
 
 __global__ void k_tile_span_max(const BwdParams p, int tiles, int *__restrict__ out)
@@ -1197,517 +1204,568 @@ __global__ void k_tile_span_max(const BwdParams p, int tiles, int *__restrict__ 
     atomicMax(out, m);
 }
 
-struct TileView {
-    double uc, vc;        // tile centre along / across the detector (FP64)
-    float cT, sT;
-    float ucf, qec;       // u of the centre; d - v of the centre
-    float hw;             // parallel: (|cos| + |sin|) / 2
-    float A, B, AB;       // fan: (cos + sin) / 2, (cos - sin) / 2 (pixel corner offsets), A B
-    int klo, nseg;
+// footprint of the direction (a, b), scaled by any positive factor: 1 / lo,
+// (foot half width) / lo, 1 / (2 shoulder half width), lo / (2 hi).  Zero ramp
+// or shoulder widths get a tiny floor: the huge ratios saturate and are
+// multiplied by the zero width.
+__device__ __forceinline__ float4 staged_footprint(float a, float b)
+{
+    a = fabsf(a);
+    b = fabsf(b);
+    const float hi = fmaxf(a, b), lo = fminf(a, b);
+    const float cw = 1.0f / fmaxf(lo, 1e-30f);
+    return make_float4(cw, 0.5f * (hi + lo) * cw, 1.0f / fmaxf(hi - lo, 1e-30f), 0.5f * lo / hi);
+}
+
+// The footprint table of a fan plan: row i < prjFull/4, entry k + W/2 + kBwdTablePad.
+__global__ void __launch_bounds__(256) k_footprints(const BwdParams p, float4 *__restrict__ foot)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= p.Wp) return;
+    const float T = (float)(k - p.g.pC - kBwdTablePad) * p.cG;
+    for (int i = blockIdx.y; i < p.g.P / 4; i += gridDim.y) {
+        const float c = p.view[i].cf, s = p.view[i].sf;
+        foot[(size_t)i * p.Wp + k] = staged_footprint(fmaf(-T, s, c), fmaf(T, c, s));
+    }
+}
+
+// Row i of the sample image (a block's threads along the detectors); the
+// entries beyond the detectors stay zero.
+__device__ __forceinline__ void sample_row(const BwdParams &p, const float *__restrict__ sino, int i,
+                                           int k0, int step)
+{
+    const Geo &g = p.g;
+    const int dmax = (g.W - 1) / 2, pC = g.pC, Q = g.P / 4;
+    const float *src[8], *src2[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        // rows of the symmetric views (the host's view_of), and of the opposite ones
+        const int q = j < 4 ? j : (j - 2) & 3;
+        int v = j < 4 ? q * Q + i : q * Q - i;
+        v = v < 0 ? v + g.P : v;
+        int v2 = v + 2 * Q;
+        v2 = v2 >= g.P ? v2 - g.P : v2;
+        src[j] = v < g.np ? sino + (size_t)v * g.W + pC : nullptr;
+        src2[j] = !g.fan && v2 < g.np ? sino + (size_t)v2 * g.W + pC : nullptr;
+    }
+    float4 *dst = p.samp + (size_t)i * 2 * p.Wp + pC + kBwdTablePad;
+    for (int k = k0 - dmax; k <= dmax; k += step) {
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = src[j] ? __ldg(src[j] + (j < 4 ? k : -k)) : 0.0f;
+        if (!g.fan)
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (src2[j]) v[j] += __ldg(src2[j] - (j < 4 ? k : -k));
+        dst[k] = make_float4(v[0], v[1], v[2], v[3]);
+        dst[p.Wp + k] = make_float4(v[4], v[5], v[6], v[7]);
+    }
+}
+
+constexpr int kSampThreads = 128;
+
+__global__ void __launch_bounds__(kSampThreads) k_samples(const BwdParams p, const float *__restrict__ sino)
+{
+    for (int i = blockIdx.y; i < p.g.P / 4; i += gridDim.y)
+        sample_row(p, sino, i, blockIdx.x * kSampThreads + threadIdx.x, gridDim.x * kSampThreads);
+}
+
+constexpr int kBwdThreads = kBwdTile * kBwdTile / 2;   // two pixels per thread
+constexpr int kBwdWarps = kBwdThreads / 32;            // one 8 x 8 pixel square each
+// Staged past the detectors' ends (zeros), so that the union of two windows up
+// to two detectors apart can lie anywhere on them; a row of the staging buffer
+// holds the plan's widest span and these.
+constexpr int kBwdPast = 2;
+constexpr int kBwdGroup = 32;  // views whose geometry the block prepares at a time
+constexpr float kBwdMagic = 12582912.0f;   // 1.5 * 2^23: x + it rounds |x| < 2^22 to an integer,
+constexpr int kBwdMagicBits = 0x4B400000;  // whose value is the sum's bits minus these
+
+// one view as a warp's pixel square sees it
+struct BwdSquare {
+    float E, T, qec;   // reference detector r: E_r and T_r; d - v of the square's centre (parallel: r)
+    int ioff;          // staged index of detector r, minus kBwdMagicBits
+    float c, s;        // direction of the view
+    float lo, hi;      // range of the union's first detector, relative to r
+    float off;         // (n - 1 + o) / 2: from a pair's projection to that detector
+    float kh, g;       // half the step of E, and of G, from the pixel at x to the one at x + 1
+    int code;          // n, and the offsets in the union of x's window << 8 and x + 1's << 16
 };
 
-// shared memory of one staged tile
+// shared memory of one staged tile: two buffers of VB views
 template <bool FAN, int SEG, int VB>
 struct TiledSmem {
-    // per staged detector, fan beam: D, cos B, sin B (all / w) and the
-    // footprint's b2 / w; its hw and w / (2 b1) (the half beam width at depth
-    // qe is qe (beam width / 2d) cos B / w: a multiple of the second
-    // component).  Parallel beam: D / w.  A pixel reads 24 (4) bytes of them
-    // per detector; the second plane keeps the 16-byte stride of the first
-    // (measured faster than a packed 8-byte plane: 4.70 against 4.75 ms at the
-    // 2048^2 fan workload, 0.90 against 1.00 ms at 1024^2 with d = 2048)
-    float4 ra[FAN ? VB : 1][FAN ? SEG : 1];
-    float4 rb[FAN && !kBwdDerive ? VB : 1][FAN && !kBwdDerive ? SEG : 1];
-    float rx[FAN ? 1 : VB][FAN ? 1 : SEG];
-    // the eight (sixteen) mirrored samples of a staged ray as two (four)
-    // float4 planes: two (four) 16-byte reads per detector and pixel, and
-    // consecutive detectors in consecutive banks
-    float4 seg[VB][2][SEG];
-    float4 seg2[FAN ? 1 : VB][2][FAN ? 1 : SEG];
-    TileView tv[VB];
-    FootprintV pfs[VB];
+    float4 seg[2][VB][FAN ? 3 : 2][SEG + 2 * kBwdPast];     // samples 0-3, samples 4-7, footprints
+    BwdSquare sq[2][kBwdGroup][kBwdWarps];
+    float4 fp[2][FAN ? 1 : kBwdGroup];       // parallel beam: the view's footprint
 };
 
-// one float from global into shared memory without a register round trip;
-// an invalid source reads nothing and writes zero
-__device__ __forceinline__ void stage_async4(float *smem, const float *gmem, bool valid)
+__device__ __forceinline__ void stage16(float4 *smem, const float4 *gmem)
 {
     const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sa), "l"(gmem), "r"(valid ? 4 : 0)
-                 : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
 
-// The footprint numbers of a staged fan detector.  All three follow from
-// t = lo / hi of the ray's direction: b2 / w = (1 + t) / (2 t), hw = t / 2 =
-// 1 / (4 b2/w - 2) and w / (2 b1) = t / (1 - t) = 1 / (2 b2/w - 2).  The
-// derived pair also holds where make_footprint_v floors a zero width: for
-// w = 0, hw comes out ~1e-31 (it multiplies a bounded term) and w / (2 b1)
-// matches the floored ratio; for b1 = 0 the floor below keeps the ratio
-// finite.  Each is within ~1e-7 of the stored value's effect on a weight.
-__device__ __forceinline__ FootprintV staged_footprint(const float4 a, const float4 &b)
+__device__ __forceinline__ float sat_fma(float a, float b, float c) { return __saturatef(fmaf(a, b, c)); }
+
+// Weight of a detector between its beam edges el and er: the trapezoid's area
+// between them (footprint_weight_v's form: rising and falling ramps P and R,
+// plateau Q).
+__device__ __forceinline__ float edge_weight(float el, float er, float4 f)
 {
-    FootprintV f;
-    f.c1 = a.w;
-    if (kBwdDerive) {
-        f.hw = __fdividef(1.0f, fmaf(4.0f, a.w, -2.0f));
-        f.rho = __fdividef(1.0f, fmaxf(fmaf(2.0f, a.w, -2.0f), 1e-30f));
+    const float P1 = sat_fma(er, f.x, f.y), R1 = sat_fma(er, -f.x, f.y), Q1 = sat_fma(er, f.z, 0.5f);
+    const float P2 = sat_fma(el, f.x, f.y), R2 = sat_fma(el, -f.x, f.y), Q2 = sat_fma(el, f.z, 0.5f);
+    const float dQ = Q1 - Q2;
+    const float X = fmaf(R2, R2, fmaf(-P2, P2, fmaf(-R1, R1, P1 * P1)));
+    return fmaf(f.w, fmaf(-2.0f, dQ, X), dQ);
+}
+
+// area of the trapezoid from its centre to the edge e, plus a constant
+// (parallel beam: every detector of a view has the same footprint, so
+// neighbouring weights share it)
+__device__ __forceinline__ float edge_area(float e, float4 f)
+{
+    const float P = sat_fma(e, f.x, f.y), R = sat_fma(e, -f.x, f.y), Q = sat_fma(e, f.z, 0.5f);
+    return fmaf(f.w, fmaf(-2.0f, Q, fmaf(-R, R, P * P)), Q);
+}
+
+// the geometry of view i for square w of tile (tx, ty), whose detectors are
+// staged from klo; the window (n, o) is returned in q.code, q.lo, q.hi left open
+template <bool FAN>
+__device__ __forceinline__ BwdSquare square_view(const BwdParams &p, const BwdView &bv, int tx, int ty, int w, int klo,
+                                                 int seg)
+{
+    const Geo &g = p.g;
+    const double xw = tx * kBwdTile + (w & 1) * 8 + 3.5, yw = ty * kBwdTile + (w >> 1) * 8 + 3.5;
+    const double uc = fma(xw, bv.c, yw * bv.s);
+    BwdSquare q;
+    q.c = bv.cf;
+    q.s = bv.sf;
+    // (r is held near the detector: squares that project far off it meet no ray
+    // whatever the reference)
+    const float rmax = (float)(g.W / 2 + 128);
+    float r, G, Gmin, slack = 0.0f;
+    if (FAN) {
+        const double qd = g.d - fma(yw, bv.c, -xw * bv.s);
+        q.qec = (float)qd;
+        r = fminf(fmaxf(rintf(__fdividef((float)uc * p.invG, q.qec)), -rmax), rmax);
+        const double T = (double)r * g.dSize * p.invd;
+        q.T = (float)T;
+        q.E = (float)fma(-T, qd, uc);
+        // a pixel lies within 5 of the square's centre and every pixel of a
+        // staged tile has qe > d / 1000; the rays that meet the square differ
+        // from r's tangent by at most (5 (1 + |T|) + G + 3/4) / qe
+        const float qm = fmaxf(q.qec - 5.0f, 1e-3f * g.dF);
+        G = q.qec * p.cG;
+        Gmin = qm * p.cG;
+        slack = __fdividef(fmaf(1.5f, G, fmaf(9.0f, fabsf(q.T), 9.0f)), qm);
     } else {
-        f.hw = b.x;
-        f.rho = b.y;
+        r = fminf(fmaxf(rintf((float)uc * p.invG), -rmax), rmax);
+        q.T = 0.0f;
+        q.qec = r;
+        q.E = (float)fma(-(double)r, g.dSize, uc);
+        G = Gmin = (float)g.dSize;
     }
-    return f;
-}
-
-// Staging of one batch of VB base views for tile (tx, ty) (every thread of the
-// block takes part; ends with a block barrier), a warp per view: A, the
-// tile's detector span and centre in the view (every lane computes it, lane 0
-// keeps it for the pixels' pass); B1, the footprint coefficients of the staged
-// detectors; B2, their mirrored sinogram samples (a lane per detector: each
-// load instruction reads one sinogram row contiguously).
-template <bool FAN, int SEG, int VB>
-__device__ __forceinline__ void stage_batch(const BwdParams &p, const float *__restrict__ sino, int tx, int ty,
-                                            double xc, double yc, int i0, int nb, TiledSmem<FAN, SEG, VB> &sm)
-{
-    const Geo &g = p.g;
-    auto &ra = sm.ra;
-    auto &rb = sm.rb;
-    auto &rx = sm.rx;
-    auto &seg = sm.seg;
-    auto &seg2 = sm.seg2;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kWarps = blockDim.x >> 5;
-    const int pC = g.pC;
-    for (int iv = warp; iv < nb; iv += kWarps) {
-        const BwdView &bv = p.view[i0 + iv];
-        // A
-        const TileSpan sp = tile_span_lanes(g, bv, tx, ty, lane);
-        TileView t;
-        t.cT = bv.cf;
-        t.sT = bv.sf;
-        t.uc = fma(xc, bv.c, yc * bv.s);
-        t.vc = fma(yc, bv.c, -xc * bv.s);
-        t.ucf = (float)t.uc;
-        t.qec = (float)(g.d - t.vc);
-        t.hw = 0.5f * (fabsf(bv.cf) + fabsf(bv.sf));
-        t.A = 0.5f * (bv.cf + bv.sf);
-        t.B = 0.5f * (bv.cf - bv.sf);
-        t.AB = t.A * t.B;
-        t.klo = sp.klo;
-        t.nseg = min(sp.nseg, SEG);   // the plan chose SEG above every span
-        const FootprintV pf = FAN ? FootprintV{} : make_footprint_v(bv.cf, bv.sf);
-        if (lane == 0) {
-            sm.tv[iv] = t;
-            if (!FAN) sm.pfs[iv] = pf;
-        }
-#if CTPRJ_BWD_ASYNC
-        // B2 first, asynchronously: the same samples as below, in flight while
-        // B1 runs; the block barrier at the end follows a wait for them
-        for (int kk = lane; kk < t.nseg; kk += 32) {
-            const int dt = t.klo + kk;
+    const float kx = fmaf(-q.T, q.s, q.c), ky = fmaf(q.T, q.c, q.s);
+    q.kh = 0.5f * kx;
+    q.g = FAN ? 0.5f * q.s * p.cG : 0.0f;
+    // 2 rho, and the range of Delta over the square
+    const float inv = __fdividef(1.0f, Gmin);
+    const float reach = fmaf(fabsf(kx) + fabsf(ky) + slack, inv, g.effRate + 2e-3f);
+    const float dlo = fmaf(-slack, inv, __fdividef(fabsf(kx), G)), dhi = fmaf(slack, inv, fabsf(kx) * inv);
+    int n = 1 << 20, o = 0;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int row = bv.row[j];
-                stage_async4(&seg[iv][j >> 2][kk].x + (j & 3),
-                             sino + (row >= 0 ? row + pC + (j < 4 ? dt : -dt) : 0), row >= 0);
-            }
-            if (!FAN) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int row2 = bv.row2[j];
-                    stage_async4(&seg2[FAN ? 0 : iv][j >> 2][FAN ? 0 : kk].x + (j & 3),
-                                 sino + (row2 >= 0 ? row2 + pC - (j < 4 ? dt : -dt) : 0), row2 >= 0);
-                }
-            }
-        }
-#endif
-        for (int kk = lane; kk < t.nseg; kk += 32) {
-            // B1
-            const DetEntry &de = p.det[t.klo + kk + pC];
-            if (FAN) {
-                const double D = fma(de.cB, t.uc - de.t, de.sB * t.vc);
-                const float cR = fmaf(de.cBf, t.cT, -de.sBf * t.sT);
-                const float sR = fmaf(de.sBf, t.cT, de.cBf * t.sT);
-                const FootprintV f = make_footprint_v(cR, sR);
-                ra[FAN ? iv : 0][FAN ? kk : 0] = make_float4((float)D * f.iw, de.cBf * f.iw, de.sBf * f.iw, f.c1);
-                if (!kBwdDerive)
-                    rb[FAN && !kBwdDerive ? iv : 0][FAN && !kBwdDerive ? kk : 0] = make_float4(f.hw, f.rho, 0.0f, 0.0f);
-            } else {
-                rx[FAN ? 0 : iv][FAN ? 0 : kk] = (float)(t.uc - de.t) * pf.iw;
-            }
-#if !CTPRJ_BWD_ASYNC
-            // B2
-            const int dt = t.klo + kk;
-            float v[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int row = bv.row[j];
-                v[j] = row >= 0 ? __ldg(sino + row + pC + (j < 4 ? dt : -dt)) : 0.0f;
-            }
-            seg[iv][0][kk] = make_float4(v[0], v[1], v[2], v[3]);
-            seg[iv][1][kk] = make_float4(v[4], v[5], v[6], v[7]);
-            if (!FAN) {   // the point-reflected detectors of the opposite view
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int row2 = bv.row2[j];
-                    v[j] = row2 >= 0 ? __ldg(sino + row2 + pC - (j < 4 ? dt : -dt)) : 0.0f;
-                }
-                seg2[FAN ? 0 : iv][0][FAN ? 0 : kk] = make_float4(v[0], v[1], v[2], v[3]);
-                seg2[FAN ? 0 : iv][1][FAN ? 0 : kk] = make_float4(v[4], v[5], v[6], v[7]);
-            }
-#endif
+    for (int t = 0; t < 3; ++t) {
+        const float need = reach + fmaxf(fabsf(dlo - (float)t), fabsf(dhi - (float)t));
+        const int nt = max(__float2int_ru(fminf(need, 4096.0f)), 2);
+        if (nt < n) {
+            n = nt;
+            o = t;
         }
     }
-#if CTPRJ_BWD_ASYNC
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-#endif
-    __syncthreads();
+    n = min(n, seg - o);   // the union never exceeds the staged detectors
+    q.off = 0.5f * (float)(n - 1 + o);
+    q.code = n | (o << (kx < 0.0f ? 8 : 16));   // the window of the pixel further along starts later
+    q.ioff = (int)r - klo - kBwdMagicBits;
+    q.lo = (float)klo - r;
+    q.hi = q.lo;
+    return q;
 }
 
-// One tile of the staged backprojection (all threads of the block take part).
-// WIN = 3: every pixel shadow of the plan is narrower than 1.9 detectors (the
-// plan's bound), so the detectors a pixel reaches in a view always lie within
-// the three centred on the projection of its centre, tc; WIN = 4: narrower
-// than 2.85, and they lie within the four from floor(tc) - 1.  Those detectors
-// are summed straight, without the per-pixel shadow range (WIN = 0: the
-// range).  A detector of the window that the reference's range rule
-// (prj/cpuPrj.c:218-244) leaves out lies beyond the pixel's footprint and adds
-// a weight of exactly zero, except within ~1e-4 detector of a shadow edge,
-// where the footprint and the exact corner shadow differ and the weight is
-// below 1e-7.
-template <bool FAN, bool FBP, int SEG, int VB, int WIN>
-__device__ __forceinline__ void backward_tile(const BwdParams &p, int tile,
-                                              const float *__restrict__ sino,
-                                              float *__restrict__ img,
-                                              TiledSmem<FAN, SEG, VB> &sm)
-{
-    const Geo &g = p.g;
-    auto &ra = sm.ra;
-    auto &rb = sm.rb;
-    auto &rx = sm.rx;
-    auto &seg = sm.seg;
-    auto &seg2 = sm.seg2;
-    auto &tv = sm.tv;
-    auto &pfs = sm.pfs;
+// what a thread's pair of pixels takes from a view before its weights
+struct PairView {
+    float EA, EB, GA, GB;   // of the pixels at x and x + 1
+    float cb;               // first detector of the union, relative to r
+    int i0;                 // its staged index
+};
 
-    if (p.zero_axes && tile == 0)
-        for (int i = threadIdx.x; i < g.n; i += blockDim.x) {
-            img[i] = 0.0f;
-            img[(size_t)i * g.n] = 0.0f;
+template <bool FAN>
+__device__ __forceinline__ PairView pair_start(const BwdParams &p, const BwdSquare &q, float dx, float dy)
+{
+    const float du = fmaf(dx, q.c, dy * q.s), dv = fmaf(dy, q.c, -dx * q.s);
+    const float E = FAN ? fmaf(q.T, dv, q.E + du) : q.E + du;
+    const float qe = FAN ? q.qec - dv : 1.0f;
+    // the pair's projection E / G in detectors from r, less its offset in the union
+    const float t = FAN ? fmaf(E * p.invG, __fdividef(1.0f, qe), -q.off) : fmaf(E, p.invG, -q.off);
+    // nearest integer by an FP32 add; its bits are the staged index
+    const float m = fminf(fmaxf(t, q.lo), q.hi) + kBwdMagic;
+    PairView v;
+    v.cb = m - kBwdMagic;
+    v.i0 = __float_as_int(m) + q.ioff;
+    v.EA = E - q.kh;
+    v.EB = E + q.kh;
+    const float G = FAN ? qe * p.cG : (float)p.g.dSize;
+    v.GA = FAN ? G - q.g : G;
+    v.GB = FAN ? G + q.g : G;
+    return v;
+}
+
+// S += w p for the eight images of a pixel
+__device__ __forceinline__ void add_samples(float (&S)[8], float w, float4 p0, float4 p1)
+{
+    S[0] = fmaf(w, p0.x, S[0]);
+    S[1] = fmaf(w, p0.y, S[1]);
+    S[2] = fmaf(w, p0.z, S[2]);
+    S[3] = fmaf(w, p0.w, S[3]);
+    S[4] = fmaf(w, p1.x, S[4]);
+    S[5] = fmaf(w, p1.y, S[5]);
+    S[6] = fmaf(w, p1.z, S[6]);
+    S[7] = fmaf(w, p1.w, S[7]);
+}
+
+// FBP weight of a pixel, (d / qe)^2 with qe = G / cG
+template <bool FAN, bool FBP>
+__device__ __forceinline__ float fbp_weight(const BwdParams &p, float G)
+{
+    if (!FAN || !FBP) return 1.0f;
+    const float f = __fdividef((float)p.g.dSize, G);
+    return f * f;
+}
+
+// One view for a pair of pixels, A and B the sums of x and x + 1: windows of N
+// detectors at OA and OB in the union.
+template <bool FAN, bool FBP, int SEG, bool UNIT, int N, int OA, int OB>
+__device__ __forceinline__ void pair_view(const BwdParams &p, const PairView &v, const float4 *__restrict__ seg,
+                                          float4 fpar, float (&A)[8], float (&B)[8])
+{
+    constexpr int U = N + (OA > OB ? OA : OB);
+    const float4 *s0 = seg + v.i0, *s1 = s0 + SEG + 2 * kBwdPast, *fp = s1 + SEG + 2 * kBwdPast;
+    const float hb = 0.5f * p.g.effRate;
+    const float fA = fbp_weight<FAN, FBP>(p, v.GA), fB = fbp_weight<FAN, FBP>(p, v.GB);
+    // left edges of the first detectors; parallel beam: the areas up to them
+    float eA = fmaf(v.cb + ((float)OA - hb), v.GA, -v.EA), eB = fmaf(v.cb + ((float)OB - hb), v.GB, -v.EB);
+    if (!FAN && UNIT) {
+        eA = edge_area(eA, fpar);
+        eB = edge_area(eB, fpar);
+    }
+    // weight of slot j: its right edge becomes the next slot's left one
+    auto weight = [&](float &e, int j, float G, float E, float4 f) {
+        const float r = fmaf(v.cb + ((float)j + hb), G, -E), l = e;
+        if (!FAN && UNIT) {
+            e = edge_area(r, f);
+            return e - l;
         }
-    int tx, ty;
-    decode_tile(tile, tx, ty);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // a warp takes an 8 x 4 block of the tile, each half-warp a 4 x 4 square:
-    // the 16 pixels of a square project onto at most 3 sqrt(2) m + 1
-    // consecutive staged detectors (m the magnification), fewer than the
-    // eight 16-byte entries that share no bank, so a half-warp's window loads
-    // never conflict (8 x 2 rows do)
-#if CTPRJ_BWD_ROWS
-    const int x = tx * kBwdTile + ((warp & 1) << 3) + (lane & 7);
-    const int y = ty * kBwdTile + ((warp >> 1) << 2) + (lane >> 3);
-#else
-    const int x = tx * kBwdTile + ((warp & 1) << 3) + ((lane >> 4) << 2) + (lane & 3);
-    const int y = ty * kBwdTile + ((warp >> 1) << 2) + ((lane >> 2) & 3);
-#endif
-    const bool valid = x <= g.half && y <= x;
-    const int nimg = (y == 0 || y == x) ? 4 : 8;
-    const double xc = tx * kBwdTile + 0.5 * (kBwdTile - 1), yc = ty * kBwdTile + 0.5 * (kBwdTile - 1);
-    const float dx = (float)(x - xc), dy = (float)(y - yc);
-    const int dmax = (g.W - 1) / 2;
-    const float invdS = (float)(1.0 / g.dSize), dFs = (float)((double)g.dF / g.dSize);
-    const float hbpar = 0.5f * g.beamWidthF;
-    // fan beam: the half beam width at depth qe on ray B, over w, is
-    // qe Kb (cos B / w) (prj/cpuPrj.c:254: bw = qe beamWidth cos B / d)
-    const float Kb = FAN ? (float)(0.5 * g.beamWidth / g.d) : 0.0f;
-    // the eight sums, S[j] += w p[j], in pairs: one fma.rn.f32x2 for two
-    // sums (each rounded as one fmaf)
-    float2 S2[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) S2[j] = make_float2(0.0f, 0.0f);
-    auto accumulate = [&](const float w, const float4 p0, const float4 p1) {
-        const float2 ww = make_float2(w, w);
-        S2[0] = __ffma2_rn(ww, make_float2(p0.x, p0.y), S2[0]);
-        S2[1] = __ffma2_rn(ww, make_float2(p0.z, p0.w), S2[1]);
-        S2[2] = __ffma2_rn(ww, make_float2(p1.x, p1.y), S2[2]);
-        S2[3] = __ffma2_rn(ww, make_float2(p1.z, p1.w), S2[3]);
+        e = UNIT ? r : fmaf(v.cb + ((float)(j + 1) - hb), G, -E);
+        return edge_weight(l, r, f);
     };
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+        const float4 f = FAN ? fp[j] : fpar, p0 = s0[j], p1 = s1[j];
+        if (j >= OA && j < OA + N) {
+            const float w = weight(eA, j, v.GA, v.EA, f);
+            add_samples(A, FBP && FAN ? w * fA : w, p0, p1);
+        }
+        if (j >= OB && j < OB + N) {
+            const float w = weight(eB, j, v.GB, v.EB, f);
+            add_samples(B, FBP && FAN ? w * fB : w, p0, p1);
+        }
+    }
+}
 
-    for (int i0 = 0; i0 < p.nv; i0 += VB) {
-        const int nb = min(VB, p.nv - i0);
-        stage_batch<FAN, SEG, VB>(p, sino, tx, ty, xc, yc, i0, nb, sm);
-        // C: every pixel of the tile over the batch
-        if (valid) {
-            for (int iv = 0; iv < nb; ++iv) {
-                const TileView &t = tv[iv];
-                const float du = fmaf(dx, t.cT, dy * t.sT);
-                const float dv = fmaf(dy, t.cT, -dx * t.sT);
-                const float u = t.ucf + du;
-                if (WIN > 0 && t.nseg >= WIN) {   // t.nseg is the same for the whole block
-                    const float qe = FAN ? t.qec - dv : 0.0f;
-                    // the detector under the pixel centre, in staged units
-                    const float tc = FAN ? __fdividef(dFs * u, qe) : u * invdS;
-                    // nearest detector, half to even as __float2int_rn, by an FP32
-                    // add: for |tc| < 2^22 (staged units: |tc| < the row length)
-                    // tc + 1.5 * 2^23 lies in [2^23, 2^24), where the add rounds to
-                    // an integer, so its low mantissa bits are that integer (one
-                    // arithmetic op instead of a conversion on the XU pipe: 0.5 %
-                    // at the 2048^2 fan workload, 1.5-2 % at 512^2 and 256^2)
-                    const int ks = WIN == 3 ? __float_as_int(tc + 12582912.0f) - 0x4B400000 : __float2int_rd(tc);
-                    const int k0 = min(max(ks - 1 - t.klo, 0), t.nseg - WIN);
-                    const float fbpw = FBP ? __fdividef(g.dF, qe) * __fdividef(g.dF, qe) : 1.0f;
-                    const FootprintV fpar = FAN ? FootprintV{} : pfs[iv];
-                    const float duw = FAN ? 0.0f : du * fpar.iw, Hpar = FAN ? 0.0f : hbpar * fpar.iw;
-                    const float qeK = qe * Kb;
-                    float w[WIN > 0 ? WIN : 1];
+// The same for any window, and with RANGE only the detectors of the pixel's
+// corner shadow (prj/cpuPrj.c:218-244), rounded to the nearest detectors.
+template <bool FAN, bool FBP, int SEG, bool RANGE>
+__device__ __forceinline__ void pair_view_any(const BwdParams &p, const BwdSquare &q, const PairView &v,
+                                              const float4 *__restrict__ seg, float4 fpar, float (&A)[8], float (&B)[8],
+                                              const BwdView &bv, int x, int y)
+{
+    const float4 *s0 = seg + v.i0, *s1 = s0 + SEG + 2 * kBwdPast, *fp = s1 + SEG + 2 * kBwdPast;
+    const int n = q.code & 255, oa = (q.code >> 8) & 255, ob = q.code >> 16;
+    const float hb = 0.5f * p.g.effRate;
+    const float fA = fbp_weight<FAN, FBP>(p, v.GA), fB = fbp_weight<FAN, FBP>(p, v.GB);
+    float loA = 0.0f, hiA = 0.0f, loB = 0.0f, hiB = 0.0f;
+    if (RANGE) {
+        const float ca = 0.5f * (q.c + q.s), cb = 0.5f * (q.c - q.s);
+        const float r = FAN ? rintf(q.T * p.invG) : q.qec;
+        auto range = [&](float E, float G, int px, float &lo, float &hi) {
+            float tlo, thi;
+            if (FAN) {
+                const float qe = G * p.invG, ea = fmaf(q.T, cb, ca), eb = fmaf(-q.T, ca, cb);
+                const float t0 = __fdividef(E - ea, qe + cb), t1 = __fdividef(E + eb, qe + ca);
+                const float t2 = __fdividef(E + ea, qe - cb), t3 = __fdividef(E - eb, qe - ca);
+                tlo = fminf(fminf(t0, t1), fminf(t2, t3)) * p.invG;
+                thi = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)) * p.invG;
+            } else {
+                // (in FP64: views along an axis put every shadow edge half way
+                // between detectors, give or take the rounding of the view's angle)
+                const double u = fma((double)px, bv.c, y * bv.s), hw = 0.5 * (fabs(bv.c) + fabs(bv.s));
+                lo = (float)(round((u - hw) / p.g.dSize) - (double)r);
+                hi = (float)(round((u + hw) / p.g.dSize) - (double)r);
+                return;
+            }
+            // nearest detector, half-way cases away from the centre as the
+            // reference's round(): relative to r, by the sign of the place
+            auto nearest = [&](float t) { return r + t < 0.0f ? ceilf(t - 0.5f) : floorf(t + 0.5f); };
+            lo = nearest(tlo);
+            hi = nearest(thi);
+        };
+        range(v.EA, v.GA, x, loA, hiA);
+        range(v.EB, v.GB, x + 1, loB, hiB);
+    }
+    for (int j = 0; j < n + oa + ob; ++j) {   // one of the offsets is zero
+        const float k = v.cb + (float)j;
+        const float4 f = FAN ? fp[j] : fpar, p0 = s0[j], p1 = s1[j];
+        if (j >= oa && j < oa + n && (!RANGE || (k >= loA && k <= hiA))) {
+            const float w = edge_weight(fmaf(k - hb, v.GA, -v.EA), fmaf(k + hb, v.GA, -v.EA), f);
+            add_samples(A, FBP && FAN ? w * fA : w, p0, p1);
+        }
+        if (j >= ob && j < ob + n && (!RANGE || (k >= loB && k <= hiB))) {
+            const float w = edge_weight(fmaf(k - hb, v.GB, -v.EB), fmaf(k + hb, v.GB, -v.EB), f);
+            add_samples(B, FBP && FAN ? w * fB : w, p0, p1);
+        }
+    }
+}
+
+// the accumulators of one quarter of the views for the next: base view i +
+// prjFull/4 finds image j's sample where view i has that of the image a quarter
+// turn on
+__device__ __forceinline__ void rotate_sums(float (&S)[8])
+{
+    const float a = S[3], b = S[4];
+    S[3] = S[2];
+    S[2] = S[1];
+    S[1] = S[0];
+    S[0] = a;
+    S[4] = S[5];
+    S[5] = S[6];
+    S[6] = S[7];
+    S[7] = b;
+}
+
+// Adds the base views [v0, v1), all of one quarter that begins at view vq, to
+// the sums of one tile: A of a thread's pixel x and B of x + 1 (all threads of
+// the block take part).  Every product that meets a sum in here and in what it
+// calls is an explicit fma, so that no kernel this is inlined into contracts
+// it differently: the batched and per-plan launches must give the same bits.
+template <bool FAN, bool FBP, int SEG, int VB, int MODE>
+__device__ __forceinline__ void quarter_sums(const BwdParams &p, int tx, int ty, int v0, int v1, int vq, float (&A)[8],
+                                             float (&B)[8], TiledSmem<FAN, SEG, VB> &sm)
+{
+    constexpr int kPer = VB / kBwdWarps;         // views a warp stages per batch
+    constexpr int kBatches = kBwdGroup / VB;     // batches per prepared group
+    constexpr bool UNIT = MODE == kBwdUnit, RANGE = MODE == kBwdRange;
+    const Geo &g = p.g;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // eight lanes of a warp take a 4 x 4 square of pixels: their window loads
+    // fall in at most six consecutive 16-byte entries, which share no bank
+    const float dx = (float)(((lane >> 3) & 1) * 4 + (lane & 1) * 2) - 3.0f;   // the pair's middle
+    const float dy = (float)((lane >> 4) * 4 + ((lane >> 1) & 3)) - 3.5f;
+    // squares above the diagonal of a diagonal tile, or past the image, hold no pixel
+    const int xw = tx * kBwdTile + (warp & 1) * 8, yw = ty * kBwdTile + (warp >> 1) * 8;
+    const bool live = xw <= g.half && yw <= xw + 7;
+    // The geometry of a group of views: lanes 4 l .. 4 l + 3 of warp w take
+    // view (l / kPer) VB + w kPer + l % kPer of the group, one corner of the
+    // tile and one square each, and keep the view's detector span, so that the
+    // warp can stage its views of a batch without waiting for another.
+    int klo = 0, cnt = 0;
+    auto prepare = [&](int grp) {
+        const int l = lane >> 2, gv = (l / kPer) * VB + warp * kPer + l % kPer;
+        const BwdView &bv = p.view[min(v0 + grp * kBwdGroup + gv, v1 - 1)];
+        int bad = 0;
+        float lo = tile_corner(g, bv.cf, bv.sf, tx, ty, lane & 3, bad), hi = lo;
 #pragma unroll
-                    for (int q = 0; q < WIN; ++q) {
-                        if (FAN) {
-                            const float4 a = ra[FAN ? iv : 0][FAN ? k0 + q : 0];
-                            const float D = fmaf(a.y, du, fmaf(a.z, dv, a.x));
-                            const FootprintV f = staged_footprint(a, rb[FAN && !kBwdDerive ? iv : 0]
-                                                                        [FAN && !kBwdDerive ? k0 + q : 0]);
-                            w[q] = footprint_weight_v(D, qeK * a.y, f);
-                            if (FBP) w[q] *= fbpw;
-                        } else {
-                            w[q] = footprint_weight_v(rx[FAN ? 0 : iv][FAN ? 0 : k0 + q] + duw, Hpar, fpar);
-                        }
-                    }
+        for (int o = 1; o <= 2; o <<= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        const TileSpan sp = span_of(g, lo, hi, 0, kBwdPast);
+        klo = sp.klo;
+        BwdSquare q = square_view<FAN>(p, bv, tx, ty, lane & 3, klo, SEG);
+        const int un = (q.code & 255) + ((q.code >> 8) & 255) + (q.code >> 16);
+        cnt = max(sp.nseg, un);
 #pragma unroll
-                    for (int q = 0; q < WIN; ++q) {
-                        accumulate(w[q], seg[iv][0][k0 + q], seg[iv][1][k0 + q]);
-                        if (!FAN)
-                            accumulate(w[q], seg2[FAN ? 0 : iv][0][FAN ? 0 : k0 + q],
-                                       seg2[FAN ? 0 : iv][1][FAN ? 0 : k0 + q]);
-                    }
-                    continue;
-                }
-                float tlo, thi, qe = 0.0f;
-                if (FAN) {
-                    // the pixel's corner shadows (prj/cpuPrj.c:218-244), in
-                    // detector units; only which detector each edge falls in
-                    // matters here
-                    qe = t.qec - dv;
-                    const float A = t.A, B = t.B;
-                    if (p.fast_shadow) {
-                        // corner i at (u + du_i, qe + dq_i): t_i = K (u + du_i) / (1 + r dq_i)
-                        // ~ K (u + du_i - rho dq_i - r du_i dq_i), K = d r, rho = r u; the
-                        // corners pair up as u + c +- a1 and u - c +- a2
-                        const float r = __fdividef(1.0f, qe), rho = r * u, c = __fmul_rn(r, t.AB);
-                        const float a1 = fabsf(fmaf(rho, B, A)), a2 = fabsf(fmaf(-rho, A, B));
-                        const float K = dFs * r;
-                        tlo = K * (u + fminf(c - a1, -c - a2));
-                        thi = K * (u + fmaxf(c + a1, a2 - c));
-                    } else {
-                        const float t0 = __fdividef(dFs * (u - A), qe + B);
-                        const float t1 = __fdividef(dFs * (u + B), qe + A);
-                        const float t2 = __fdividef(dFs * (u + A), qe - B);
-                        const float t3 = __fdividef(dFs * (u - B), qe - A);
-                        tlo = fminf(fminf(t0, t1), fminf(t2, t3));
-                        thi = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3));
-                    }
-                } else {
-                    tlo = (u - t.hw) * invdS;
-                    thi = (u + t.hw) * invdS;
-                }
-                // float-to-int conversion saturates, so far-out shadows clamp
-                int dl = __float2int_rn(tlo);
-                int dr = __float2int_rn(thi);
-                dl = max(max(dl, -dmax) - t.klo, 0);
-                dr = min(min(dr, dmax) - t.klo, t.nseg - 1);
-                const float fbpw = FBP ? __fdividef(g.dF, qe) * __fdividef(g.dF, qe) : 1.0f;
-                const FootprintV fpar = FAN ? FootprintV{} : pfs[iv];
-                const float duw = FAN ? 0.0f : du * fpar.iw, Hpar = FAN ? 0.0f : hbpar * fpar.iw;
-                const float qeK = qe * Kb;
-                // the weight of staged detector kk for this pixel
-                auto weight = [&](const int kk) {
-                    float w;
-                    if (FAN) {
-                        const float4 a = ra[FAN ? iv : 0][FAN ? kk : 0];
-                        const float D = fmaf(a.y, du, fmaf(a.z, dv, a.x));
-                        const FootprintV f = staged_footprint(a, rb[FAN && !kBwdDerive ? iv : 0]
-                                                                    [FAN && !kBwdDerive ? kk : 0]);
-                        w = footprint_weight_v(D, qeK * a.y, f);
-                        if (FBP) w *= fbpw;
-                    } else {
-                        w = footprint_weight_v(rx[FAN ? 0 : iv][FAN ? 0 : kk] + duw, Hpar, fpar);
-                    }
-                    return w;
-                };
-                // two detectors per step, their shared-memory reads issued
-                // together (the second of an odd-length run re-reads dr and is
-                // skipped); per sum the order of the terms is unchanged
-                for (int kk = dl; kk <= dr; kk += 2) {
-                    const bool two = kk < dr;
-                    const int kb = two ? kk + 1 : kk;
-                    const float4 p0 = seg[iv][0][kk], p1 = seg[iv][1][kk];
-                    const float4 r0 = seg[iv][0][kb], r1 = seg[iv][1][kb];
-                    const float w0 = weight(kk);
-                    const float w1 = weight(kb);
-                    accumulate(w0, p0, p1);
-                    if (!FAN) accumulate(w0, seg2[FAN ? 0 : iv][0][FAN ? 0 : kk], seg2[FAN ? 0 : iv][1][FAN ? 0 : kk]);
-                    if (two) {
-                        accumulate(w1, r0, r1);
-                        if (!FAN) accumulate(w1, seg2[FAN ? 0 : iv][0][FAN ? 0 : kb], seg2[FAN ? 0 : iv][1][FAN ? 0 : kb]);
-                    }
-                }
+        for (int o = 1; o <= 2; o <<= 1) cnt = max(cnt, __shfl_xor_sync(0xffffffffu, cnt, o));
+        cnt = min(cnt, SEG + 2 * kBwdPast);   // the plan chose SEG above every span
+        q.hi = q.lo + (float)(cnt - un);
+        sm.sq[grp & 1][gv][lane & 3] = q;
+        if (!FAN && (lane & 3) == 0) sm.fp[grp & 1][FAN ? 0 : gv] = staged_footprint(q.c, q.s);
+    };
+    auto stage = [&](int b) {
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            const int l = (b % kBatches) * kPer + u, iv = warp * kPer + u;
+            const int k0 = __shfl_sync(0xffffffffu, klo, 4 * l), n = __shfl_sync(0xffffffffu, cnt, 4 * l);
+            const int i = v0 + b * VB + iv;
+            if (i >= v1) continue;
+            const float4 *sp = p.samp + (size_t)(i - vq) * 2 * p.Wp + (k0 + g.pC + kBwdTablePad);
+            const float4 *fp = p.foot + (size_t)(i - vq) * p.Wp + (k0 + g.pC + kBwdTablePad);
+            for (int kk = lane; kk < n; kk += 32) {
+                stage16(&sm.seg[b & 1][iv][0][kk], sp + kk);
+                stage16(&sm.seg[b & 1][iv][1][kk], sp + p.Wp + kk);
+                if (FAN) stage16(&sm.seg[b & 1][iv][FAN ? 2 : 0][kk], fp + kk);
             }
         }
-        __syncthreads();
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    const int nbatch = (v1 - v0 + VB - 1) / VB;
+    prepare(0);
+    stage(0);
+    for (int b = 0; b < nbatch; ++b) {
+        const bool more = b + 1 < nbatch;
+        if (more && (b + 1) % kBatches == 0) prepare((b + 1) / kBatches);
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();   // batch b and its geometry have landed; the other buffer is free
+        if (more) stage(b + 1);
+        if (!live) continue;
+        const int nb = min(VB, v1 - (v0 + b * VB)), gv = (b % kBatches) * VB, gb = (b / kBatches) & 1;
+        const BwdSquare *sq = &sm.sq[gb][gv][warp];
+        const float4 *fp = &sm.fp[gb][FAN ? 0 : gv], *seg = &sm.seg[b & 1][0][0][0];
+        for (int iv = 0; iv < nb; ++iv, sq += kBwdWarps, seg += (FAN ? 3 : 2) * (SEG + 2 * kBwdPast), fp += FAN ? 0 : 1) {
+            const BwdSquare q = *sq;
+            const float4 fpar = FAN ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : *fp;
+            const PairView v = pair_start<FAN>(p, q, dx, dy);
+            if (RANGE) {
+                pair_view_any<FAN, FBP, SEG, true>(p, q, v, seg, fpar, A, B, p.view[v0 + b * VB + iv],
+                                                   xw + (int)(dx + 3.0f), yw + (int)(dy + 3.5f));
+                continue;
+            }
+            switch (q.code) {
+            case 3 | (1 << 16): pair_view<FAN, FBP, SEG, UNIT, 3, 0, 1>(p, v, seg, fpar, A, B); break;
+            case 3 | (1 << 8): pair_view<FAN, FBP, SEG, UNIT, 3, 1, 0>(p, v, seg, fpar, A, B); break;
+            case 3: pair_view<FAN, FBP, SEG, UNIT, 3, 0, 0>(p, v, seg, fpar, A, B); break;
+            case 4 | (1 << 16): pair_view<FAN, FBP, SEG, UNIT, 4, 0, 1>(p, v, seg, fpar, A, B); break;
+            case 4 | (1 << 8): pair_view<FAN, FBP, SEG, UNIT, 4, 1, 0>(p, v, seg, fpar, A, B); break;
+            default: pair_view_any<FAN, FBP, SEG, false>(p, q, v, seg, fpar, A, B, *p.view, 0, 0); break;
+            }
+        }
     }
-    float S[8];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        S[2 * j] = S2[j].x;
-        S[2 * j + 1] = S2[j].y;
-    }
-    if (valid) write_octant(p, img, x, y, nimg, S);
+    __syncthreads();   // the buffers are free for what follows
 }
 
-#if CTPRJ_BWD_PAIR
-// ------------------------------------- backward, two pixels per thread
-//
-// Build-time variant (CTPRJ_BWD_PAIR=1) of the fan-beam window kernel: a
-// thread owns two horizontally adjacent pixels of the tile (128 threads per
-// 16 x 16 tile), and for each view reads the staged detectors of the union of
-// their two windows once: three to five detectors for two pixels instead of
-// six.  Each pixel takes a weight for every detector of the union; those
-// outside its own window lie beyond its shadow and add exactly zero, so the
-// sums equal the one-pixel kernel's.
-template <bool FBP, int SEG, int VB>
-__global__ void __launch_bounds__(kBwdTile * kBwdTile / 2, 6)
-k_backward_pair(const BwdParams p, const float *__restrict__ sino, float *__restrict__ img)
+// The sums of one tile over the base views [v0, v1)
+template <bool FAN, bool FBP, int SEG, int VB, int MODE>
+__device__ __forceinline__ void tile_sums(const BwdParams &p, int tx, int ty, int v0, int v1, float (&A)[8],
+                                          float (&B)[8], TiledSmem<FAN, SEG, VB> &sm)
 {
-    __shared__ TiledSmem<true, SEG, VB> sm;
+    const int Q = p.g.P / 4;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) A[j] = B[j] = 0.0f;
+    int turn = v0 / Q;
+    for (int v = v0; v < v1; ++turn) {
+        const int e = min(v1, (turn + 1) * Q);
+        quarter_sums<FAN, FBP, SEG, VB, MODE>(p, tx, ty, v, e, turn * Q, A, B, sm);
+        v = e;
+        rotate_sums(A);
+        rotate_sums(B);
+    }
+    for (; (turn & 3) != 0; ++turn) {   // a full turn: each image's sums are back in its place
+        rotate_sums(A);
+        rotate_sums(B);
+    }
+}
+
+// the octant pixel (x, y) of thread t of tile (tx, ty); it owns (x + 1, y) too
+__device__ __forceinline__ void pair_of(int t, int tx, int ty, int &x, int &y)
+{
+    const int lane = t & 31, warp = t >> 5;
+    x = tx * kBwdTile + (warp & 1) * 8 + ((lane >> 3) & 1) * 4 + (lane & 1) * 2;
+    y = ty * kBwdTile + (warp >> 1) * 8 + (lane >> 4) * 4 + ((lane >> 1) & 3);
+}
+
+// image j of octant pixel (x, y), if the pixel is one and the image its own
+// (the centre pixel's four images are one pixel, which image 3 is kept for)
+__device__ __forceinline__ void write_image(const BwdParams &p, float *__restrict__ img, int x, int y, int j, float sum)
+{
     const Geo &g = p.g;
-    const int tile = blockIdx.x;
-    if (p.zero_axes && tile == 0)
-        for (int i = threadIdx.x; i < g.n; i += blockDim.x) {
-            img[i] = 0.0f;
-            img[(size_t)i * g.n] = 0.0f;
-        }
+    if (x > g.half || y > x || (j >= 4 && (y == 0 || y == x)) || (x == 0 && j != 3)) return;
+    int gx, gy;
+    image_of(j, x, y, gx, gy);
+    const float val = sum * p.scale;
+    img[(size_t)(gy + g.h2) * g.n + (gx + g.h2)] = val / g.effRate;
+}
+
+// base views of part s of S
+__device__ __forceinline__ int part_begin(int nv, int s, int S) { return (int)((long long)nv * s / S); }
+
+__device__ __forceinline__ void zero_axes(const BwdParams &p, float *__restrict__ img)
+{
+    for (int i = threadIdx.x; i < p.g.n; i += blockDim.x) {
+        img[i] = 0.0f;
+        img[(size_t)i * p.g.n] = 0.0f;
+    }
+}
+
+// Staged backprojection, one tile per cluster of p.split blocks, each block
+// the views of its part.  The parts' sums meet in distributed shared memory:
+// every block adds up its share of the tile's pixel images over the parts, in
+// the parts' order, and writes it.
+template <bool FAN, bool FBP, int SEG, int VB, int MODE>
+__global__ void __launch_bounds__(kBwdThreads, CTPRJ_BWD_MINBLOCKS)
+k_backward_tiled(const BwdParams p, float *__restrict__ img)
+{
+    __shared__ union {
+        TiledSmem<FAN, SEG, VB> st;
+        float part[16][kBwdThreads];
+    } sm;
+    const int S = p.split, tile = blockIdx.x / S, s = blockIdx.x % S;
+    if (p.zero_axes && blockIdx.x == 0) zero_axes(p, img);
     int tx, ty;
     decode_tile(tile, tx, ty);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // a warp takes 8 x 8 pixels: lane (2 (lane % 4), lane / 4) and its right
-    // neighbour.  Eight lanes of a quarter-warp then span 8 x 2 pixels, whose
-    // windows fall in consecutive staged detectors (16 x 1 would spread them
-    // over twice as many entries and double the shared-memory wavefronts)
-    const int x1 = tx * kBwdTile + ((warp & 1) << 3) + ((lane & 3) << 1), x2 = x1 + 1;
-    const int y = ty * kBwdTile + ((warp >> 1) << 3) + (lane >> 2);
-    const bool valid1 = x1 <= g.half && y <= x1, valid2 = x2 <= g.half && y <= x2;
-    const double xc = tx * kBwdTile + 0.5 * (kBwdTile - 1), yc = ty * kBwdTile + 0.5 * (kBwdTile - 1);
-    const float dx1 = (float)(x1 - xc), dx2 = (float)(x2 - xc), dy = (float)(y - yc);
-    const float dFs = (float)((double)g.dF / g.dSize);
-    const float Kb = (float)(0.5 * g.beamWidth / g.d);
-    float S1[8], S2[8];
+    float A[8], B[8];
+    tile_sums<FAN, FBP, SEG, VB, MODE>(p, tx, ty, part_begin(p.nv, s, S), part_begin(p.nv, s + 1, S), A, B, sm.st);
+    int x, y;
+    if (S == 1) {
+        pair_of(threadIdx.x, tx, ty, x, y);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) S1[j] = S2[j] = 0.0f;
-#if CTPRJ_BWD_PAIR == 2
-    unsigned long long A1[4] = {0ull, 0ull, 0ull, 0ull}, A2[4] = {0ull, 0ull, 0ull, 0ull};
-#endif
+        for (int v = 0; v < 16; ++v) write_image(p, img, x + (v >> 3), y, v & 7, v < 8 ? A[v & 7] : B[v & 7]);
+        return;
+    }
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+#pragma unroll
+    for (int v = 0; v < 16; ++v) sm.part[v][threadIdx.x] = v < 8 ? A[v & 7] : B[v & 7];
+    cl.sync();
+    for (int e = s * kBwdThreads + threadIdx.x; e < 16 * kBwdThreads; e += S * kBwdThreads) {
+        const int v = e / kBwdThreads, t = e % kBwdThreads;
+        float sum = *cl.map_shared_rank(&sm.part[v][t], 0);
+        for (int q = 1; q < S; ++q) sum += *cl.map_shared_rank(&sm.part[v][t], q);
+        pair_of(t, tx, ty, x, y);
+        write_image(p, img, x + (v >> 3), y, v & 7, sum);
+    }
+    cl.sync();   // a block's sums stay until every block has read them
+}
 
-    for (int i0 = 0; i0 < p.nv; i0 += VB) {
-        const int nb = min(VB, p.nv - i0);
-        stage_batch<true, SEG, VB>(p, sino, tx, ty, xc, yc, i0, nb, sm);
-        for (int iv = 0; iv < nb; ++iv) {
-            const TileView &t = sm.tv[iv];
-            const float du1 = fmaf(dx1, t.cT, dy * t.sT), du2 = fmaf(dx2, t.cT, dy * t.sT);
-            const float dv1 = fmaf(dy, t.cT, -dx1 * t.sT), dv2 = fmaf(dy, t.cT, -dx2 * t.sT);
-            const float qe1 = t.qec - dv1, qe2 = t.qec - dv2;
-            const float tc1 = __fdividef(dFs * (t.ucf + du1), qe1);
-            const float tc2 = __fdividef(dFs * (t.ucf + du2), qe2);
-            // each pixel's window (staged units, unclipped) and their union, as
-            // wide as the widest of the warp; a detector of the union outside
-            // the staged span [0, nseg) lies beyond the tile's reach or the
-            // detector's edge and is skipped
-            const int k1 = __float2int_rn(tc1) - 1 - t.klo, k2 = __float2int_rn(tc2) - 1 - t.klo;
-            const int un = __reduce_max_sync(0xffffffffu, max(k1, k2) - min(k1, k2) + 3);
-            const int kb = min(k1, k2);
-            const float fbpw1 = FBP ? __fdividef(g.dF, qe1) * __fdividef(g.dF, qe1) : 1.0f;
-            const float fbpw2 = FBP ? __fdividef(g.dF, qe2) * __fdividef(g.dF, qe2) : 1.0f;
-            auto slot = [&](const int kk) {
-                if ((unsigned)kk >= (unsigned)t.nseg) return;
-                const float4 a = sm.ra[iv][kk];
-                const FootprintV f = staged_footprint(a, sm.rb[kBwdDerive ? 0 : iv][kBwdDerive ? 0 : kk]);
-                float w1 = footprint_weight_v(fmaf(a.y, du1, fmaf(a.z, dv1, a.x)), (qe1 * Kb) * a.y, f);
-                float w2 = footprint_weight_v(fmaf(a.y, du2, fmaf(a.z, dv2, a.x)), (qe2 * Kb) * a.y, f);
-                if (FBP) {
-                    w1 *= fbpw1;
-                    w2 *= fbpw2;
-                }
-#if CTPRJ_BWD_PAIR == 2
-                // packed: {S[2i], S[2i+1]} += {w, w} {p[2i], p[2i+1]}, one
-                // fma.rn.f32x2 for two sums (each lane rounds as fmaf)
-                const ulonglong2 q0 = *reinterpret_cast<const ulonglong2 *>(&sm.seg[iv][0][kk]);
-                const ulonglong2 q1 = *reinterpret_cast<const ulonglong2 *>(&sm.seg[iv][1][kk]);
-                unsigned long long ww1, ww2;
-                asm("mov.b64 %0, {%1, %1};" : "=l"(ww1) : "f"(w1));
-                asm("mov.b64 %0, {%1, %1};" : "=l"(ww2) : "f"(w2));
-                asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(A1[0]) : "l"(ww1), "l"(q0.x));
-                asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(A1[1]) : "l"(ww1), "l"(q0.y));
-                asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(A1[2]) : "l"(ww1), "l"(q1.x));
-                asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(A1[3]) : "l"(ww1), "l"(q1.y));
-                asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(A2[0]) : "l"(ww2), "l"(q0.x));
-                asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(A2[1]) : "l"(ww2), "l"(q0.y));
-                asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(A2[2]) : "l"(ww2), "l"(q1.x));
-                asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(A2[3]) : "l"(ww2), "l"(q1.y));
-#else
-                const float4 p0 = sm.seg[iv][0][kk], p1 = sm.seg[iv][1][kk];
-                S1[0] = fmaf(w1, p0.x, S1[0]);
-                S1[1] = fmaf(w1, p0.y, S1[1]);
-                S1[2] = fmaf(w1, p0.z, S1[2]);
-                S1[3] = fmaf(w1, p0.w, S1[3]);
-                S1[4] = fmaf(w1, p1.x, S1[4]);
-                S1[5] = fmaf(w1, p1.y, S1[5]);
-                S1[6] = fmaf(w1, p1.z, S1[6]);
-                S1[7] = fmaf(w1, p1.w, S1[7]);
-                S2[0] = fmaf(w2, p0.x, S2[0]);
-                S2[1] = fmaf(w2, p0.y, S2[1]);
-                S2[2] = fmaf(w2, p0.z, S2[2]);
-                S2[3] = fmaf(w2, p0.w, S2[3]);
-                S2[4] = fmaf(w2, p1.x, S2[4]);
-                S2[5] = fmaf(w2, p1.y, S2[5]);
-                S2[6] = fmaf(w2, p1.z, S2[6]);
-                S2[7] = fmaf(w2, p1.w, S2[7]);
-#endif
-            };
-            slot(kb);
-            slot(kb + 1);
-            slot(kb + 2);
-            if (un > 3) slot(kb + 3);
-            if (un > 4) slot(kb + 4);
+// One tile by one block, for the persistent launches: the parts one after the
+// other, added in the same order.
+template <bool FAN, bool FBP, int SEG, int VB, int MODE>
+__device__ __forceinline__ void backward_tile(const BwdParams &p, int tile, float *__restrict__ img,
+                                              TiledSmem<FAN, SEG, VB> &sm, float (&tot)[16][kBwdThreads])
+{
+    const int S = p.split;
+    if (p.zero_axes && tile == 0) zero_axes(p, img);
+    int tx, ty, x, y;
+    decode_tile(tile, tx, ty);
+    pair_of(threadIdx.x, tx, ty, x, y);
+    for (int s = 0; s < S; ++s) {
+        float A[8], B[8];
+        tile_sums<FAN, FBP, SEG, VB, MODE>(p, tx, ty, part_begin(p.nv, s, S), part_begin(p.nv, s + 1, S), A, B, sm);
+#pragma unroll
+        for (int v = 0; v < 16; ++v) {
+            const float a = v < 8 ? A[v & 7] : B[v & 7];
+            const float sum = s == 0 ? a : tot[v][threadIdx.x] + a;
+            if (s == S - 1) write_image(p, img, x + (v >> 3), y, v & 7, sum);
+            else tot[v][threadIdx.x] = sum;
         }
-        __syncthreads();
     }
-#if CTPRJ_BWD_PAIR == 2
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(S1[2 * j]), "=f"(S1[2 * j + 1]) : "l"(A1[j]));
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(S2[2 * j]), "=f"(S2[2 * j + 1]) : "l"(A2[j]));
-    }
-#endif
-    if (valid1) write_octant(p, img, x1, y, (y == 0 || y == x1) ? 4 : 8, S1);
-    if (valid2) write_octant(p, img, x2, y, (y == 0 || y == x2) ? 4 : 8, S2);
-}
-#endif
-
-template <bool FAN, bool FBP, int SEG, int VB, int WIN>
-__global__ void __launch_bounds__(kBwdTile * kBwdTile, CTPRJ_BWD_MINBLOCKS)
-k_backward_tiled(const BwdParams p, const float *__restrict__ sino, float *__restrict__ img)
-{
-    __shared__ TiledSmem<FAN, SEG, VB> sm;
-    backward_tile<FAN, FBP, SEG, VB, WIN>(p, blockIdx.x, sino, img, sm);
-}
-
-// upper bound of a pixel's shadow width in detectors, or 0 where none holds
-// (a fan source inside or next to the image)
-static double shadow_width_bound(const Geo &g)
-{
-    const double s2 = 1.4142135623730951;
-    if (!g.fan) return s2 / g.dSize;
-    const double R = (g.half + 1.0) * s2, d = g.d;
-    if (!(d > 2.0 * R)) return 0.0;
-    const double tg = R / (d - R);
-    return s2 * d / (d - R) * (1.0 + tg * tg) / g.dSize;
 }
 
 static BwdParams bwd_params(const ctprj_plan *pl, int fbp, float scale)
@@ -1722,36 +1780,14 @@ static BwdParams bwd_params(const ctprj_plan *pl, int fbp, float scale)
                   : scale;
     p.view = pl->d_bview;
     p.det = pl->d_det;
-    // The staged fan kernel may bound a pixel's shadow from 1/qe and a first-
-    // order expansion in (pixel half-diagonal) / qe instead of four divisions
-    // when the dropped second-order terms stay below 1e-4 detector: at most
-    //   K (h + 1) r^2 / 2,  r = 1 / (d - h),  K = d r / dSize,
-    // h = the image's half-diagonal.  Detectors that the exact and the
-    // bounded shadow disagree on lie within that distance of a shadow edge,
-    // where the footprint weight is of the order of its square.
-    p.fast_shadow = 0;
-    if (pl->g.fan) {
-        const double h = (pl->g.half + 0.5) * 1.4142135623730951 + 1.0;
-        const double d = pl->g.d;
-        if (d > 2.0 * h) {
-            const double r = 1.0 / (d - h), K = d * r / pl->g.dSize;
-            p.fast_shadow = K * (h + 1.0) * r * r * 0.5 <= 1e-4;
-        }
-    }
-    // Widest pixel shadow, in detectors: a unit pixel spans at most sqrt(2)
-    // across any ray; a fan magnifies that by d / qe <= d / (d - R) at the
-    // pixel nearest the source (R: the image corner's distance from the
-    // isocentre) and the detector's obliquity adds 1 + tan^2 of the fan
-    // angle, tan <= R / (d - R).  Below 1.9 detectors the three detectors
-    // centred on a pixel's projection hold its whole shadow.  (Below 2.85 the
-    // four from floor(tc) - 1 would, but at the 1024^2 fan configuration, the
-    // one such plan measured, four straight detectors ran slower than the
-    // range: 1.82 against 1.66 ms per polychromatic gradient iteration.)  A
-    // beam wider than the detector pitch (effectiveRate > 1) also reaches
-    // detectors outside the shadow, which the reference's range rule leaves
-    // out: such plans keep the per-pixel range.
-    const double width = shadow_width_bound(pl->g);
-    p.win = width > 0.0 && width <= 1.9 && pl->g.effRate <= 1.0f ? 3 : 0;
+    p.invd = pl->g.fan ? 1.0 / pl->g.d : 0.0;
+    p.cG = pl->g.fan ? (float)(pl->g.dSize / pl->g.d) : 0.0f;
+    p.invG = (float)(pl->g.fan ? pl->g.d / pl->g.dSize : 1.0 / pl->g.dSize);
+    p.split = pl->bwd_split > 0 ? pl->bwd_split : 1;
+    p.mode = pl->g.effRate == 1.0f ? kBwdUnit : (pl->g.effRate < 1.0f ? kBwdNarrow : kBwdRange);
+    p.Wp = pl->g.W + 2 * kBwdTablePad;
+    p.samp = pl->d_samp;
+    p.foot = pl->d_foot;
     return p;
 }
 
@@ -1760,39 +1796,99 @@ int backward_max_span(const ctprj_plan *pl, int *max_span)
 {
     const BwdParams p = bwd_params(pl, 0, 1.0f);
     const int tiles = p.tiles_side * (p.tiles_side + 1) / 2;
-    int *d = nullptr;
-    int st = cuda_error(cudaMalloc((void **)&d, sizeof(int)), "span scratch");
-    if (st) return st;
-    int h = 0;
-    if (!(st = cuda_error(cudaMemset(d, 0, sizeof(int)), "span reset"))) {
-        k_tile_span_max<<<296, 256>>>(p, tiles, d);
-        if (!(st = cuda_error(cudaGetLastError(), "span launch")))
-            st = cuda_error(cudaMemcpy(&h, d, sizeof(int), cudaMemcpyDeviceToHost), "span readback");
-    }
-    cudaFree(d);
-    *max_span = h;
+    int *d = (int *)pl->d_count;   // zero since the upload
+    int st;
+    k_tile_span_max<<<296, 256>>>(p, tiles, d);
+    if (!(st = cuda_error(cudaGetLastError(), "span launch")))
+        st = cuda_error(cudaMemcpy(max_span, d, sizeof(int), cudaMemcpyDeviceToHost), "span readback");
     return st;
 }
 
-template <int SEG, int VB, int WIN>
-static void launch_tiled_win(const BwdParams &p, bool fan, int fbp, dim3 grid, dim3 block,
-                             const float *sino, float *img, cudaStream_t s)
+// Parts the staged backprojection sums a plan's base views in: a cluster of as
+// many blocks per tile.  A small image has fewer tiles than the GPU holds blocks
+// (36 at 256^2 against 740), so its views are split to fill it; beyond one
+// wave a split evens out the last one.  The cost of a split weighs both: waves
+// of blocks (the last one half used on average) per part, and 2.5 % per part
+// for the blocks' start and the sums' meeting.  Measured, split 1 / 2 / 4 / 8:
+// 256^2 parallel 55 / 35 / 27 / 19 us, 512^2 fan 115 / 84 / 70 / 77,
+// 1024^2 fan 453 / 451 / 443 / 443, 2048^2 fan 3114 / 3006 / 3113 / 3171.
+int backward_split(const ctprj_plan *pl)
 {
-    if (fan) {
-        if (fbp) k_backward_tiled<true, true, SEG, VB, WIN><<<grid, block, 0, s>>>(p, sino, img);
-        else k_backward_tiled<true, false, SEG, VB, WIN><<<grid, block, 0, s>>>(p, sino, img);
-    } else {
-        if (fbp) k_backward_tiled<false, true, SEG, VB, WIN><<<grid, block, 0, s>>>(p, sino, img);
-        else k_backward_tiled<false, false, SEG, VB, WIN><<<grid, block, 0, s>>>(p, sino, img);
+    const int T = (pl->g.half + 1 + kBwdTile - 1) / kBwdTile, tiles = T * (T + 1) / 2;
+    int sms = 148, best = 1;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device);
+    const double slots = (double)CTPRJ_BWD_MINBLOCKS * sms;
+    double cost = 0.0;
+    for (int S = 1; S <= 8 && pl->nv >= 4 * S; S *= 2) {
+        const double x = tiles * S / slots, c = (x <= 1.0 ? 1.0 : x + 0.5) / S * (1.0 + 0.025 * S);
+        if (S == 1 || c < cost) {
+            cost = c;
+            best = S;
+        }
     }
+    return best;
+}
+
+// The tables of the staged backprojection in `mem`: the sample image (zero
+// beyond the detectors) and, for fan beam, the rays' footprints.
+size_t backward_table_bytes(const Geo &g)
+{
+    return sizeof(float4) * (size_t)(g.W + 2 * kBwdTablePad) * (size_t)(g.P / 4) * (g.fan ? 3 : 2);
+}
+
+int backward_tables(ctprj_plan *pl, float4 *mem)
+{
+    const BwdParams p = bwd_params(pl, 0, 1.0f);
+    const size_t samples = 2 * (size_t)(pl->g.P / 4) * p.Wp;
+    int st;
+    pl->d_samp = mem;
+    if ((st = cuda_error(cudaMemsetAsync(mem, 0, sizeof(float4) * samples, 0), "sample image"))) return st;
+    if (pl->g.fan) {
+        pl->d_foot = mem + samples;
+        const int Q = pl->g.P / 4;
+        k_footprints<<<dim3((p.Wp + 255) / 256, Q < 32768 ? Q : 32768), 256>>>(p, pl->d_foot);
+        st = cuda_error(cudaGetLastError(), "footprint table");
+    }
+    return st;
+}
+
+static void launch_samples(const BwdParams &p, const float *sino, cudaStream_t s)
+{
+    const int Q = p.g.P / 4;
+    k_samples<<<dim3((p.g.W + kSampThreads - 1) / kSampThreads, Q < 32768 ? Q : 32768), kSampThreads, 0, s>>>(p, sino);
+}
+
+template <bool FAN, bool FBP, int SEG, int VB, int MODE>
+static cudaError_t launch_tiled_t(const BwdParams &p, int tiles, float *img, cudaStream_t s)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(tiles * p.split);
+    c.blockDim = dim3(kBwdThreads);
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = p.split;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = p.split > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&c, k_backward_tiled<FAN, FBP, SEG, VB, MODE>, p, img);
+}
+
+template <bool FAN, bool FBP, int SEG, int VB>
+static cudaError_t launch_tiled_mode(const BwdParams &p, int tiles, float *img, cudaStream_t s)
+{
+    if (p.mode == kBwdRange) return launch_tiled_t<FAN, FBP, SEG, VB, kBwdRange>(p, tiles, img, s);
+    if (p.mode == kBwdNarrow) return launch_tiled_t<FAN, FBP, SEG, VB, kBwdNarrow>(p, tiles, img, s);
+    return launch_tiled_t<FAN, FBP, SEG, VB, kBwdUnit>(p, tiles, img, s);
 }
 
 template <int SEG, int VB>
-static void launch_tiled(const BwdParams &p, bool fan, int fbp, dim3 grid, dim3 block,
-                         const float *sino, float *img, cudaStream_t s)
+static cudaError_t launch_tiled(const BwdParams &p, int fbp, int tiles, float *img, cudaStream_t s)
 {
-    if (p.win == 3) launch_tiled_win<SEG, VB, 3>(p, fan, fbp, grid, block, sino, img, s);
-    else launch_tiled_win<SEG, VB, 0>(p, fan, fbp, grid, block, sino, img, s);
+    // the FBP distance weight is a fan's: parallel beam takes the plain kernel
+    if (!p.g.fan) return launch_tiled_mode<false, false, SEG, VB>(p, tiles, img, s);
+    return fbp ? launch_tiled_mode<true, true, SEG, VB>(p, tiles, img, s)
+               : launch_tiled_mode<true, false, SEG, VB>(p, tiles, img, s);
 }
 
 int launch_backward(const ctprj_plan *pl, const float *sino, float *img, int fbp,
@@ -1813,21 +1909,11 @@ int launch_backward(const ctprj_plan *pl, const float *sino, float *img, int fbp
             if (fan) k_backward<true, false, false><<<grid, block, 0, s>>>(p, sino, img, counter);
             else k_backward<false, false, false><<<grid, block, 0, s>>>(p, sino, img, counter);
         }
-#if CTPRJ_BWD_PAIR
-    } else if (fan && p.win == 3) {
-        const dim3 pblock(kBwdTile * kBwdTile / 2);
-        if (pl->bwd_seg <= 32) {
-            if (fbp) k_backward_pair<true, 32, 16><<<grid, pblock, 0, s>>>(p, sino, img);
-            else k_backward_pair<false, 32, 16><<<grid, pblock, 0, s>>>(p, sino, img);
-        } else {
-            if (fbp) k_backward_pair<true, 64, 8><<<grid, pblock, 0, s>>>(p, sino, img);
-            else k_backward_pair<false, 64, 8><<<grid, pblock, 0, s>>>(p, sino, img);
-        }
-#endif
-    } else if (pl->bwd_seg <= 32) {
-        launch_tiled<32, 16>(p, fan, fbp, grid, block, sino, img, s);
     } else {
-        launch_tiled<64, 8>(p, fan, fbp, grid, block, sino, img, s);
+        launch_samples(p, sino, s);
+        const cudaError_t e = pl->bwd_seg <= 32 ? launch_tiled<32, 8>(p, fbp, (int)grid.x, img, s)
+                                                : launch_tiled<64, 4>(p, fbp, (int)grid.x, img, s);
+        if (e != cudaSuccess) return cuda_error(e, "backward launch");
     }
     return cuda_error(cudaGetLastError(), "backward launch");
 }
@@ -1891,33 +1977,50 @@ __global__ void __launch_bounds__(32 * V, 4 * CTPRJ_FWD_MINBLOCKS / V) k_forward
     }
 }
 
-template <int SEG, int VB>
-constexpr size_t tiled_smem_bytes()
+// the sample images of every staged slice: item = a row of a slice
+__global__ void __launch_bounds__(kSampThreads) k_samples_batch(const BatchArgs a)
 {
-    return sizeof(TiledSmem<true, SEG, VB>) > sizeof(TiledSmem<false, SEG, VB>)
-               ? sizeof(TiledSmem<true, SEG, VB>)
-               : sizeof(TiledSmem<false, SEG, VB>);
+    for (long long e = blockIdx.x; e < a.stotal; e += gridDim.x) {
+        const int i = find_slot(a.sprefix, a.nslices, e);
+        const BatchSlice &sl = a.slices[i];
+        sample_row(sl.bp, sl.bsino, (int)(e - a.sprefix[i]), threadIdx.x, kSampThreads);
+    }
 }
 
-// one staged tile of a batch slice, with the slice's own window choice
+// shared memory of a persistent backprojection block, for either beam
 template <int SEG, int VB>
-__device__ __forceinline__ void batch_tile(const BatchSlice &sl, int tile, unsigned char *raw)
+struct BatchSmem {
+    union {
+        TiledSmem<true, SEG, VB> fan;
+        TiledSmem<false, SEG, VB> par;
+    } st;
+    float tot[16][kBwdThreads];
+};
+
+// one tile of a batch slice
+template <int SEG, int VB>
+__device__ __forceinline__ void batch_tile(const BatchSlice &sl, int tile, BatchSmem<SEG, VB> &sm)
 {
-    if (sl.bp.g.fan) {
-        auto &sm = *reinterpret_cast<TiledSmem<true, SEG, VB> *>(raw);
-        if (sl.bp.win == 3) backward_tile<true, false, SEG, VB, 3>(sl.bp, tile, sl.bsino, sl.bimg, sm);
-        else backward_tile<true, false, SEG, VB, 0>(sl.bp, tile, sl.bsino, sl.bimg, sm);
+    const BwdParams &p = sl.bp;
+    if (!sl.tiled) {
+        if (p.g.fan) backward_tile_direct<true>(p, tile, sl.bsino, sl.bimg);
+        else backward_tile_direct<false>(p, tile, sl.bsino, sl.bimg);
+    } else if (p.g.fan) {
+        if (p.mode == kBwdUnit) backward_tile<true, false, SEG, VB, kBwdUnit>(p, tile, sl.bimg, sm.st.fan, sm.tot);
+        else if (p.mode == kBwdNarrow) backward_tile<true, false, SEG, VB, kBwdNarrow>(p, tile, sl.bimg, sm.st.fan, sm.tot);
+        else backward_tile<true, false, SEG, VB, kBwdRange>(p, tile, sl.bimg, sm.st.fan, sm.tot);
     } else {
-        auto &sm = *reinterpret_cast<TiledSmem<false, SEG, VB> *>(raw);
-        if (sl.bp.win == 3) backward_tile<false, false, SEG, VB, 3>(sl.bp, tile, sl.bsino, sl.bimg, sm);
-        else backward_tile<false, false, SEG, VB, 0>(sl.bp, tile, sl.bsino, sl.bimg, sm);
+        if (p.mode == kBwdUnit) backward_tile<false, false, SEG, VB, kBwdUnit>(p, tile, sl.bimg, sm.st.par, sm.tot);
+        else if (p.mode == kBwdNarrow) backward_tile<false, false, SEG, VB, kBwdNarrow>(p, tile, sl.bimg, sm.st.par, sm.tot);
+        else backward_tile<false, false, SEG, VB, kBwdRange>(p, tile, sl.bimg, sm.st.par, sm.tot);
     }
 }
 
 template <int SEG, int VB>
-__global__ void __launch_bounds__(kBwdTile * kBwdTile, 4) k_backward_batch(const BatchArgs a)
+__global__ void __launch_bounds__(kBwdThreads, CTPRJ_BWD_MINBLOCKS) k_backward_batch(const BatchArgs a)
 {
-    __shared__ __align__(16) unsigned char raw[tiled_smem_bytes<SEG, VB>()];
+    extern __shared__ __align__(16) unsigned char batch_smem[];
+    BatchSmem<SEG, VB> &sm = *reinterpret_cast<BatchSmem<SEG, VB> *>(batch_smem);
     __shared__ long long slot;
     for (;;) {
         const long long item = next_item(a.counter, &slot);
@@ -1925,13 +2028,7 @@ __global__ void __launch_bounds__(kBwdTile * kBwdTile, 4) k_backward_batch(const
         const int i = find_slot(a.prefix, a.nslices, item);
         const BatchSlice &sl = a.slices[a.order[i]];
         const int tile = (int)(item - a.prefix[i]);
-        const bool fan = sl.bp.g.fan != 0;
-        if (sl.tiled) {
-            batch_tile<SEG, VB>(sl, tile, raw);
-        } else {
-            if (fan) backward_tile_direct<true>(sl.bp, tile, sl.bsino, sl.bimg);
-            else backward_tile_direct<false>(sl.bp, tile, sl.bsino, sl.bimg);
-        }
+        batch_tile<SEG, VB>(sl, tile, sm);
     }
 }
 
@@ -1953,60 +2050,90 @@ __device__ __forceinline__ unsigned long long global_ns()
     return t;
 }
 
+// Waits until word[0] reaches `want` (one thread), while the slice is not given
+// up; past the deadline the slice is.  Returns whether the word got there.
+__device__ __forceinline__ int wait_for(const volatile int *word, int want, int *status, unsigned long long timeout_ns)
+{
+    const unsigned long long t0 = global_ns();
+    for (;;) {
+        if (*word >= want) return 1;
+        if (*(volatile int *)status != 0) return 0;
+        if (global_ns() - t0 > timeout_ns) {
+            atomicExch(status, 1);
+            return 0;
+        }
+        __nanosleep(1000);
+    }
+}
+
+// Items of slice i: its sample rows, then its tiles.  A sample row waits for
+// the host's flag, a tile for the slice's rows, which blocks that are running
+// have taken before it (items are handed out in order).
 template <int SEG, int VB>
-__global__ void __launch_bounds__(kBwdTile * kBwdTile, 4)
-k_backward_stream(const BatchArgs a, const volatile int *__restrict__ ready,
+__global__ void __launch_bounds__(kBwdThreads, CTPRJ_BWD_MINBLOCKS)
+k_backward_stream(const BatchArgs a, const volatile int *__restrict__ ready, int *__restrict__ rows_done,
                   int *__restrict__ status, unsigned long long timeout_ns)
 {
-    __shared__ __align__(16) unsigned char raw[tiled_smem_bytes<SEG, VB>()];
+    extern __shared__ __align__(16) unsigned char batch_smem[];
+    BatchSmem<SEG, VB> &sm = *reinterpret_cast<BatchSmem<SEG, VB> *>(batch_smem);
     __shared__ long long slot;
     __shared__ int go;
     for (;;) {
         const long long item = next_item(a.counter, &slot);
-        if (item >= a.total) return;
-        const int i = find_slot(a.prefix, a.nslices, item);
-        const int s = a.order[i];
-        if (threadIdx.x == 0) {
-            int ok = 0;
-            if (((volatile int *)status)[s] == 0) {
-                const unsigned long long t0 = global_ns();
-                for (;;) {
-                    if (ready[s]) { ok = 1; break; }
-                    if (((volatile int *)status)[s] != 0) break;
-                    if (global_ns() - t0 > timeout_ns) {
-                        atomicExch(&status[s], 1);
-                        break;
-                    }
-                    __nanosleep(1000);
-                }
-            }
-            go = ok;
+        if (item >= a.total + a.stotal) return;
+        // items before slice position i: its tiles' and its sample rows' prefixes
+        int lo = 0, hi = a.nslices;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (a.prefix[mid] + a.oprefix[mid] <= item) lo = mid;
+            else hi = mid;
         }
+        const int i = lo, s = a.order[i];
+        const BatchSlice &sl = a.slices[s];
+        const int local = (int)(item - a.prefix[i] - a.oprefix[i]), rows = (int)(a.oprefix[i + 1] - a.oprefix[i]);
+        const bool sample = local < rows;
+        if (threadIdx.x == 0)
+            go = ((volatile int *)status)[s] == 0 &&
+                 (sample || rows == 0 ? wait_for(ready + s, 1, status + s, timeout_ns)
+                                      : wait_for(rows_done + s, rows, status + s, timeout_ns));
         __syncthreads();
         if (!go) continue;
-        __threadfence();   // the sinogram was published before the flag
-        const BatchSlice &sl = a.slices[s];
-        const int tile = (int)(item - a.prefix[i]);
-        const bool fan = sl.bp.g.fan != 0;
-        if (sl.tiled) {
-            batch_tile<SEG, VB>(sl, tile, raw);
+        __threadfence();   // the sinogram was published before the flag, the rows before their count
+        if (sample) {
+            sample_row(sl.bp, sl.bsino, local, threadIdx.x, kBwdThreads);
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0) atomicAdd(&rows_done[s], 1);
         } else {
-            if (fan) backward_tile_direct<true>(sl.bp, tile, sl.bsino, sl.bimg);
-            else backward_tile_direct<false>(sl.bp, tile, sl.bsino, sl.bimg);
+            batch_tile<SEG, VB>(sl, local - rows, sm);
         }
     }
 }
 
-int launch_backward_stream(const BatchArgs &a, int seg, int vb, int ctas, const int *ready,
+template <int SEG, int VB, class K>
+static int batch_kernel_smem(K kern)
+{
+    return cuda_error(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)sizeof(BatchSmem<SEG, VB>)), "batch shared memory");
+}
+
+template <int SEG, int VB>
+static int launch_stream_t(const BatchArgs &a, int ctas, const int *ready, int *rows_done, int *status,
+                           unsigned long long timeout_ns, cudaStream_t s)
+{
+    const int st = batch_kernel_smem<SEG, VB>(k_backward_stream<SEG, VB>);
+    if (st) return st;
+    k_backward_stream<SEG, VB><<<ctas, kBwdThreads, sizeof(BatchSmem<SEG, VB>), s>>>(a, ready, rows_done, status,
+                                                                                      timeout_ns);
+    return cuda_error(cudaGetLastError(), "streaming backward launch");
+}
+
+int launch_backward_stream(const BatchArgs &a, int seg, int vb, int ctas, const int *ready, int *rows_done,
                            int *status, unsigned long long timeout_ns, cudaStream_t s)
 {
-    if (seg <= 32 && vb == 16)
-        k_backward_stream<32, 16><<<ctas, 256, 0, s>>>(a, ready, status, timeout_ns);
-    else if (seg <= 32)
-        k_backward_stream<32, 8><<<ctas, 256, 0, s>>>(a, ready, status, timeout_ns);
-    else
-        k_backward_stream<64, 8><<<ctas, 256, 0, s>>>(a, ready, status, timeout_ns);
-    return cuda_error(cudaGetLastError(), "streaming backward launch");
+    if (seg > 32) return launch_stream_t<64, 4>(a, ctas, ready, rows_done, status, timeout_ns, s);
+    return vb == 16 ? launch_stream_t<32, 8>(a, ctas, ready, rows_done, status, timeout_ns, s)
+                    : launch_stream_t<32, 4>(a, ctas, ready, rows_done, status, timeout_ns, s);
 }
 
 int launch_quad_batch(const BatchArgs &a, cudaStream_t s)
@@ -2026,16 +2153,32 @@ int launch_forward_batch(const BatchArgs &a, int views, int ctas, cudaStream_t s
     return cuda_error(cudaGetLastError(), "batched forward launch");
 }
 
-int launch_backward_batch(const BatchArgs &a, int seg, int vb, int ctas, cudaStream_t s)
+template <int SEG, int VB>
+static int launch_backward_batch_t(const BatchArgs &a, int ctas, cudaStream_t s)
 {
-    if (seg <= 32 && vb == 16) k_backward_batch<32, 16><<<ctas, 256, 0, s>>>(a);
-    else if (seg <= 32) k_backward_batch<32, 8><<<ctas, 256, 0, s>>>(a);
-    else k_backward_batch<64, 8><<<ctas, 256, 0, s>>>(a);
+    const int st = batch_kernel_smem<SEG, VB>(k_backward_batch<SEG, VB>);
+    if (st) return st;
+    if (a.stotal > 0) k_samples_batch<<<(int)(a.stotal < 65536 ? a.stotal : 65536), kSampThreads, 0, s>>>(a);
+    k_backward_batch<SEG, VB><<<ctas, kBwdThreads, sizeof(BatchSmem<SEG, VB>), s>>>(a);
     return cuda_error(cudaGetLastError(), "batched backward launch");
 }
 
+int launch_backward_batch(const BatchArgs &a, int seg, int vb, int ctas, cudaStream_t s)
+{
+    if (seg > 32) return launch_backward_batch_t<64, 4>(a, ctas, s);
+    return vb == 16 ? launch_backward_batch_t<32, 8>(a, ctas, s) : launch_backward_batch_t<32, 4>(a, ctas, s);
+}
+
+template <int SEG, int VB>
+static cudaError_t batch_occupancy(int *per_sm)
+{
+    if (batch_kernel_smem<SEG, VB>(k_backward_batch<SEG, VB>)) return cudaGetLastError();
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_backward_batch<SEG, VB>, kBwdThreads,
+                                                         sizeof(BatchSmem<SEG, VB>));
+}
+
 // resident blocks per SM of a batched kernel: kind 0 forward (param = views),
-// kind 1 backward (param = seg * 100 + vb)
+// kind 1 backward (param = seg * 100 + views in its two staging buffers)
 int batch_max_ctas(int kind, int param, int *per_sm)
 {
     cudaError_t e;
@@ -2044,9 +2187,9 @@ int batch_max_ctas(int kind, int param, int *per_sm)
         else if (param == 8) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_forward_batch<8>, 256, 0);
         else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_forward_batch<4>, 128, 0);
     } else {
-        if (param == 3216) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_backward_batch<32, 16>, 256, 0);
-        else if (param == 3208) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_backward_batch<32, 8>, 256, 0);
-        else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_backward_batch<64, 8>, 256, 0);
+        if (param == 3216) e = batch_occupancy<32, 8>(per_sm);
+        else if (param == 3208) e = batch_occupancy<32, 4>(per_sm);
+        else e = batch_occupancy<64, 4>(per_sm);
     }
     return cuda_error(e, "occupancy query");
 }
