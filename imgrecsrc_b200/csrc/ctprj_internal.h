@@ -250,8 +250,10 @@ struct WvltProx {
     float *buf = nullptr;
     double *part = nullptr;
     void *state = nullptr;
+    size_t part_cap = 0;      // doubles in part
     int rows = 0, cols = 0;
     int alloc(int m, int n, cudaStream_t s);
+    int reserve_parts(size_t need, cudaStream_t s);
     void release(cudaStream_t s);
 };
 // alpha = argmin 1/2 |alpha - a|^2 + I(alpha >= 0) + u |W alpha|_1 by npg/admm.m

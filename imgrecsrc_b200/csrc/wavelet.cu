@@ -704,9 +704,21 @@ int WvltProx::alloc(int m, int n, cudaStream_t s)
         release(s);
         return st;
     }
+    part_cap = nparts;
     rows = m;
     cols = n;
     return CTPRJ_OK;
+}
+
+int WvltProx::reserve_parts(size_t need, cudaStream_t s)
+{
+    if (part_cap >= need) return CTPRJ_OK;
+    if (part) cudaFreeAsync(part, s);
+    part = nullptr;
+    part_cap = 0;
+    const int st = cuda_error(cudaMallocAsync((void **)&part, sizeof(double) * need, s), "wavelet partials");
+    if (!st) part_cap = need;
+    return st;
 }
 
 void WvltProx::release(cudaStream_t s)
@@ -714,6 +726,7 @@ void WvltProx::release(cudaStream_t s)
     if (buf) cudaFreeAsync(buf, s);
     if (part) cudaFreeAsync(part, s);
     if (state) cudaFreeAsync(state, s);
+    part_cap = 0;
     buf = nullptr;
     part = nullptr;
     state = nullptr;
@@ -728,6 +741,13 @@ int wvlt_admm(WvltProx &ws, const float *a, int rows, int cols, const double *h,
     int st;
     if ((st = check_args(a, alpha, rows, cols, h, lh, levels, &f))) return st;
     if ((st = ws.alloc(rows, cols, s))) return st;
+    // two-tap filters up to kHaarMaxLevels levels: the fused per-tile iteration
+    // (CTPRJ_WVLT_KERNEL=levels keeps the level-by-level passes, for comparison).
+    // It writes two partial sums per 2^levels x 2^levels tile: more of them, at
+    // few levels, than the level passes have blocks.
+    const char *kenv = getenv("CTPRJ_WVLT_KERNEL");
+    const bool fused = lh == 2 && levels <= kHaarMaxLevels && !(kenv && !strcmp(kenv, "levels"));
+    if (fused && (st = ws.reserve_parts(2 * (size_t)(rows >> levels) * (size_t)(cols >> levels), s))) return st;
     const size_t px = (size_t)rows * cols;
     float *scratch = ws.buf, *s0 = ws.buf + px / 2, *s1 = s0 + px, *nu = s1 + px;
     AdmmState *dst = (AdmmState *)ws.state;
@@ -753,10 +773,6 @@ int wvlt_admm(WvltProx &ws, const float *a, int rows, int cols, const double *h,
         return st;
     k_admm_start<<<1, 1, 0, s>>>(dst, tol, max_itr);
     const int nblocks = analysis_blocks(rows, cols, levels);
-    // two-tap filters up to kHaarMaxLevels levels: the fused per-tile iteration
-    // (CTPRJ_WVLT_KERNEL=levels keeps the level-by-level passes, for comparison)
-    const char *kenv = getenv("CTPRJ_WVLT_KERNEL");
-    const bool fused = lh == 2 && levels <= kHaarMaxLevels && !(kenv && !strcmp(kenv, "levels"));
     HaarArgs ha;
     ha.h0 = f.h[0];
     ha.h1 = f.h[1];
