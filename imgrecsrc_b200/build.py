@@ -8,7 +8,7 @@ Build-time variants (launch shapes and staging choices that were measured
 against the default) go to a library of their own, which the package loads
 when CTPRJ_LIB names it:
 
-    python -m imgrecsrc_b200.build -D CTPRJ_FWD_STAGE=1 -o imgrecsrc_b200/libctprj_fwdstage.so
+    python -m imgrecsrc_b200.build -D CTPRJ_FWD_MINBLOCKS=6 -o imgrecsrc_b200/libctprj_fwd6.so
 """
 import concurrent.futures
 import os

@@ -211,27 +211,251 @@ __device__ __forceinline__ FwdRay fwd_ray(const FwdParams &p, int b, int k)
 }
 
 // The rays of one forward block: V adjacent base views (one per warp) x 32
-// adjacent detectors; block (bx, by) of the per-plan grid.  Returns this
-// thread's Poisson terms in polychromatic mode.
-// Build-time variant CTPRJ_FWD_WARP_VIEWS = G > 1: a warp takes G adjacent
-// views x 32 / G detectors instead (measured slower: G unaligned pixel runs per
-// gather touch more 128-byte lines than one contiguous run of 32 rays).
-#ifndef CTPRJ_FWD_WARP_VIEWS
-#define CTPRJ_FWD_WARP_VIEWS 1
-#endif
-template <bool FAN, int MODE, int V>
-__device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int by,
-                                               const float4 *__restrict__ quad,
-                                               float *__restrict__ sino,
-                                               unsigned long long *__restrict__ counter,
-                                               const double *tab, const double *Ie)
+// adjacent detectors; block (bx, by) of the per-plan grid.  `part` of the rows
+// (of p.rsplit) is summed by this thread: its warp's, or, with kAllParts, every
+// part in turn, for the persistent launches.  The sums of the parts are added
+// in their order either way.  Returns this thread's likelihood terms in
+// polychromatic mode.
+constexpr int kAllParts = -1;
+
+// The rows of one part for one ray: S += the eight images' sums.  Row y reads
+// the quad row |y|:
+//   q[x] = {I(x, |y|), I(x, -|y|), I(|y|, x), I(-|y|, x)},
+// so that for y >= 0 the eight sums take, per pixel x,
+//   S0 += I(x, y), S6 += I(-x, y), S4 += I(x, -y), S2 += I(-x, -y),
+//   S5 += I(y, x), S3 += I(y, -x), S1 += I(-y, x), S7 += I(-y, -x)
+// from q[x] and q[-x]; for y < 0 the pairs of components swap.
+// wcode: 3 / 4: window of 3 / 4 pixels; 5: bounded range loop (one for the warp).
+template <bool FAN, int MODE>
+__device__ __forceinline__ void march_rows(const Geo &g, const FwdRay &ray, int wcode, int ytop, int ybot,
+                                           const float4 *__restrict__ quad, float (&S)[8], unsigned long long &nz)
+{
+    const double cR = ray.cR, sR = ray.sR, off = ray.off;
+    const float Alf = ray.Al, Slf = ray.Sl, Arf = ray.Ar, Srf = ray.Sr;
+    const float cTf = ray.cT, sTf = ray.sT, bwc = ray.bwc, kbw = ray.kbw;
+    const FootprintV fp = ray.fp;
+    const float cRw = ray.cRw, dhbw = ray.dhbw;
+    const int half = g.half;
+    const int QW = 2 * half + 1;
+    auto march_row = [&](const int y, const float4 *__restrict__ q, auto neg) {
+        constexpr bool NEG = decltype(neg)::value;
+        const float yf = (float)y;
+        const float xl = fmaf(-yf, Slf, Alf), xr = fmaf(-yf, Srf, Arf);
+        // nearest pixel to each edge; exact half-way ties (where the
+        // reference rounds away from zero) only decide pixels whose
+        // footprint just touches the beam edge, with weight zero; the
+        // conversion saturates, so far-out edges clamp
+        const int x0 = max(__float2int_rn(xl), -half);
+        const int x1 = min(__float2int_rn(xr), half);
+        if (x0 > x1) return;
+        // distance of pixel (x0, y) from the ray, in FP64 then rounded;
+        // distances and half beam widths in units of the footprint's ramp
+        const float r0 = (float)fma((double)x0, cR, fma((double)y, sR, -off)) * fp.iw;
+        const float hb0 = (FAN ? 0.5f * fmaf(fmaf((float)x0, sTf, -yf * cTf), kbw, bwc)
+                               : 0.5f * g.beamWidthF) * fp.iw;
+        auto accumulate = [&](const float w, const float4 pp, const float4 pm) {
+            const float ap = NEG ? pp.y : pp.x, am = NEG ? pm.y : pm.x;   // I(+-x, y)
+            const float bp = NEG ? pp.x : pp.y, bm = NEG ? pm.x : pm.y;   // I(+-x, -y)
+            const float cp = NEG ? pp.w : pp.z, cm = NEG ? pm.w : pm.z;   // I(y, +-x)
+            const float dp = NEG ? pp.z : pp.w, dm = NEG ? pm.z : pm.w;   // I(-y, +-x)
+            S[0] = fmaf(w, ap, S[0]);
+            S[6] = fmaf(w, am, S[6]);
+            S[4] = fmaf(w, bp, S[4]);
+            S[2] = fmaf(w, bm, S[2]);
+            S[5] = fmaf(w, cp, S[5]);
+            S[3] = fmaf(w, cm, S[3]);
+            S[1] = fmaf(w, dp, S[1]);
+            S[7] = fmaf(w, dm, S[7]);
+        };
+        // Pixel x0 + j sits at D = fma(j, cRw, r0) (j even) or that of
+        // j - 1 plus cRw (j odd), and likewise for H.  At unit beam width
+        // a ray crosses one to three pixels of a row below 37 degrees of
+        // obliquity and two to four above, so one straight-line step takes
+        // the first three pixels, their gathers issued together and each
+        // predicated on the pixel being in the run (a lane past its run
+        // sends no request), and single steps the rest; per sum the order
+        // of the terms is x0, x0 + 1, ...
+        auto coef = [&](const int j, float &D, float &H) {
+            const float je = (float)(j & ~1);
+            D = fmaf(je, cRw, r0);
+            H = FAN ? fmaf(je, dhbw, hb0) : hb0;
+            if (j & 1) {
+                D += cRw;
+                if (FAN) H += dhbw;
+            }
+        };
+        {
+            const bool p1 = x0 < x1, p2 = x0 + 1 < x1;
+            float D0, H0, D1, H1, D2, H2;
+            coef(0, D0, H0);
+            coef(1, D1, H1);
+            coef(2, D2, H2);
+            if (MODE == kModeCount) {
+                nz += (footprint_weight_v(D0, H0, fp) != 0.0f);
+                if (p1) nz += (footprint_weight_v(D1, H1, fp) != 0.0f);
+                if (p2) nz += (footprint_weight_v(D2, H2, fp) != 0.0f);
+            } else {
+                const float4 pp0 = __ldg(q + x0), pm0 = __ldg(q - x0);
+                float4 pp1 = {}, pm1 = {}, pp2 = {}, pm2 = {};
+                if (p1) {
+                    pp1 = __ldg(q + x0 + 1);
+                    pm1 = __ldg(q - x0 - 1);
+                }
+                if (p2) {
+                    pp2 = __ldg(q + x0 + 2);
+                    pm2 = __ldg(q - x0 - 2);
+                }
+                accumulate(footprint_weight_v(D0, H0, fp), pp0, pm0);
+                if (p1) accumulate(footprint_weight_v(D1, H1, fp), pp1, pm1);
+                if (p2) accumulate(footprint_weight_v(D2, H2, fp), pp2, pm2);
+            }
+        }
+        for (int x = x0 + 3; x <= x1; ++x) {
+            float D, H;
+            coef(x - x0, D, H);
+            if (MODE == kModeCount) {
+                nz += (footprint_weight_v(D, H, fp) != 0.0f);
+                continue;
+            }
+            accumulate(footprint_weight_v(D, H, fp), __ldg(q + x), __ldg(q - x));
+        }
+    };
+    // The fixed-window march (plain and polychromatic modes).  Where a
+    // ray's run across a row is always narrower than 1.95 (2.95) pixels,
+    // the pixels of the run lie within the 3 (4) centred on the ray's
+    // crossing xc = (xl + xr) / 2: they are summed straight, without the
+    // run's bounds.  A pixel of the window outside the run lies beyond
+    // the beam and adds a weight of exactly zero (for fan beams: below
+    // 1e-7 within ~1e-4 pixel of a run edge, where the footprint and the
+    // beam edges differ).  The window is chosen per warp (the widest any
+    // of its rays needs), so the warp stays converged.
+    const float Acf = 0.5f * (Alf + Arf), Scf = 0.5f * (Slf + Srf);
+    auto march_win = [&](const int y, const float4 *__restrict__ q, auto neg, auto wn) {
+        constexpr bool NEG = decltype(neg)::value;
+        constexpr int WN = decltype(wn)::value;
+        const float yf = (float)y;
+        const float xc = fmaf(-yf, Scf, Acf);
+        // rows whose run misses the image (the run lies within xc +- 1.5)
+        if (xc < -(float)half - 2.0f || xc > (float)half + 2.0f) return;
+        int xs = (WN == 3 ? __float2int_rn(xc) : __float2int_rd(xc)) - 1;
+        xs = min(max(xs, -half), half - (WN - 1));
+        const float r0 = (float)fma((double)xs, cR, fma((double)y, sR, -off)) * fp.iw;
+        const float hb0 = (FAN ? 0.5f * fmaf(fmaf((float)xs, sTf, -yf * cTf), kbw, bwc)
+                               : 0.5f * g.beamWidthF) * fp.iw;
+        float4 pp[WN], pm[WN];
+#pragma unroll
+        for (int j = 0; j < WN; ++j) {
+            pp[j] = __ldg(q + xs + j);
+            pm[j] = __ldg(q - xs - j);
+        }
+#pragma unroll
+        for (int j = 0; j < WN; ++j) {
+            const float D = fmaf((float)j, cRw, r0);
+            const float H = FAN ? fmaf((float)j, dhbw, hb0) : hb0;
+            const float w = footprint_weight_v(D, H, fp);
+            const float ap = NEG ? pp[j].y : pp[j].x, am = NEG ? pm[j].y : pm[j].x;
+            const float bp = NEG ? pp[j].x : pp[j].y, bm = NEG ? pm[j].x : pm[j].y;
+            const float cp = NEG ? pp[j].w : pp[j].z, cm = NEG ? pm[j].w : pm[j].z;
+            const float dp = NEG ? pp[j].z : pp[j].w, dm = NEG ? pm[j].z : pm[j].w;
+            S[0] = fmaf(w, ap, S[0]);
+            S[6] = fmaf(w, am, S[6]);
+            S[4] = fmaf(w, bp, S[4]);
+            S[2] = fmaf(w, bm, S[2]);
+            S[5] = fmaf(w, cp, S[5]);
+            S[3] = fmaf(w, cm, S[3]);
+            S[1] = fmaf(w, dp, S[1]);
+            S[7] = fmaf(w, dm, S[7]);
+        }
+    };
+    const float4 *q = quad + (size_t)max(ytop, 0) * QW + half;   // row |y|, x = 0
+    const int ypos = max(ybot, 0), yneg = min(ytop, -1);
+    if (wcode == 3) {
+        for (int y = ytop; y >= ypos; --y, q -= QW)
+            march_win(y, q, std::false_type{}, std::integral_constant<int, 3>{});
+    } else if (wcode == 4) {
+        for (int y = ytop; y >= ypos; --y, q -= QW)
+            march_win(y, q, std::false_type{}, std::integral_constant<int, 4>{});
+    } else {
+        for (int y = ytop; y >= ypos; --y, q -= QW) march_row(y, q, std::false_type{});
+    }
+    q = quad + (size_t)(-yneg) * QW + half;
+    if (wcode == 3) {
+        for (int y = yneg; y >= ybot; --y, q += QW)
+            march_win(y, q, std::true_type{}, std::integral_constant<int, 3>{});
+    } else if (wcode == 4) {
+        for (int y = yneg; y >= ybot; --y, q += QW)
+            march_win(y, q, std::true_type{}, std::integral_constant<int, 4>{});
+    } else {
+        for (int y = yneg; y >= ybot; --y, q += QW) march_row(y, q, std::true_type{});
+    }
+}
+
+// rows [top, bottom] of part s of R, of the image's 2 half + 1
+__device__ __forceinline__ void part_rows(int half, int s, int R, int &top, int &bottom)
+{
+    const int M = 2 * half + 1;
+    top = half - (int)((long long)M * s / R);
+    bottom = half - (int)((long long)M * (s + 1) / R) + 1;
+}
+
+// Narrows [top, bottom] to the rows in which a ray of the warp can meet the
+// image: its crossing xc = Ac - y Sc is affine in y, and rows with |xc| > half
+// + 2 are skipped anyway; two rows of margin cover the division's rounding.
+// Every lane of the warp takes part, lanes without a ray with no rows.
+__device__ __forceinline__ void clip_rows(const FwdRay &ray, bool live, int half, int &top, int &bottom)
+{
+    const float A = 0.5f * (ray.Al + ray.Ar), S = 0.5f * (ray.Sl + ray.Sr), lim = (float)half + 2.0f;
+    float lo = (float)-half, hi = (float)half;
+    if (fabsf(S) > 1e-6f) {
+        const float a = __fdividef(A - lim, S), b = __fdividef(A + lim, S);
+        lo = fmaxf(lo, fminf(a, b) - 2.0f);
+        hi = fminf(hi, fmaxf(a, b) + 2.0f);
+    } else if (fabsf(A) > lim + 1.0f) {
+        lo = 1.0f;
+        hi = 0.0f;
+    }
+    const int ylo = live && lo <= hi ? __float2int_rd(lo) : INT_MAX, yhi = live && lo <= hi ? __float2int_ru(hi) : INT_MIN;
+    bottom = max(bottom, __reduce_min_sync(0xffffffffu, ylo));
+    top = min(top, __reduce_max_sync(0xffffffffu, yhi));
+}
+
+// Stores image j's sum of ray (view b, detector k), scaled, or takes it through
+// the polychromatic epilogue: to its sinogram row and detector, and for
+// parallel beam to the point-reflected detector of the view that image j ^ 2
+// belongs to (prj/cpuPrj.c:403-460), which is the one kept where the two
+// coincide (the central detector).  Returns the likelihood terms.
+template <bool FAN, int MODE>
+__device__ __forceinline__ double put_image(const FwdParams &p, int b, int k, int j, float sum,
+                                            float *__restrict__ sino, const double *tab, const double *Ie)
 {
     const Geo &g = p.g;
-    constexpr int G = V < CTPRJ_FWD_WARP_VIEWS ? V : CTPRJ_FWD_WARP_VIEWS, D = 32 / G;
+    const int det = j < 4 ? k : 2 * g.pC - k, det2 = 2 * g.pC - det;
+    const int v = p.view[b].out[j], v2 = FAN ? -1 : p.view[b].out[j ^ 2];
+    const float val = sum / g.effRate;
+    double f = 0.0;
+    auto put = [&](size_t idx) {
+        if constexpr (MODE == kModeBhc) {
+            f += bhc_entry(p.bhc, tab, Ie, val, idx);
+            if (p.bhc.proj_out) p.bhc.proj_out[idx] = val;
+        } else {
+            sino[idx] = val;
+        }
+    };
+    if (v >= 0 && (FAN || det2 != det)) put((size_t)v * g.W + det);
+    if (!FAN && v2 >= 0) put((size_t)v2 * g.W + det2);
+    return f;
+}
+
+template <bool FAN, int MODE, int V, int R>
+__device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int by, const float4 *__restrict__ quad,
+                                               float *__restrict__ sino, unsigned long long *__restrict__ counter,
+                                               const double *tab, const double *Ie, float *parts)
+{
+    const Geo &g = p.g;
     const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
-    const int b = bx * V + (warp / G) * G + lane / D;
-    const int r = by * 32 + (warp % G) * D + lane % D;
-    double fsum = 0.0;            // polychromatic mode: this thread's Poisson terms
+    const int b = bx * V + warp % V, seg = warp / V;
+    const int r = by * 32 + lane;
+    double fsum = 0.0;            // polychromatic mode: this thread's likelihood terms
     // detector 0 of an even-width sinogram: no ray, zero projection
     if (MODE != kModeCount && p.zero_col0 && bx == 0 && by == 0)
         for (int v = threadIdx.x; v < g.np; v += blockDim.x) {
@@ -243,12 +467,11 @@ __device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int b
             }
         }
 
-    // The window a warp marches with (below) is the widest any of its rays
-    // needs: xr - xl is affine in y, so a ray's widest run is at the first or
-    // the last row.  Every lane of the (full) warp takes part in the maximum,
-    // lanes without a ray with 0, so the choice depends on the warp's rays
-    // alone and a batched launch makes the same one (the variant with G views
-    // per warp takes it per view, over that view's lanes).
+    // The window a warp marches with is the widest any of its rays needs: xr -
+    // xl is affine in y, so a ray's widest run is at the first or the last row.
+    // Every lane of the (full) warp takes part in the maximum, lanes without a
+    // ray with 0, so the choice depends on the warp's rays alone and a batched
+    // launch makes the same one.
     const bool live = b < p.nb && r < p.nk;
     const int k = p.k0 + r;
     FwdRay ray = {};
@@ -262,275 +485,61 @@ __device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int b
             wcode = wmax < 1.95f ? 3 : (wmax < 2.95f ? 4 : 5);
         }
     }
-    if (G == 1) {
-        wcode = __reduce_max_sync(0xffffffffu, wcode);
-    } else {
-#pragma unroll
-        for (int o = 1; o < D; o <<= 1) wcode = max(wcode, __shfl_xor_sync(0xffffffffu, wcode, o));
-    }
-    if (live) {
-        const double cR = ray.cR, sR = ray.sR, off = ray.off;
-        const float Alf = ray.Al, Slf = ray.Sl, Arf = ray.Ar, Srf = ray.Sr;
-        const float cTf = ray.cT, sTf = ray.sT, bwc = ray.bwc, kbw = ray.kbw;
-        const FootprintV fp = ray.fp;
-        const float cRw = ray.cRw, dhbw = ray.dhbw;
-
-        const int half = g.half;
-        float S[8];
+    wcode = __reduce_max_sync(0xffffffffu, wcode);
+    float S[8];
+    unsigned long long nz = 0;
+    auto rows_of = [&](int s) {
+        int top, bottom;
+        part_rows(g.half, s, p.rsplit, top, bottom);
+        if (wcode != 5) clip_rows(ray, live, g.half, top, bottom);
 #pragma unroll
         for (int j = 0; j < 8; ++j) S[j] = 0.0f;
-        unsigned long long nz = 0;
-
-        // The march down the rows.  Row y reads the quad row |y|:
-        // q[x] = {I(x, |y|), I(x, -|y|), I(|y|, x), I(-|y|, x)}, so that for
-        // y >= 0 the eight sums take, per pixel x,
-        //   S0 += I(x, y), S6 += I(-x, y), S4 += I(x, -y), S2 += I(-x, -y),
-        //   S5 += I(y, x), S3 += I(y, -x), S1 += I(-y, x), S7 += I(-y, -x)
-        // from q[x] and q[-x]; for y < 0 the pairs of components swap.
-        const int QW = 2 * half + 1;
-        auto march_row = [&](const int y, const float4 *__restrict__ q, auto neg) {
-            constexpr bool NEG = decltype(neg)::value;
-            const float yf = (float)y;
-            const float xl = fmaf(-yf, Slf, Alf), xr = fmaf(-yf, Srf, Arf);
-            // nearest pixel to each edge; exact half-way ties (where the
-            // reference rounds away from zero) only decide pixels whose
-            // footprint just touches the beam edge, with weight zero; the
-            // conversion saturates, so far-out edges clamp
-            const int x0 = max(__float2int_rn(xl), -half);
-            const int x1 = min(__float2int_rn(xr), half);
-            if (x0 > x1) return;
-            // distance of pixel (x0, y) from the ray, in FP64 then rounded;
-            // distances and half beam widths in units of the footprint's ramp
-            const float r0 = (float)fma((double)x0, cR, fma((double)y, sR, -off)) * fp.iw;
-            const float hb0 = (FAN ? 0.5f * fmaf(fmaf((float)x0, sTf, -yf * cTf), kbw, bwc)
-                                   : 0.5f * g.beamWidthF) * fp.iw;
-            auto accumulate = [&](const float w, const float4 pp, const float4 pm) {
-                const float ap = NEG ? pp.y : pp.x, am = NEG ? pm.y : pm.x;   // I(+-x, y)
-                const float bp = NEG ? pp.x : pp.y, bm = NEG ? pm.x : pm.y;   // I(+-x, -y)
-                const float cp = NEG ? pp.w : pp.z, cm = NEG ? pm.w : pm.z;   // I(y, +-x)
-                const float dp = NEG ? pp.z : pp.w, dm = NEG ? pm.z : pm.w;   // I(-y, +-x)
-                S[0] = fmaf(w, ap, S[0]);
-                S[6] = fmaf(w, am, S[6]);
-                S[4] = fmaf(w, bp, S[4]);
-                S[2] = fmaf(w, bm, S[2]);
-                S[5] = fmaf(w, cp, S[5]);
-                S[3] = fmaf(w, cm, S[3]);
-                S[1] = fmaf(w, dp, S[1]);
-                S[7] = fmaf(w, dm, S[7]);
-            };
-            // Pixel x0 + j sits at D = fma(j, cRw, r0) (j even) or that of
-            // j - 1 plus cRw (j odd), and likewise for H.  At unit beam width
-            // a ray crosses one to three pixels of a row below 37 degrees of
-            // obliquity and two to four above, so one straight-line step takes
-            // the first three pixels, their gathers issued together and each
-            // predicated on the pixel being in the run (a lane past its run
-            // sends no request), and single steps the rest; per sum the order
-            // of the terms is x0, x0 + 1, ...
-            auto coef = [&](const int j, float &D, float &H) {
-                const float je = (float)(j & ~1);
-                D = fmaf(je, cRw, r0);
-                H = FAN ? fmaf(je, dhbw, hb0) : hb0;
-                if (j & 1) {
-                    D += cRw;
-                    if (FAN) H += dhbw;
-                }
-            };
-            {
-                const bool p1 = x0 < x1, p2 = x0 + 1 < x1;
-                float D0, H0, D1, H1, D2, H2;
-                coef(0, D0, H0);
-                coef(1, D1, H1);
-                coef(2, D2, H2);
-                if (MODE == kModeCount) {
-                    nz += (footprint_weight_v(D0, H0, fp) != 0.0f);
-                    if (p1) nz += (footprint_weight_v(D1, H1, fp) != 0.0f);
-                    if (p2) nz += (footprint_weight_v(D2, H2, fp) != 0.0f);
-                } else {
-                    const float4 pp0 = __ldg(q + x0), pm0 = __ldg(q - x0);
-                    float4 pp1 = {}, pm1 = {}, pp2 = {}, pm2 = {};
-                    if (p1) {
-                        pp1 = __ldg(q + x0 + 1);
-                        pm1 = __ldg(q - x0 - 1);
-                    }
-                    if (p2) {
-                        pp2 = __ldg(q + x0 + 2);
-                        pm2 = __ldg(q - x0 - 2);
-                    }
-                    accumulate(footprint_weight_v(D0, H0, fp), pp0, pm0);
-                    if (p1) accumulate(footprint_weight_v(D1, H1, fp), pp1, pm1);
-                    if (p2) accumulate(footprint_weight_v(D2, H2, fp), pp2, pm2);
-                }
-            }
-            for (int x = x0 + 3; x <= x1; ++x) {
-                float D, H;
-                coef(x - x0, D, H);
-                if (MODE == kModeCount) {
-                    nz += (footprint_weight_v(D, H, fp) != 0.0f);
-                    continue;
-                }
-                accumulate(footprint_weight_v(D, H, fp), __ldg(q + x), __ldg(q - x));
-            }
-        };
-        // The fixed-window march (plain and polychromatic modes).  Where a
-        // ray's run across a row is always narrower than 1.95 (2.95) pixels,
-        // the pixels of the run lie within the 3 (4) centred on the ray's
-        // crossing xc = (xl + xr) / 2: they are summed straight, without the
-        // run's bounds.  A pixel of the window outside the run lies beyond
-        // the beam and adds a weight of exactly zero (for fan beams: below
-        // 1e-7 within ~1e-4 pixel of a run edge, where the footprint and the
-        // beam edges differ).  The window is chosen per warp (the widest any
-        // of its rays needs), so the warp stays converged.
-        const float Acf = 0.5f * (Alf + Arf), Scf = 0.5f * (Slf + Srf);
-        auto march_win = [&](const int y, const float4 *__restrict__ q, auto neg, auto wn) {
-            constexpr bool NEG = decltype(neg)::value;
-            constexpr int WN = decltype(wn)::value;
-            const float yf = (float)y;
-            const float xc = fmaf(-yf, Scf, Acf);
-            // rows whose run misses the image (the run lies within xc +- 1.5)
-            if (xc < -(float)half - 2.0f || xc > (float)half + 2.0f) return;
-            int xs = (WN == 3 ? __float2int_rn(xc) : __float2int_rd(xc)) - 1;
-            xs = min(max(xs, -half), half - (WN - 1));
-#if CTPRJ_FWD_PREFETCH
-            // Build-time variant: ask L1 for the quad lines this ray will read
-            // CTPRJ_FWD_PREFETCH rows further on (at this row's x: the run
-            // moves less than a pixel per row), where that row is in the image
-            {
-                constexpr int PD = CTPRJ_FWD_PREFETCH;
-                if (NEG ? PD - y <= half : y - PD >= 0) {
-                    const float4 *qa = NEG ? q + PD * QW : q - PD * QW;
-                    asm volatile("prefetch.L1 [%0];" ::"l"(qa + xs));
-                    asm volatile("prefetch.L1 [%0];" ::"l"(qa - xs));
-                }
-            }
-#endif
-            const float r0 = (float)fma((double)xs, cR, fma((double)y, sR, -off)) * fp.iw;
-            const float hb0 = (FAN ? 0.5f * fmaf(fmaf((float)xs, sTf, -yf * cTf), kbw, bwc)
-                                   : 0.5f * g.beamWidthF) * fp.iw;
-            float4 pp[WN], pm[WN];
+        if (live && top >= bottom) march_rows<FAN, MODE>(g, ray, wcode, top, bottom, quad, S, nz);
+    };
+    if constexpr (R > 1) {
+        // a part of the rows per warp; each warp then takes its share of the images
+        rows_of(seg);
+        float(*ps)[8][32] = reinterpret_cast<float(*)[8][32]>(parts);
 #pragma unroll
-            for (int j = 0; j < WN; ++j) {
-                pp[j] = __ldg(q + xs + j);
-                pm[j] = __ldg(q - xs - j);
-            }
+        for (int j = 0; j < 8; ++j) ps[warp][j][lane] = S[j];
+        __syncthreads();
+        if (live) {
+#pragma unroll 1
+            for (int j = seg; j < 8; j += R) {
+                float sum = ps[warp % V][j][lane];
 #pragma unroll
-            for (int j = 0; j < WN; ++j) {
-                const float D = fmaf((float)j, cRw, r0);
-                const float H = FAN ? fmaf((float)j, dhbw, hb0) : hb0;
-                const float w = footprint_weight_v(D, H, fp);
-                const float ap = NEG ? pp[j].y : pp[j].x, am = NEG ? pm[j].y : pm[j].x;
-                const float bp = NEG ? pp[j].x : pp[j].y, bm = NEG ? pm[j].x : pm[j].y;
-                const float cp = NEG ? pp[j].w : pp[j].z, cm = NEG ? pm[j].w : pm[j].z;
-                const float dp = NEG ? pp[j].z : pp[j].w, dm = NEG ? pm[j].z : pm[j].w;
-                S[0] = fmaf(w, ap, S[0]);
-                S[6] = fmaf(w, am, S[6]);
-                S[4] = fmaf(w, bp, S[4]);
-                S[2] = fmaf(w, bm, S[2]);
-                S[5] = fmaf(w, cp, S[5]);
-                S[3] = fmaf(w, cm, S[3]);
-                S[1] = fmaf(w, dp, S[1]);
-                S[7] = fmaf(w, dm, S[7]);
-            }
-        };
-#if CTPRJ_FWD_PIPE
-        // Build-time variant (CTPRJ_FWD_PIPE=1): the window march software-
-        // pipelined two rows deep, the next row's gathers issued before this
-        // row's footprints (rows ya, ya - 1, ..., yb; q is row ya's quad row
-        // and moves by dq per row).  Same sums as march_win.
-        auto march_pipe = [&](const int ya, const int yb, const float4 *q, const int dq, auto neg, auto wn) {
-            constexpr bool NEG = decltype(neg)::value;
-            constexpr int WN = decltype(wn)::value;
-            struct Row {
-                float4 pp[WN], pm[WN];
-                int xs;
-                bool on;
-            };
-            auto fetch = [&](const int y, const float4 *__restrict__ qq, Row &R) {
-                const float xc = fmaf(-(float)y, Scf, Acf);
-                R.on = !(xc < -(float)half - 2.0f || xc > (float)half + 2.0f);
-                int xs = (WN == 3 ? __float2int_rn(xc) : __float2int_rd(xc)) - 1;
-                xs = min(max(xs, -half), half - (WN - 1));
-                R.xs = xs;
-#pragma unroll
-                for (int j = 0; j < WN; ++j) {
-                    R.pp[j] = __ldg(qq + xs + j);
-                    R.pm[j] = __ldg(qq - xs - j);
-                }
-            };
-            auto sum = [&](const int y, const Row &R) {
-                if (!R.on) return;
-                const float yf = (float)y;
-                const float r0 = (float)fma((double)R.xs, cR, fma((double)y, sR, -off)) * fp.iw;
-                const float hb0 = (FAN ? 0.5f * fmaf(fmaf((float)R.xs, sTf, -yf * cTf), kbw, bwc)
-                                       : 0.5f * g.beamWidthF) * fp.iw;
-#pragma unroll
-                for (int j = 0; j < WN; ++j) {
-                    const float D = fmaf((float)j, cRw, r0);
-                    const float H = FAN ? fmaf((float)j, dhbw, hb0) : hb0;
-                    const float w = footprint_weight_v(D, H, fp);
-                    const float4 pp = R.pp[j], pm = R.pm[j];
-                    S[0] = fmaf(w, NEG ? pp.y : pp.x, S[0]);
-                    S[6] = fmaf(w, NEG ? pm.y : pm.x, S[6]);
-                    S[4] = fmaf(w, NEG ? pp.x : pp.y, S[4]);
-                    S[2] = fmaf(w, NEG ? pm.x : pm.y, S[2]);
-                    S[5] = fmaf(w, NEG ? pp.w : pp.z, S[5]);
-                    S[3] = fmaf(w, NEG ? pm.w : pm.z, S[3]);
-                    S[1] = fmaf(w, NEG ? pp.z : pp.w, S[1]);
-                    S[7] = fmaf(w, NEG ? pm.z : pm.w, S[7]);
-                }
-            };
-            Row A, B;
-            fetch(ya, q, A);
-            int y = ya;
-            for (; y - 1 >= yb; y -= 2, q += 2 * dq) {
-                fetch(y - 1, q + dq, B);
-                sum(y, A);
-                if (y - 2 >= yb) fetch(y - 2, q + 2 * dq, A);
-                sum(y - 1, B);
-            }
-            if (y == yb) sum(y, A);
-        };
-        if (wcode == 3 || wcode == 4) {
-            const float4 *qp = quad + (size_t)half * QW + half, *qn = quad + (size_t)QW + half;
-            if (wcode == 3) {
-                march_pipe(half, 0, qp, -QW, std::false_type{}, std::integral_constant<int, 3>{});
-                march_pipe(-1, -half, qn, QW, std::true_type{}, std::integral_constant<int, 3>{});
-            } else {
-                march_pipe(half, 0, qp, -QW, std::false_type{}, std::integral_constant<int, 4>{});
-                march_pipe(-1, -half, qn, QW, std::true_type{}, std::integral_constant<int, 4>{});
-            }
-        } else
-#endif
-        {
-            const float4 *q = quad + (size_t)half * QW + half;   // row |y| = half, x = 0
-            if (wcode == 3) {
-                for (int y = half; y >= 0; --y, q -= QW)
-                    march_win(y, q, std::false_type{}, std::integral_constant<int, 3>{});
-            } else if (wcode == 4) {
-                for (int y = half; y >= 0; --y, q -= QW)
-                    march_win(y, q, std::false_type{}, std::integral_constant<int, 4>{});
-            } else {
-                for (int y = half; y >= 0; --y, q -= QW) march_row(y, q, std::false_type{});
-            }
-            q = quad + (size_t)QW + half;                          // row |y| = 1
-            if (wcode == 3) {
-                for (int y = -1; y >= -half; --y, q += QW)
-                    march_win(y, q, std::true_type{}, std::integral_constant<int, 3>{});
-            } else if (wcode == 4) {
-                for (int y = -1; y >= -half; --y, q += QW)
-                    march_win(y, q, std::true_type{}, std::integral_constant<int, 4>{});
-            } else {
-                for (int y = -1; y >= -half; --y, q += QW) march_row(y, q, std::true_type{});
+                for (int q = 1; q < R; ++q) sum += ps[q * V + warp % V][j][lane];
+                fsum += put_image<FAN, MODE>(p, b, k, j, sum, sino, tab, Ie);
             }
         }
-
-        // Scatter to the eight symmetric views (prj/cpuPrj.c:577-615); parallel
-        // beam also writes the point-reflected detector of the same view
-        // (prj/cpuPrj.c:403-460), which image j ^ 2 holds.  Where the two
-        // coincide (the central detector) the second write is the one kept.
-        const int pC = g.pC;
+        return fsum;
+    }
+    rows_of(0);
+    if constexpr (R == kAllParts) {
+        if (p.rsplit > 1) {
+            float *tot = parts + threadIdx.x;
+            const int step = blockDim.x;
+            for (int s = 1; s < p.rsplit; ++s) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) tot[j * step] = s == 1 ? S[j] : tot[j * step] + S[j];
+                rows_of(s);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) S[j] = tot[j * step] + S[j];
+        }
+    }
+    if (!live) return fsum;
+    if constexpr (MODE == kModeCount) {
         unsigned long long entries = 0;
-        // polychromatic mode: the entries this ray sum feeds, gathered first so
-        // that one copy of the FP64 epilogue serves them all
+        for (int j = 0; j < 8; ++j) {
+            const int det = j < 4 ? k : 2 * g.pC - k;
+            if (p.view[b].out[j] >= 0) entries += (!FAN && 2 * g.pC - det != det) ? 2 : 1;
+        }
+        if (nz * entries) atomicAdd(counter, nz * entries);
+    } else if constexpr (MODE == kModeBhc) {
+        // the entries this ray sum feeds, gathered first so that one copy of
+        // the FP64 epilogue serves them all
+        const int pC = g.pC;
         float eval[16];
         int eidx[16];
         int ne = 0;
@@ -541,40 +550,37 @@ __device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int b
             const int det = j < 4 ? k : 2 * pC - k;
             const int det2 = 2 * pC - det;
             const size_t row = (size_t)v * g.W;
-            if constexpr (MODE == kModeCount) {
-                entries += (!FAN && det2 != det) ? 2 : 1;
-            } else if constexpr (MODE == kModeBhc) {
-                if (FAN) {
-                    eval[ne] = S[j] / g.effRate; eidx[ne++] = (int)(row + det);
-                } else if (det2 != det) {
-                    eval[ne] = S[j] / g.effRate; eidx[ne++] = (int)(row + det);
-                    eval[ne] = S[j ^ 2] / g.effRate; eidx[ne++] = (int)(row + det2);
-                } else {
-                    eval[ne] = S[j ^ 2] / g.effRate; eidx[ne++] = (int)(row + det);
-                }
+            if (FAN) {
+                eval[ne] = S[j] / g.effRate; eidx[ne++] = (int)(row + det);
+            } else if (det2 != det) {
+                eval[ne] = S[j] / g.effRate; eidx[ne++] = (int)(row + det);
+                eval[ne] = S[j ^ 2] / g.effRate; eidx[ne++] = (int)(row + det2);
             } else {
-                sino[row + det] = S[j] / g.effRate;
-                if (!FAN) sino[row + det2] = S[j ^ 2] / g.effRate;
+                eval[ne] = S[j ^ 2] / g.effRate; eidx[ne++] = (int)(row + det);
             }
         }
-        if constexpr (MODE == kModeBhc) {
 #pragma unroll 1
-            for (int e = 0; e < ne; ++e) {
-                fsum += bhc_entry(p.bhc, tab, Ie, eval[e], (size_t)eidx[e]);
-                if (p.bhc.proj_out) p.bhc.proj_out[eidx[e]] = eval[e];
-            }
+        for (int e = 0; e < ne; ++e) {
+            fsum += bhc_entry(p.bhc, tab, Ie, eval[e], (size_t)eidx[e]);
+            if (p.bhc.proj_out) p.bhc.proj_out[eidx[e]] = eval[e];
         }
-        if (MODE == kModeCount && nz * entries) atomicAdd(counter, nz * entries);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) put_image<FAN, MODE>(p, b, k, j, S[j], sino, tab, Ie);
     }
     return fsum;
 }
 
-template <bool FAN, int MODE>
-__global__ void __launch_bounds__(kFwdThreads, CTPRJ_FWD_MINBLOCKS)
+// floats of shared memory a forward block of `warps` warps needs for its parts
+__host__ __device__ constexpr int fwd_part_floats(int warps) { return warps * 8 * 32; }
+
+template <bool FAN, int MODE, int V, int R>
+__global__ void __launch_bounds__(32 * V * R, V * R <= 4 ? CTPRJ_FWD_MINBLOCKS : 2)
 k_forward(const FwdParams p, const float4 *__restrict__ quad, float *__restrict__ sino,
           unsigned long long *__restrict__ counter)
 {
     const double *tab = nullptr, *Ie = nullptr;
+    __shared__ float parts[R > 1 ? fwd_part_floats(V * R) : 1];
     if constexpr (MODE == kModeBhc) {
         __shared__ double sm[kMaxJ * (kSplStride + 1)];
         for (int i = threadIdx.x; i < p.bhc.J * kSplStride; i += blockDim.x) sm[i] = p.bhc.tab[i];
@@ -583,287 +589,36 @@ k_forward(const FwdParams p, const float4 *__restrict__ quad, float *__restrict_
         tab = sm;
         Ie = sm + kMaxJ * kSplStride;
     }
-    int bx = blockIdx.x, by = blockIdx.y;
-#if CTPRJ_FWD_REMAP
-    // Build-time variant: the block scheduler starts blocks i, i + S, i + 2S, ...
-    // (S = SM count) on one SM in its first wave, so hand them consecutive view
-    // groups of one ray group: their rays cross nearly the same quad-image
-    // lines and could share that SM's L1.  A bijection of the block indices.
-    {
-        const int S = p.sms, total = gridDim.x * gridDim.y, i = blockIdx.y * gridDim.x + blockIdx.x;
-        const int q = total / S, r = total % S, sl = i % S, k = i / S;
-        const int item = sl * q + min(sl, r) + k;
-        bx = item % gridDim.x;
-        by = item / gridDim.x;
-    }
-#endif
-    const double fsum = forward_rays<FAN, MODE, kFwdViews>(p, bx, by, quad, sino, counter, tab, Ie);
+    const int bx = blockIdx.x, by = blockIdx.y;
+    const double fsum = forward_rays<FAN, MODE, V, R>(p, bx, by, quad, sino, counter, tab, Ie, parts);
     if constexpr (MODE == kModeBhc) {
-        __shared__ double red[kFwdThreads / 32];
+        __shared__ double red[V * R];
         const double t = block_sum(fsum, red);
         if (threadIdx.x == 0) p.bhc.part[(size_t)by * gridDim.x + bx] = t;
     }
 }
 
-#if CTPRJ_FWD_STAGE
-// -------------------------------------------- forward, staged by bulk copies
-//
-// Build-time variant (CTPRJ_FWD_STAGE=1), measured against k_forward.  The
-// block's rays read the quad-image rows of a chunk of kStRows rows from shared
-// memory: one thread brings the row segments in with bulk asynchronous copies
-// (cp.async.bulk, completion counted on an mbarrier), double-buffered so that
-// the copies of chunk c + 1 are in flight while chunk c is summed.  A segment
-// is the union of the block's pixel windows over the chunk's rows, on the +x
-// side and its mirror; a chunk whose union exceeds kStCols pixels is read from
-// global memory instead, and so are warps whose rays need the range loop.
-// Plain mode only.  Waits are bounded (%globaltimer, 1 s): past it the block
-// records the timeout in g_fwd_stage_timeout, writes NaN to its outputs and
-// returns.
-
-#ifndef CTPRJ_FWD_STAGE_ROWS
-#define CTPRJ_FWD_STAGE_ROWS 4
-#endif
-constexpr int kStRows = CTPRJ_FWD_STAGE_ROWS;
-constexpr int kStCols = 128;
-
-struct FwdStage {
-    float4 buf[2][kStRows][2][kStCols];   // [buffer][row][+x side, -x side][pixel]
-    unsigned long long bar[2];
-    int lo[2], hi[2];                      // staged pixels [lo, hi] of each buffer; hi < lo: none
-    int wlo[kFwdViews], whi[kFwdViews];
-};
-
-__device__ int g_fwd_stage_timeout;
-
-__device__ __forceinline__ unsigned long long stage_ns()
+// Parts a plan's image rows are summed in, one warp each.  The base rays alone
+// fill only part of the GPU below 1024^2 (276 warps at 256^2, where it holds
+// 2960), and up to three and a half waves of warps a split still evens out the
+// rays' uneven ways through the image.  Measured, 1 / 2 / 4 / 8 parts: 64^2 fan 28.7 / 20.5 /
+// 14.4 / 10.3 us, 256^2 parallel 84 / 51 / 31 / 21, 512^2 fan (1024 detectors)
+// 176 / 143 / 128 / 114, parallel 164 / 107 / 104 / 102, 1001^2 parallel 559 /
+// 553 / 531 / 600, 2048^2 fan 3538 / 3530 / 3561 / 3774; 16 parts gain nothing.
+static int forward_split(const ctprj_plan *pl)
 {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device);
+    const long long warps = (long long)pl->nb * ((pl->nk + 31) / 32), wave = 4LL * CTPRJ_FWD_MINBLOCKS * sms;
+    int R = 1;
+    while (R < 8 && 2 * warps * R < 7 * wave) R *= 2;
+    return R;
 }
-
-__device__ __forceinline__ unsigned smem_u32(const void *ptr)
-{
-    return (unsigned)__cvta_generic_to_shared(ptr);
-}
-
-// true when the phase of parity `ph` of barrier `bar` completed within 1 s
-__device__ __forceinline__ bool stage_wait(unsigned long long *bar, unsigned ph)
-{
-    const unsigned a = smem_u32(bar);
-    const unsigned long long t0 = stage_ns();
-    for (;;) {
-        unsigned done;
-        asm volatile("{\n\t.reg .pred p;\n\t"
-                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done) : "r"(a), "r"(ph) : "memory");
-        if (done) return true;
-        if (stage_ns() - t0 > 1000000000ull) return false;
-    }
-}
-
-template <bool FAN>
-__global__ void __launch_bounds__(kFwdThreads, CTPRJ_FWD_MINBLOCKS)
-k_forward_staged(const FwdParams p, const float4 *__restrict__ quad, float *__restrict__ sino)
-{
-    __shared__ __align__(128) FwdStage st;
-    const Geo &g = p.g;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b = blockIdx.x * kFwdViews + warp;
-    const int r = blockIdx.y * 32 + lane;
-    const bool live = b < p.nb && r < p.nk;
-    if (p.zero_col0 && blockIdx.x == 0 && blockIdx.y == 0)
-        for (int v = threadIdx.x; v < g.np; v += blockDim.x) sino[(size_t)v * g.W] = 0.0f;
-    const int half = g.half, QW = 2 * half + 1;
-    const int k = p.k0 + r;
-    FwdRay ray = {};
-    int wcode = 0;   // 0: no ray, 3 / 4: window, 5: range loop (global reads)
-    if (live) {
-        ray = fwd_ray<FAN>(p, b, k);
-        const float wa = ray.Ar - ray.Al, ws = ray.Sr - ray.Sl;
-        const float wmax = fmaxf(fabsf(fmaf(-(float)half, ws, wa)), fabsf(fmaf((float)half, ws, wa)));
-        wcode = half < 3 ? 5 : (wmax < 1.95f ? 3 : (wmax < 2.95f ? 4 : 5));
-    }
-    wcode = __reduce_max_sync(0xffffffffu, wcode);
-    const float Acf = 0.5f * (ray.Al + ray.Ar), Scf = 0.5f * (ray.Sl + ray.Sr);
-    // the window start of this lane's ray at row y (window rays only)
-    auto wstart = [&](int y) {
-        const float xc = fmaf(-(float)y, Scf, Acf);
-        const int xs = (wcode == 3 ? __float2int_rn(xc) : __float2int_rd(xc)) - 1;
-        return min(max(xs, -half), half - (wcode - 1));
-    };
-    const int steps = 2 * half + 1;               // rows y = half - m, m = 0 .. 2 half
-    const int nchunks = (steps + kStRows - 1) / kStRows;
-    // this warp's union of windows over chunk c, then the block's, into buffer c & 1
-    auto plan_chunk = [&](int c) {
-        int lo = INT_MAX, hi = INT_MIN;
-        if (live && (wcode == 3 || wcode == 4)) {
-            const int m0 = c * kStRows, m1 = min(m0 + kStRows, steps) - 1;
-            const int a0 = wstart(half - m0), a1 = wstart(half - m1);
-            lo = min(a0, a1);
-            hi = max(a0, a1) + wcode - 1;
-        }
-        lo = __reduce_min_sync(0xffffffffu, lo);
-        hi = __reduce_max_sync(0xffffffffu, hi);
-        if (lane == 0) {
-            st.wlo[warp] = lo;
-            st.whi[warp] = hi;
-        }
-    };
-    auto issue_chunk = [&](int c) {   // thread 0, after a block barrier
-        const int bc = c & 1;
-        int lo = INT_MAX, hi = INT_MIN;
-        for (int w = 0; w < kFwdViews; ++w) {
-            lo = min(lo, st.wlo[w]);
-            hi = max(hi, st.whi[w]);
-        }
-        if (hi < lo || hi - lo + 1 > kStCols) {
-            st.lo[bc] = 1;
-            st.hi[bc] = 0;
-            return;
-        }
-        st.lo[bc] = lo;
-        st.hi[bc] = hi;
-        const int m0 = c * kStRows, nr = min(kStRows, steps - m0);
-        const unsigned bytes = (unsigned)(hi - lo + 1) * 16u;
-        const unsigned bar = smem_u32(&st.bar[bc]);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                     :: "r"(bar), "r"(bytes * 2u * (unsigned)nr) : "memory");
-        for (int i = 0; i < nr; ++i) {
-            const int y = half - (m0 + i), row = y < 0 ? -y : y;
-            const float4 *src = quad + (size_t)row * QW + half;
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         :: "r"(smem_u32(&st.buf[bc][i][0][0])), "l"(src + lo), "r"(bytes), "r"(bar)
-                         : "memory");
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         :: "r"(smem_u32(&st.buf[bc][i][1][0])), "l"(src - hi), "r"(bytes), "r"(bar)
-                         : "memory");
-        }
-    };
-
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&st.bar[0])) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&st.bar[1])) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    plan_chunk(0);
-    __syncthreads();
-    if (threadIdx.x == 0) issue_chunk(0);
-
-    float S[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) S[j] = 0.0f;
-    unsigned ph[2] = {0u, 0u};
-    bool failed = false;
-    for (int c = 0; c < nchunks; ++c) {
-        const int bc = c & 1;
-        if (c + 1 < nchunks) plan_chunk(c + 1);
-        // chunk c - 1 read; windows of chunk c + 1 visible; a wait that timed
-        // out in any thread ends the march of the whole block
-        if (__syncthreads_or(failed)) {
-            failed = true;
-            break;
-        }
-        if (threadIdx.x == 0 && c + 1 < nchunks) issue_chunk(c + 1);
-        const int lo = st.lo[bc], hi = st.hi[bc];
-        const bool staged = lo <= hi;
-        if (staged) {
-            if (!stage_wait(&st.bar[bc], ph[bc])) {
-                failed = true;
-                continue;
-            }
-            ph[bc] ^= 1u;
-        }
-        if (!live) continue;
-        const int m0 = c * kStRows, nr = min(kStRows, steps - m0);
-        for (int i = 0; i < nr; ++i) {
-            const int y = half - (m0 + i), row = y < 0 ? -y : y;
-            const bool neg = y < 0;
-            const float4 *q = quad + (size_t)row * QW + half;
-            const float yf = (float)y;
-            if (wcode == 5) {
-                // range loop from global memory (prj/cpuPrj.c:365-369, :514-536 ranges)
-                const int x0 = max(__float2int_rn(fmaf(-yf, ray.Sl, ray.Al)), -half);
-                const int x1 = min(__float2int_rn(fmaf(-yf, ray.Sr, ray.Ar)), half);
-                for (int x = x0; x <= x1; ++x) {
-                    const float D = (float)fma((double)x, ray.cR, fma((double)y, ray.sR, -ray.off)) * ray.fp.iw;
-                    const float H = (FAN ? 0.5f * fmaf(fmaf((float)x, ray.sT, -yf * ray.cT), ray.kbw, ray.bwc)
-                                         : 0.5f * g.beamWidthF) * ray.fp.iw;
-                    const float w = footprint_weight_v(D, H, ray.fp);
-                    const float4 pp = __ldg(q + x), pm = __ldg(q - x);
-                    S[0] = fmaf(w, neg ? pp.y : pp.x, S[0]);
-                    S[6] = fmaf(w, neg ? pm.y : pm.x, S[6]);
-                    S[4] = fmaf(w, neg ? pp.x : pp.y, S[4]);
-                    S[2] = fmaf(w, neg ? pm.x : pm.y, S[2]);
-                    S[5] = fmaf(w, neg ? pp.w : pp.z, S[5]);
-                    S[3] = fmaf(w, neg ? pm.w : pm.z, S[3]);
-                    S[1] = fmaf(w, neg ? pp.z : pp.w, S[1]);
-                    S[7] = fmaf(w, neg ? pm.z : pm.w, S[7]);
-                }
-                continue;
-            }
-            const float xc = fmaf(-yf, Scf, Acf);
-            if (xc < -(float)half - 2.0f || xc > (float)half + 2.0f) continue;
-            const int xs = wstart(y);
-            const float r0 = (float)fma((double)xs, ray.cR, fma((double)y, ray.sR, -ray.off)) * ray.fp.iw;
-            const float hb0 = (FAN ? 0.5f * fmaf(fmaf((float)xs, ray.sT, -yf * ray.cT), ray.kbw, ray.bwc)
-                                   : 0.5f * g.beamWidthF) * ray.fp.iw;
-            // the window's pixels, unrolled for the warp's window width
-            auto row_sum = [&](auto wn) {
-                constexpr int WN = decltype(wn)::value;
-                float4 pp[WN], pm[WN];
-#pragma unroll
-                for (int j = 0; j < WN; ++j) {
-                    pp[j] = staged ? st.buf[bc][i][0][xs + j - lo] : __ldg(q + xs + j);
-                    pm[j] = staged ? st.buf[bc][i][1][hi - xs - j] : __ldg(q - xs - j);
-                }
-#pragma unroll
-                for (int j = 0; j < WN; ++j) {
-                    const float D = fmaf((float)j, ray.cRw, r0);
-                    const float H = FAN ? fmaf((float)j, ray.dhbw, hb0) : hb0;
-                    const float w = footprint_weight_v(D, H, ray.fp);
-                    S[0] = fmaf(w, neg ? pp[j].y : pp[j].x, S[0]);
-                    S[6] = fmaf(w, neg ? pm[j].y : pm[j].x, S[6]);
-                    S[4] = fmaf(w, neg ? pp[j].x : pp[j].y, S[4]);
-                    S[2] = fmaf(w, neg ? pm[j].x : pm[j].y, S[2]);
-                    S[5] = fmaf(w, neg ? pp[j].w : pp[j].z, S[5]);
-                    S[3] = fmaf(w, neg ? pm[j].w : pm[j].z, S[3]);
-                    S[1] = fmaf(w, neg ? pp[j].z : pp[j].w, S[1]);
-                    S[7] = fmaf(w, neg ? pm[j].z : pm[j].w, S[7]);
-                }
-            };
-            if (wcode == 3) row_sum(std::integral_constant<int, 3>{});
-            else row_sum(std::integral_constant<int, 4>{});
-        }
-    }
-    failed = __syncthreads_or(failed);
-    if (failed) {
-        if (threadIdx.x == 0) atomicExch(&g_fwd_stage_timeout, 1);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) S[j] = __int_as_float(0x7fc00000);
-    }
-    if (!live) return;
-    const int pC = g.pC;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int v = p.view[b].out[j];
-        if (v < 0) continue;
-        const int det = j < 4 ? k : 2 * pC - k;
-        const int det2 = 2 * pC - det;
-        const size_t row = (size_t)v * g.W;
-        sino[row + det] = S[j] / g.effRate;
-        if (!FAN) sino[row + det2] = S[j ^ 2] / g.effRate;
-    }
-}
-#endif
 
 static FwdParams fwd_params(const ctprj_plan *pl)
 {
     FwdParams p;
-    p.sms = 148;
-    cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, pl->device);
+    p.rsplit = forward_split(pl);
     p.g = pl->g;
     p.nb = pl->nb;
     p.k0 = pl->k0;
@@ -875,34 +630,48 @@ static FwdParams fwd_params(const ctprj_plan *pl)
     return p;
 }
 
-static dim3 fwd_grid(const ctprj_plan *pl)
+// views per forward block when the rows are summed in R parts: blocks of four
+// warps, eight for eight parts
+static int fwd_views(int R) { return R >= 4 ? 1 : kFwdViews / R; }
+
+static dim3 fwd_grid(const ctprj_plan *pl, int R)
 {
-    return dim3((pl->nb + kFwdViews - 1) / kFwdViews, (pl->nk + 31) / 32);
+    const int V = fwd_views(R);
+    return dim3((pl->nb + V - 1) / V, (pl->nk + 31) / 32);
 }
 
 int forward_blocks(const ctprj_plan *pl)
 {
-    const dim3 g = fwd_grid(pl);
+    const dim3 g = fwd_grid(pl, forward_split(pl));
     return (int)(g.x * g.y);
+}
+
+template <bool FAN, int MODE>
+static void launch_forward_t(const FwdParams &p, dim3 grid, const float4 *quad, float *sino,
+                             unsigned long long *counter, cudaStream_t s)
+{
+    switch (p.rsplit) {
+    case 1: k_forward<FAN, MODE, kFwdViews, 1><<<grid, kFwdThreads, 0, s>>>(p, quad, sino, counter); break;
+    case 2: k_forward<FAN, MODE, kFwdViews / 2, 2><<<grid, kFwdThreads, 0, s>>>(p, quad, sino, counter); break;
+    case 4: k_forward<FAN, MODE, 1, 4><<<grid, kFwdThreads, 0, s>>>(p, quad, sino, counter); break;
+    default: k_forward<FAN, MODE, 1, 8><<<grid, 256, 0, s>>>(p, quad, sino, counter); break;
+    }
 }
 
 int launch_forward(const ctprj_plan *pl, const float4 *quad, float *sino,
                    unsigned long long *counter, cudaStream_t s)
 {
-    const FwdParams p = fwd_params(pl);
-    const dim3 grid = fwd_grid(pl), block(kFwdThreads);
+    FwdParams p = fwd_params(pl);
     const bool fan = pl->g.fan != 0;
     if (counter) {
-        if (fan) k_forward<true, kModeCount><<<grid, block, 0, s>>>(p, quad, sino, counter);
-        else k_forward<false, kModeCount><<<grid, block, 0, s>>>(p, quad, sino, counter);
+        p.rsplit = 1;
+        const dim3 grid = fwd_grid(pl, 1);
+        if (fan) k_forward<true, kModeCount, kFwdViews, 1><<<grid, kFwdThreads, 0, s>>>(p, quad, sino, counter);
+        else k_forward<false, kModeCount, kFwdViews, 1><<<grid, kFwdThreads, 0, s>>>(p, quad, sino, counter);
     } else {
-#if CTPRJ_FWD_STAGE
-        if (fan) k_forward_staged<true><<<grid, block, 0, s>>>(p, quad, sino);
-        else k_forward_staged<false><<<grid, block, 0, s>>>(p, quad, sino);
-#else
-        if (fan) k_forward<true, kModePlain><<<grid, block, 0, s>>>(p, quad, sino, counter);
-        else k_forward<false, kModePlain><<<grid, block, 0, s>>>(p, quad, sino, counter);
-#endif
+        const dim3 grid = fwd_grid(pl, p.rsplit);
+        if (fan) launch_forward_t<true, kModePlain>(p, grid, quad, sino, counter, s);
+        else launch_forward_t<false, kModePlain>(p, grid, quad, sino, counter, s);
     }
     return cuda_error(cudaGetLastError(), "forward launch");
 }
@@ -912,9 +681,9 @@ int launch_forward_bhc(const ctprj_plan *pl, const float4 *quad,
 {
     FwdParams p = fwd_params(pl);
     p.bhc = a;
-    const dim3 grid = fwd_grid(pl), block(kFwdThreads);
-    if (pl->g.fan) k_forward<true, kModeBhc><<<grid, block, 0, s>>>(p, quad, nullptr, nullptr);
-    else k_forward<false, kModeBhc><<<grid, block, 0, s>>>(p, quad, nullptr, nullptr);
+    const dim3 grid = fwd_grid(pl, p.rsplit);
+    if (pl->g.fan) launch_forward_t<true, kModeBhc>(p, grid, quad, nullptr, nullptr, s);
+    else launch_forward_t<false, kModeBhc>(p, grid, quad, nullptr, nullptr, s);
     if (nparts) *nparts = (int)(grid.x * grid.y);
     return cuda_error(cudaGetLastError(), "fused polychromatic forward launch");
 }
@@ -1962,6 +1731,7 @@ template <int V>
 __global__ void __launch_bounds__(32 * V, 4 * CTPRJ_FWD_MINBLOCKS / V) k_forward_batch(const BatchArgs a)
 {
     __shared__ long long slot;
+    __shared__ float parts[fwd_part_floats(V)];
     for (;;) {
         const long long item = next_item(a.counter, &slot);
         if (item >= a.total) return;
@@ -1971,9 +1741,9 @@ __global__ void __launch_bounds__(32 * V, 4 * CTPRJ_FWD_MINBLOCKS / V) k_forward
         const int gx = (sl.fp.nb + V - 1) / V;
         const int bx = local % gx, by = local / gx;
         if (sl.fp.g.fan)
-            forward_rays<true, kModePlain, V>(sl.fp, bx, by, sl.quad, sl.sino, nullptr, nullptr, nullptr);
+            forward_rays<true, kModePlain, V, kAllParts>(sl.fp, bx, by, sl.quad, sl.sino, nullptr, nullptr, nullptr, parts);
         else
-            forward_rays<false, kModePlain, V>(sl.fp, bx, by, sl.quad, sl.sino, nullptr, nullptr, nullptr);
+            forward_rays<false, kModePlain, V, kAllParts>(sl.fp, bx, by, sl.quad, sl.sino, nullptr, nullptr, nullptr, parts);
     }
 }
 
