@@ -1442,12 +1442,29 @@ __device__ __forceinline__ void tile_sums(const BwdParams &p, int tx, int ty, in
     }
 }
 
-// the octant pixel (x, y) of thread t of tile (tx, ty); it owns (x + 1, y) too
-__device__ __forceinline__ void pair_of(int t, int tx, int ty, int &x, int &y)
+// A tile's sums by image and pixel, for the stores: a row of 16 pixels and one
+// of padding, so that rows and columns are read without bank conflicts.
+constexpr int kBwdRow = kBwdTile + 1;
+using TileSums = float[8][kBwdTile * kBwdRow];
+constexpr int kBwdValues = 8 * kBwdTile * kBwdTile;
+
+// this thread's slot of pixel x (pixel x + 1 is the next)
+__device__ __forceinline__ int own_slot()
 {
-    const int lane = t & 31, warp = t >> 5;
-    x = tx * kBwdTile + (warp & 1) * 8 + ((lane >> 3) & 1) * 4 + (lane & 1) * 2;
-    y = ty * kBwdTile + (warp >> 1) * 8 + (lane >> 4) * 4 + ((lane >> 1) & 3);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lx = (warp & 1) * 8 + ((lane >> 3) & 1) * 4 + (lane & 1) * 2;
+    const int ly = (warp >> 1) * 8 + (lane >> 4) * 4 + ((lane >> 1) & 3);
+    return ly * kBwdRow + lx;
+}
+
+// image and pixel of value e: consecutive values are consecutive pixels of an
+// image row, which runs along x for even images and along y for odd ones
+__device__ __forceinline__ void value_of(int e, int &j, int &lx, int &ly)
+{
+    j = e / (kBwdTile * kBwdTile);
+    const int a = e % kBwdTile, b = e / kBwdTile % kBwdTile;
+    lx = (j & 1) ? b : a;
+    ly = (j & 1) ? a : b;
 }
 
 // image j of octant pixel (x, y), if the pixel is one and the image its own
@@ -1476,14 +1493,16 @@ __device__ __forceinline__ void zero_axes(const BwdParams &p, float *__restrict_
 // Staged backprojection, one tile per cluster of p.split blocks, each block
 // the views of its part.  The parts' sums meet in distributed shared memory:
 // every block adds up its share of the tile's pixel images over the parts, in
-// the parts' order, and writes it.
+// the parts' order, and writes it, sixteen pixels of an image row at a time
+// (the caller's image may be page-locked host memory, where scattered words
+// cost a bus transaction each).
 template <bool FAN, bool FBP, int SEG, int VB, int MODE>
 __global__ void __launch_bounds__(kBwdThreads, CTPRJ_BWD_MINBLOCKS)
 k_backward_tiled(const BwdParams p, float *__restrict__ img)
 {
     __shared__ union {
         TiledSmem<FAN, SEG, VB> st;
-        float part[16][kBwdThreads];
+        TileSums sums;
     } sm;
     const int S = p.split, tile = blockIdx.x / S, s = blockIdx.x % S;
     if (p.zero_axes && blockIdx.x == 0) zero_axes(p, img);
@@ -1491,49 +1510,52 @@ k_backward_tiled(const BwdParams p, float *__restrict__ img)
     decode_tile(tile, tx, ty);
     float A[8], B[8];
     tile_sums<FAN, FBP, SEG, VB, MODE>(p, tx, ty, part_begin(p.nv, s, S), part_begin(p.nv, s + 1, S), A, B, sm.st);
-    int x, y;
-    if (S == 1) {
-        pair_of(threadIdx.x, tx, ty, x, y);
+    const int own = own_slot();
 #pragma unroll
-        for (int v = 0; v < 16; ++v) write_image(p, img, x + (v >> 3), y, v & 7, v < 8 ? A[v & 7] : B[v & 7]);
-        return;
+    for (int j = 0; j < 8; ++j) {
+        sm.sums[j][own] = A[j];
+        sm.sums[j][own + 1] = B[j];
     }
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
-#pragma unroll
-    for (int v = 0; v < 16; ++v) sm.part[v][threadIdx.x] = v < 8 ? A[v & 7] : B[v & 7];
-    cl.sync();
-    for (int e = s * kBwdThreads + threadIdx.x; e < 16 * kBwdThreads; e += S * kBwdThreads) {
-        const int v = e / kBwdThreads, t = e % kBwdThreads;
-        float sum = *cl.map_shared_rank(&sm.part[v][t], 0);
-        for (int q = 1; q < S; ++q) sum += *cl.map_shared_rank(&sm.part[v][t], q);
-        pair_of(t, tx, ty, x, y);
-        write_image(p, img, x + (v >> 3), y, v & 7, sum);
+    if (S > 1) cl.sync();
+    else __syncthreads();
+    for (int e = s * (kBwdValues / S) + threadIdx.x; e < (s + 1) * (kBwdValues / S); e += kBwdThreads) {
+        int j, lx, ly;
+        value_of(e, j, lx, ly);
+        float *v = &sm.sums[j][ly * kBwdRow + lx];
+        float sum = S > 1 ? *cl.map_shared_rank(v, 0) : *v;
+        for (int q = 1; q < S; ++q) sum += *cl.map_shared_rank(v, q);
+        write_image(p, img, tx * kBwdTile + lx, ty * kBwdTile + ly, j, sum);
     }
-    cl.sync();   // a block's sums stay until every block has read them
+    if (S > 1) cl.sync();   // a block's sums stay until every block has read them
 }
 
 // One tile by one block, for the persistent launches: the parts one after the
 // other, added in the same order.
 template <bool FAN, bool FBP, int SEG, int VB, int MODE>
 __device__ __forceinline__ void backward_tile(const BwdParams &p, int tile, float *__restrict__ img,
-                                              TiledSmem<FAN, SEG, VB> &sm, float (&tot)[16][kBwdThreads])
+                                              TiledSmem<FAN, SEG, VB> &sm, TileSums &sums)
 {
     const int S = p.split;
     if (p.zero_axes && tile == 0) zero_axes(p, img);
-    int tx, ty, x, y;
+    int tx, ty;
     decode_tile(tile, tx, ty);
-    pair_of(threadIdx.x, tx, ty, x, y);
+    const int own = own_slot();
     for (int s = 0; s < S; ++s) {
         float A[8], B[8];
         tile_sums<FAN, FBP, SEG, VB, MODE>(p, tx, ty, part_begin(p.nv, s, S), part_begin(p.nv, s + 1, S), A, B, sm);
 #pragma unroll
-        for (int v = 0; v < 16; ++v) {
-            const float a = v < 8 ? A[v & 7] : B[v & 7];
-            const float sum = s == 0 ? a : tot[v][threadIdx.x] + a;
-            if (s == S - 1) write_image(p, img, x + (v >> 3), y, v & 7, sum);
-            else tot[v][threadIdx.x] = sum;
+        for (int j = 0; j < 8; ++j) {
+            sums[j][own] = s == 0 ? A[j] : sums[j][own] + A[j];
+            sums[j][own + 1] = s == 0 ? B[j] : sums[j][own + 1] + B[j];
         }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < kBwdValues; e += kBwdThreads) {
+        int j, lx, ly;
+        value_of(e, j, lx, ly);
+        write_image(p, img, tx * kBwdTile + lx, ty * kBwdTile + ly, j, sums[j][ly * kBwdRow + lx]);
     }
 }
 
@@ -1764,7 +1786,7 @@ struct BatchSmem {
         TiledSmem<true, SEG, VB> fan;
         TiledSmem<false, SEG, VB> par;
     } st;
-    float tot[16][kBwdThreads];
+    TileSums sums;
 };
 
 // one tile of a batch slice
@@ -1776,13 +1798,13 @@ __device__ __forceinline__ void batch_tile(const BatchSlice &sl, int tile, Batch
         if (p.g.fan) backward_tile_direct<true>(p, tile, sl.bsino, sl.bimg);
         else backward_tile_direct<false>(p, tile, sl.bsino, sl.bimg);
     } else if (p.g.fan) {
-        if (p.mode == kBwdUnit) backward_tile<true, false, SEG, VB, kBwdUnit>(p, tile, sl.bimg, sm.st.fan, sm.tot);
-        else if (p.mode == kBwdNarrow) backward_tile<true, false, SEG, VB, kBwdNarrow>(p, tile, sl.bimg, sm.st.fan, sm.tot);
-        else backward_tile<true, false, SEG, VB, kBwdRange>(p, tile, sl.bimg, sm.st.fan, sm.tot);
+        if (p.mode == kBwdUnit) backward_tile<true, false, SEG, VB, kBwdUnit>(p, tile, sl.bimg, sm.st.fan, sm.sums);
+        else if (p.mode == kBwdNarrow) backward_tile<true, false, SEG, VB, kBwdNarrow>(p, tile, sl.bimg, sm.st.fan, sm.sums);
+        else backward_tile<true, false, SEG, VB, kBwdRange>(p, tile, sl.bimg, sm.st.fan, sm.sums);
     } else {
-        if (p.mode == kBwdUnit) backward_tile<false, false, SEG, VB, kBwdUnit>(p, tile, sl.bimg, sm.st.par, sm.tot);
-        else if (p.mode == kBwdNarrow) backward_tile<false, false, SEG, VB, kBwdNarrow>(p, tile, sl.bimg, sm.st.par, sm.tot);
-        else backward_tile<false, false, SEG, VB, kBwdRange>(p, tile, sl.bimg, sm.st.par, sm.tot);
+        if (p.mode == kBwdUnit) backward_tile<false, false, SEG, VB, kBwdUnit>(p, tile, sl.bimg, sm.st.par, sm.sums);
+        else if (p.mode == kBwdNarrow) backward_tile<false, false, SEG, VB, kBwdNarrow>(p, tile, sl.bimg, sm.st.par, sm.sums);
+        else backward_tile<false, false, SEG, VB, kBwdRange>(p, tile, sl.bimg, sm.st.par, sm.sums);
     }
 }
 
