@@ -25,11 +25,13 @@
 // launch reduces the partials in a fixed order and advances the scalars
 // (count, restart, t, the momentum coefficient, done), so every decision
 // stays on the device; the host checks the done flag every eight
-// iterations, and launches after convergence change nothing.
+// iterations, and launches after convergence change nothing.  Images that fit
+// the GPU's registers and shared memory take k_tv_loop instead.
 #include <algorithm>
 #include <cmath>
 
 #include "ctprj_internal.h"
+#include "grid_sums.cuh"
 #include "../../include/ctprj_tv.h"
 
 namespace ctprj {
@@ -342,6 +344,159 @@ __global__ void k_tv_start(TvState *st, int done)
     st->arrived = 0;
 }
 
+// ---- images that fit the GPU's registers and shared memory: one launch ----
+// Up to about 1.2 million pixels every tile of the image has a block of its own
+// on the GPU, so the whole iteration loop is one cooperative launch: a thread
+// keeps the dual P and P_prev of its eight pixels in registers, the tile's Xobs
+// and D stay in shared memory, and per iteration a block reads only its halo of
+// P and writes the edge of its new P.  The blocks meet once per iteration, at the
+// sums of the stopping rule (grid_sums.cuh), after which every block advances its
+// own copy of the scalars: no host check, no second launch.  What bounds an
+// iteration is the chain of latencies (halo from L2, three phases in shared
+// memory, the meeting).
+constexpr int kTvpW = 64, kTvpH = 32, kTvpRows = 4;   // tile, thread rows
+constexpr int kTvpPer = kTvpH / kTvpRows;             // pixels per thread
+
+struct TvpSmem {
+    float R1[kTvpH + 2][kTvpW + 1];   // rows i0-1 .. i0+H, columns j0 .. j0+W
+    float R2[kTvpH + 1][kTvpW + 2];   // rows i0 .. i0+H, columns j0-1 .. j0+W
+    float D[kTvpH + 1][kTvpW + 1];    // rows i0 .. i0+H, columns j0 .. j0+W
+    float X[kTvpH + 1][kTvpW + 1];
+    GridSumsSmem<4, kTvThreads> sums;
+};
+
+__global__ void __launch_bounds__(kTvThreads, 4)
+k_tv_loop(const TvArgs a, const GridMeet meet, float *__restrict__ out, int tiles_x)
+{
+    __shared__ TvpSmem S;
+    const int t = threadIdx.x, tx = t % kTvpW, ty = t / kTvpW;
+    const int i0 = (blockIdx.x / tiles_x) * kTvpH, j0 = (blockIdx.x % tiles_x) * kTvpW;
+    const int m = a.m, n = a.n, j = j0 + tx;
+    const float lam = a.lam, lb = a.lb, ub = a.ub, inv8l = 1.0f / (8.0f * lam);
+    for (int e = t; e < (kTvpH + 1) * (kTvpW + 1); e += kTvThreads) {
+        const int r = e / (kTvpW + 1), c = e % (kTvpW + 1);
+        S.X[r][c] = i0 + r < m && j0 + c < n ? a.xobs[(size_t)(i0 + r) * n + j0 + c] : 0.0f;
+        S.D[r][c] = 0.0f;
+    }
+    float2 P[kTvpPer], Q[kTvpPer];
+#pragma unroll
+    for (int k = 0; k < kTvpPer; ++k) P[k] = Q[k] = make_float2(0.0f, 0.0f);
+    // this thread's halo cell: the row above with the right corner, the row
+    // below, the left column with the bottom corner, the right column
+    int hr = 0, hc = 0;
+    bool halo = true;
+    if (t <= kTvpW) {
+        hr = -1;
+        hc = t;
+    } else if (t <= 2 * kTvpW) {
+        hr = kTvpH;
+        hc = t - kTvpW - 1;
+    } else if (t <= 2 * kTvpW + 1 + kTvpH) {
+        hr = t - 2 * kTvpW - 1;
+        hc = -1;
+    } else if (t <= 2 * kTvpW + 1 + 2 * kTvpH) {
+        hr = t - 2 * kTvpW - 2 - kTvpH;
+        hc = kTvpW;
+    } else {
+        halo = false;
+    }
+    const int hi = i0 + hr, hj = j0 + hc;
+    const bool inside = halo && hi >= 0 && hi < m && hj >= 0 && hj < n;
+    const size_t hq = inside ? (size_t)hi * n + hj : 0;
+    float2 hp = make_float2(0.0f, 0.0f);   // the halo cell's P of the last iteration
+    TvState st;
+    st.tk = 1.0;
+    st.c = 0.0;
+    st.fold = INFINITY;
+    st.count = st.iter = 0;
+    st.done = a.max_iter <= 0;
+    bool ok = true;
+    __syncthreads();
+    while (!st.done) {
+        const float c = (float)st.c;
+        if (halo) {   // R on the halo
+            float2 p = hp;
+            if (inside && st.iter > 0) p = __ldcg(tv_p(a.buf, a.px, st.iter & 1) + hq);
+            const float2 q = hp;
+            hp = p;
+            const float r1 = fmaf(c, p.x - q.x, p.x), r2 = fmaf(c, p.y - q.y, p.y);
+            if (hc >= 0) S.R1[hr + 1][hc] = r1;
+            if (hr >= 0) S.R2[hr][hc + 1] = r2;
+        }
+#pragma unroll
+        for (int k = 0; k < kTvpPer; ++k) {
+            const int r = ty + kTvpRows * k;
+            S.R1[r + 1][tx] = fmaf(c, P[k].x - Q[k].x, P[k].x);
+            S.R2[r][tx + 1] = fmaf(c, P[k].y - Q[k].y, P[k].y);
+        }
+        __syncthreads();
+        // C = Xobs - lambda L(R), D = clamp(C) on the tile (partials) and its halo
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < kTvpPer; ++k) {
+            const int r = ty + kTvpRows * k;
+            if (i0 + r < m && j < n) {
+                const float L = (S.R1[r + 1][tx] - S.R1[r][tx]) + (S.R2[r][tx + 1] - S.R2[r][tx]);
+                const float C = fmaf(-lam, L, S.X[r][tx]);
+                const float Dv = fminf(fmaxf(C, lb), ub);
+                const double dd = (double)Dv - (double)S.D[r][tx], cd = (double)C - (double)Dv;
+                S.D[r][tx] = Dv;
+                s[0] = fma(dd, dd, s[0]);
+                s[1] = fma((double)Dv, (double)Dv, s[1]);
+                s[2] = fma(cd, cd, s[2]);
+                s[3] = fma((double)C, (double)C, s[3]);
+            }
+        }
+        if (t < kTvpW + kTvpH) {   // the bottom row and the right column
+            const int r = t < kTvpW ? kTvpH : t - kTvpW, cc = t < kTvpW ? t : kTvpW;
+            if (i0 + r < m && j0 + cc < n) {
+                const float L = (S.R1[r + 1][cc] - S.R1[r][cc]) + (S.R2[r][cc + 1] - S.R2[r][cc]);
+                S.D[r][cc] = fminf(fmaxf(fmaf(-lam, L, S.X[r][cc]), lb), ub);
+            }
+        }
+        __syncthreads();
+        // P_new = proj(R + Ltrans(D) / (8 lambda)) on the tile
+        float2 *N = tv_p(a.buf, a.px, (st.iter + 1) & 1);
+#pragma unroll
+        for (int k = 0; k < kTvpPer; ++k) {
+            const int r = ty + kTvpRows * k, i = i0 + r;
+            Q[k] = P[k];
+            if (i < m && j < n) {
+                const float d = S.D[r][tx];
+                float p1 = i < m - 1 ? fmaf(d - S.D[r + 1][tx], inv8l, S.R1[r + 1][tx]) : 0.0f;
+                float p2 = j < n - 1 ? fmaf(d - S.D[r][tx + 1], inv8l, S.R2[r][tx + 1]) : 0.0f;
+                if (a.iso) {   // P / max(1, |P|): scaled only outside the unit ball
+                    const float q2 = fmaf(p1, p1, p2 * p2);
+                    if (q2 > 1.0f) {
+                        const float rs = rsqrtf(q2);
+                        p1 *= rs;
+                        p2 *= rs;
+                    }
+                } else {
+                    p1 = fminf(fmaxf(p1, -1.0f), 1.0f);
+                    p2 = fminf(fmaxf(p2, -1.0f), 1.0f);
+                }
+                P[k] = make_float2(p1, p2);
+                // only the tile's edge is another block's halo
+                if (r == 0 || r == kTvpH - 1 || tx == 0 || tx == kTvpW - 1) __stcg(N + (size_t)i * n + j, P[k]);
+            }
+        }
+        ok = grid_sums(meet, st.iter + 1, blockIdx.x, gridDim.x, s, S.sums);
+        if (!ok) break;
+        tv_advance(&st, s, a.max_iter, a.eps);
+    }
+    if (!ok) return;
+#pragma unroll
+    for (int k = 0; k < kTvpPer; ++k) {
+        const int r = ty + kTvpRows * k, i = i0 + r;
+        if (i < m && j < n) out[(size_t)i * n + j] = S.D[r][tx];
+    }
+    if (blockIdx.x == 0 && t == 0) {
+        a.st->iter = st.iter;
+        a.st->done = 1;
+    }
+}
+
 // per-block partials of the TV of x (utils/tlv.m): block 32 x 8 over a
 // 32-column, kTvValueRows-row strip
 __global__ void __launch_bounds__(kTvThreads)
@@ -366,6 +521,14 @@ __global__ void k_tv_sum(const double *__restrict__ part, int nblocks, double *_
     sum_partials(part, nblocks, 1, 1, out);
 }
 
+static int tv_loop_tiles(int m, int n)
+{
+    return ((n + kTvpW - 1) / kTvpW) * ((m + kTvpH - 1) / kTvpH);
+}
+
+// the state, and the one-launch loop's failure word and count
+constexpr size_t kTvStateBytes = sizeof(TvState) + 2 * sizeof(int);
+
 int TvWorkspace::alloc(int m, int n, cudaStream_t s)
 {
     if (buf && rows == m && cols == n) return CTPRJ_OK;
@@ -373,11 +536,13 @@ int TvWorkspace::alloc(int m, int n, cudaStream_t s)
     const size_t px = (size_t)m * n;
     const size_t iter_blocks = (size_t)((n + kTvTile - 1) / kTvTile) * ((m + kTvTile - 1) / kTvTile);
     const size_t value_blocks = (size_t)((n + 31) / 32) * ((m + kTvValueRows - 1) / kTvValueRows);
-    blocks = (int)(iter_blocks > value_blocks ? iter_blocks : value_blocks);
+    // the one-launch loop keeps the partials of two iterations
+    const size_t loop_blocks = 2 * (size_t)tv_loop_tiles(m, n);
+    blocks = (int)std::max(std::max(iter_blocks, value_blocks), loop_blocks);
     int st;
     if ((st = cuda_error(cudaMallocAsync((void **)&buf, sizeof(float) * px * 8, s), "TV buffers")) ||
         (st = cuda_error(cudaMallocAsync((void **)&part, sizeof(double) * 4 * (size_t)blocks, s), "TV partials")) ||
-        (st = cuda_error(cudaMallocAsync((void **)&state, sizeof(TvState), s), "TV state"))) {
+        (st = cuda_error(cudaMallocAsync((void **)&state, kTvStateBytes, s), "TV state"))) {
         release(s);
         return st;
     }
@@ -417,12 +582,40 @@ int tv_denoise(TvWorkspace &ws, const float *xobs, int m, int n, double lambda, 
     a.eps = eps;
     a.st = (TvState *)ws.state;
     a.part = ws.part;
+    int dev = 0, sms = 148, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // every tile a block of its own on the GPU at once: the loop in one launch
+    // (12.7 -> 6.1 us per iteration at 512^2, 21 -> 10 at 1024^2, where launches
+    // and the loads' latency took most of it; a round's chain of latencies, 5 us,
+    // is what is left).  Larger images stream through the persistent blocks below.
+    if ((st = cuda_error(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tv_loop, kTvThreads, 0),
+                         "TV occupancy")))
+        return st;
+    if (tv_loop_tiles(m, n) <= sms * per_sm) {
+        struct {
+            TvState st;
+            int failed;
+        } h{};
+        // after the state: the failure word and the count of the meetings
+        int *failed = (int *)(a.st + 1);
+        GridMeet meet = {(unsigned *)(failed + 1), failed, ws.part};
+        const int ntiles = tv_loop_tiles(m, n);
+        int tx = (n + kTvpW - 1) / kTvpW;
+        void *args[] = {&a, &meet, &out, &tx};
+        if ((st = cuda_error(cudaMemsetAsync(a.st, 0, kTvStateBytes, s), "TV start")) ||
+            (st = cuda_error(cudaLaunchCooperativeKernel((void *)k_tv_loop, dim3(ntiles), dim3(kTvThreads), args, 0, s),
+                             "TV loop")) ||
+            (st = cuda_error(cudaMemcpyAsync(&h, a.st, sizeof h, cudaMemcpyDeviceToHost, s), "TV state")) ||
+            (st = cuda_error(cudaStreamSynchronize(s), "TV state")))
+            return st;
+        if (!h.st.done) return set_error(CTPRJ_ETIMEOUT, "the TV loop's blocks did not meet");
+        if (iterations) *iterations = h.st.iter;
+        return CTPRJ_OK;
+    }
     const int tiles_x = (n + kTvTile - 1) / kTvTile, ntiles = tiles_x * ((m + kTvTile - 1) / kTvTile);
     const dim3 block(32, kTvThreads / 32);
     const size_t smem = sizeof(TvSmem);
-    int dev = 0, sms = 148, per_sm = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // 16-byte aligned rows for the vector copies
     const bool vec = n % 4 == 0 && ((uintptr_t)xobs & 15) == 0;
     auto kern = vec ? k_tv_iter<true> : k_tv_iter<false>;
