@@ -14,17 +14,17 @@
 // [0, nc) are skipped as in the reference (prj/parPrj.c:170), and also those
 // beyond prjWidth, which the reference would write past its row.
 //
-//  forward   one thread per (angle, detector), gathering from a dense copy of
-//            the masked image the pixels whose footprint reaches the detector.
-//            Where the detector's band is closer to the rows than to the
-//            columns (|sin| >= |cos|) they are taken column by column and row
-//            by row -- increasing column-major index, the order in which the
-//            reference sums a sorted mask -- otherwise row by row from a
-//            row-major copy, so that the lanes of a warp (adjacent detectors)
-//            always walk their bands in step.  No atomics: results repeat bit
-//            for bit.
-//  backward  one thread per masked pixel, gathering over angles and detectors
-//            in the reference's order; no atomics.
+//  forward   from a dense copy of the masked image, so that the sum does not
+//            depend on the order in which the mask lists its pixels.  Lines of
+//            the image (rows where the angle's band is closer to the columns,
+//            else columns) are taken in turn, the pixels of a line from the
+//            copy in which they are contiguous.  With unit beams a lane owns a
+//            detector edge (edge_lines below); otherwise, and at angles whose
+//            footprint is a box, a detector whose pixels it weighs one by one.
+//            No atomics on sums: results repeat bit for bit.
+//  backward  one thread (or eight) per masked pixel, gathering over angles and
+//            detectors; no atomics.
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -38,18 +38,22 @@ namespace ctprj {
 struct ParView {
     double c, s, height, b1, b2, areaT, areaR;
     double inv_s, inv_c;   // 1 / s and 1 / c, 0 where zero
+    double half, iw;       // half the footprint's area; 1 / (b2 - b1)
+    int edges;             // 1: the edge form below holds (bw = 1, a footprint with ramps)
+    int pad;
 };
 
 struct ParArgs {
     double bw;
     int nc, nr, np, W, xC, yC, pC;
+    int parts;             // warps (thread groups) that share a detector's (pixel's) sum
     const ParView *view;
 };
 
 constexpr double kParPi = 3.14159265;   // prj/parPrj.c:29
 constexpr double kParEps = 1e-8;        // prj/parPrj.h:8
 
-static ParView par_view(double theta)
+static ParView par_view(double theta, double bw)
 {
     ParView v;
     int whole = (int)(fmod(theta, 90) - 45);
@@ -64,6 +68,10 @@ static ParView par_view(double theta)
     v.s = sin(theta * kParPi / 180);
     v.inv_s = v.s != 0.0 ? 1.0 / v.s : 0.0;
     v.inv_c = v.c != 0.0 ? 1.0 / v.c : 0.0;
+    v.half = v.areaT + 0.5 * v.areaR;
+    v.iw = 1.0 / (v.b2 - v.b1);
+    v.edges = bw == 1.0 && v.b2 - v.b1 > 1e-6;
+    v.pad = 0;
     return v;
 }
 
@@ -124,92 +132,236 @@ __global__ void k_par_scatter(const double *__restrict__ x, const double *__rest
     }
 }
 
-// y[it, kk] = (y[it, kk] + sum of w * x over the pixels that reach detector
-// kk) / bw.  The rows a column can contribute are bracketed from
-// |dist - k| <= b2 + bw/2 with a margin; each pixel then takes the reference's
-// own detector range test (prj/parPrj.c:124-125) and weight.
-__global__ void __launch_bounds__(kParThreads)
+// The edge form.  With bw = 1 the beams tile the detector and a beam is never
+// wider than the footprint (2 b2 >= 1), so the reference's overlap is the
+// footprint's area between the beam's two edges, and neighbouring detectors
+// share an edge.  par_area(u): that area from the footprint's centre to u, odd
+// in u, without branches: with z = |u| it is half the area less the falling
+// ramp's rest and the plateau's.  The reference also leaves out a detector
+// whose beam reaches less than 1e-8 into a footprint (prj/parPrj.c:124-125);
+// that sliver weighs below 1e-14 unless the footprint has no ramps (angles that
+// are multiples of 90 degrees), and those angles keep the pixel-by-pixel form.
+__device__ __forceinline__ double par_area(const ParView &v, double u)
+{
+    const double z = fabs(u);
+    const double p = fmin(fmax((v.b2 - z) * v.iw, 0.0), 1.0), m = fmax(v.b1 - z, 0.0);
+    return copysign(fma(-v.height, m, fma(-v.areaT * p, p, v.half)), u);
+}
+
+// sum of w * x over the pixels that reach detector kk, added to acc: the
+// pixel's own range test (prj/parPrj.c:124-125) and weight (:133-168).  The
+// rows a column can contribute are bracketed from |dist - k| <= b2 + bw/2 with
+// a margin.
+__device__ __noinline__ double par_gather(const ParArgs &a, const ParView &v, double k, const double *__restrict__ ximg,
+                                          const double *__restrict__ ximgT, double acc)
+{
+    const double hw = v.b2 + a.bw / 2 + 1e-6;
+    const double ylo = (double)-a.yC, yhi = (double)(a.nr - 1 - a.yC);
+    const double xlo = (double)-a.xC, xhi = (double)(a.nc - 1 - a.xC);
+    auto add = [&](int px, int py, double xv) {
+        if (xv == 0.0) return;
+        const double dist = par_dist(v, px, py);
+        const double ub = floor(dist + v.b2 + a.bw / 2 - kParEps);
+        const double lb = ceil(dist - v.b2 - a.bw / 2 + kParEps);
+        if (k < lb || k > ub) return;
+        const double w = par_overlap(v, dist, k, a.bw);
+        if (w != 0.0) acc += w * xv;
+    };
+    if (fabs(v.s) < fabs(v.c)) {
+        // the band is closer to the columns: row by row, a few columns each
+        for (int ry = 0; ry < a.nr; ++ry) {
+            const int py = ry - a.yC;
+            const double ps = (double)py * v.s;
+            double c0 = (k - hw - ps) * v.inv_c, c1 = (k + hw - ps) * v.inv_c;
+            if (c0 > c1) { const double t = c0; c0 = c1; c1 = t; }
+            const int px0 = (int)ceil(fmax(c0, xlo)), px1 = (int)floor(fmin(c1, xhi));
+            const double *row = ximgT + (size_t)ry * a.nc + a.xC;
+            for (int px = px0; px <= px1; ++px) add(px, py, row[px]);
+        }
+        return acc;
+    }
+    for (int cx = 0; cx < a.nc; ++cx) {
+        const int px = cx - a.xC;
+        const double pc = (double)px * v.c;
+        double r0, r1;
+        if (v.inv_s != 0.0) {
+            r0 = (k - hw - pc) * v.inv_s;
+            r1 = (k + hw - pc) * v.inv_s;
+            if (r0 > r1) { const double t = r0; r0 = r1; r1 = t; }
+        } else if (fabs(pc - k) <= hw) {
+            r0 = ylo;
+            r1 = yhi;
+        } else {
+            continue;
+        }
+        const int py0 = (int)ceil(fmax(r0, ylo)), py1 = (int)floor(fmin(r1, yhi));
+        const double *col = ximg + (size_t)cx * a.nr + a.yC;
+        for (int py = py0; py <= py1; ++py) add(px, py, col[py]);
+    }
+    return acc;
+}
+
+// One warp of the forward: 32 detector edges kk0 - 1/2 + lane of angle v over
+// the lines [l0, l1) of the image (rows where the band is closer to the columns,
+// else columns), 31 detectors.  Per line, with q the pixel index along it in the
+// direction of growing distance, lane e's edge has the pixels q0 .. q0 + 2 whose
+// footprints it cuts (2 b2 / max(|c|, |s|) <= 2 apart); everything before q0
+// lies left of it.  The mass left of the edge is that of the pixels before q0
+// plus S = sum x (area(edge - dist) + half), so detector k's share of the line
+// is 2 half X + S(k + 1) - S(k), X the pixels between the two edges' q0 (one or
+// two, at hand).  Summed over the lines before the lanes meet, so a pixel costs
+// one area instead of two per detector that it might reach (3.3 on average).
+template <bool ROWS>
+__device__ __forceinline__ void edge_lines(const ParArgs &a, const ParView &v, int k, int l0, int l1,
+                                           const double *__restrict__ img, double &S, double &X)
+{
+    // along a line: step per pixel (> 0 in q), offset per line
+    const double along = ROWS ? v.c : v.s, across = ROWS ? v.s : v.c, inv = fabs(ROWS ? v.inv_c : v.inv_s);
+    const int sg = along < 0.0 ? -1 : 1, len = ROWS ? a.nc : a.nr, mid = ROWS ? a.xC : a.yC, lmid = ROWS ? a.yC : a.xC;
+    const double step = fabs(along), kMagic = 6755399441055744.0;   // 1.5 * 2^52: rounds to an integer
+    // first pixel with dist > edge - b2: floor(t) + 1, t = (edge - b2 - offset) / step,
+    // by the same arithmetic for an edge in every lane
+    auto first = [&](int kk, double ps) { return (((double)kk - 0.5) - ps - v.b2) * inv - 0.5 + kMagic; };
+    for (int l = l0; l < l1; ++l) {
+        const double ps = (double)(l - lmid) * across;
+        const double m = first(k, ps), mn = first(k + 1, ps);
+        const int q0 = __double2loint(m) + 1, two = __double2loint(mn) - __double2loint(m);
+        const double u = (((double)k - 0.5) - ps) - step * ((m - kMagic) + 1.0);
+        const double *line = img + (size_t)l * len;
+        double x[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int i = mid + sg * (q0 + j);
+            x[j] = (unsigned)i < (unsigned)len ? __ldg(line + i) : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const double w = par_area(v, fma(-step, (double)j, u)) + v.half;
+            if (w != 0.0) S = fma(w, x[j], S);
+        }
+        X += two > 1 ? x[0] + x[1] : (two == 1 ? x[0] : 0.0);
+    }
+}
+
+// lines of the image that a detector of the warp can meet: offset + along * q
+// = k has |q| <= len / 2 + 4 (every lane takes part)
+__device__ __forceinline__ void clip_lines(double k, double along, double across, int half, int lines, int lmid, int &l0,
+                                           int &l1)
+{
+    float lo = 0.0f, hi = (float)(lines - 1);
+    if (fabs(across) > 1e-6) {
+        const float r = (float)(fabs(along) * (half + 4)), ia = 1.0f / (float)across;
+        const float p = ((float)k - r) * ia, q = ((float)k + r) * ia;
+        lo = fmaxf(lo, fminf(p, q) + (float)lmid - 2.0f);
+        hi = fminf(hi, fmaxf(p, q) + (float)lmid + 2.0f);
+    }
+    l0 = max(l0, __reduce_min_sync(0xffffffffu, lo <= hi ? __float2int_rd(lo) : INT_MAX));
+    l1 = min(l1, __reduce_max_sync(0xffffffffu, lo <= hi ? __float2int_ru(hi) + 1 : INT_MIN));
+}
+
+constexpr int kParWarps = 4;
+
+// y[it, kk] = (y[it, kk] + sum of w * x) / bw.  Block: 4 warps that take the
+// detectors (a.parts = 1) or the lines (4: their sums meet in shared memory, in
+// order) of one angle.
+__global__ void __launch_bounds__(32 * kParWarps)
 k_par_forward(const ParArgs a, const double *__restrict__ ximg, const double *__restrict__ ximgT,
               double *__restrict__ y)
 {
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long long)a.np * a.W) return;
-    const int it = (int)(e / a.W), kk = (int)(e % a.W);
-    double acc = y[e];
-    if (kk < a.nc) {   // detectors with k + centre >= nc are skipped (prj/parPrj.c:170)
-        const ParView v = a.view[it];
-        const double k = (double)(kk - a.pC);
-        const double hw = v.b2 + a.bw / 2 + 1e-6;
-        const double ylo = (double)-a.yC, yhi = (double)(a.nr - 1 - a.yC);
-        const double xlo = (double)-a.xC, xhi = (double)(a.nc - 1 - a.xC);
-        // the pixel's own range test and weight (prj/parPrj.c:124-125, :133-168)
-        auto add = [&](int px, int py, double xv) {
-            if (xv == 0.0) return;
-            const double dist = par_dist(v, px, py);
-            const double ub = floor(dist + v.b2 + a.bw / 2 - kParEps);
-            const double lb = ceil(dist - v.b2 - a.bw / 2 + kParEps);
-            if (k < lb || k > ub) return;
-            const double w = par_overlap(v, dist, k, a.bw);
-            if (w != 0.0) acc += w * xv;
-        };
-        if (fabs(v.s) < fabs(v.c)) {
-            // the band is closer to the columns: row by row, a few columns each
-            for (int ry = 0; ry < a.nr; ++ry) {
-                const int py = ry - a.yC;
-                const double ps = (double)py * v.s;
-                double c0 = (k - hw - ps) * v.inv_c, c1 = (k + hw - ps) * v.inv_c;
-                if (c0 > c1) { const double t = c0; c0 = c1; c1 = t; }
-                const int px0 = (int)ceil(fmax(c0, xlo)), px1 = (int)floor(fmin(c1, xhi));
-                const double *row = ximgT + (size_t)ry * a.nc + a.xC;
-                for (int px = px0; px <= px1; ++px) add(px, py, row[px]);
-            }
-            y[e] = acc / a.bw;
-            return;
-        }
-        for (int cx = 0; cx < a.nc; ++cx) {
-            const int px = cx - a.xC;
-            const double pc = (double)px * v.c;
-            double r0, r1;
-            if (v.inv_s != 0.0) {
-                r0 = (k - hw - pc) * v.inv_s;
-                r1 = (k + hw - pc) * v.inv_s;
-                if (r0 > r1) { const double t = r0; r0 = r1; r1 = t; }
-            } else if (fabs(pc - k) <= hw) {
-                r0 = ylo;
-                r1 = yhi;
-            } else {
-                continue;
-            }
-            const int py0 = (int)ceil(fmax(r0, ylo)), py1 = (int)floor(fmin(r1, yhi));
-            const double *col = ximg + (size_t)cx * a.nr + a.yC;
-            for (int py = py0; py <= py1; ++py) add(px, py, col[py]);
+    __shared__ double sums[kParWarps][2][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, it = blockIdx.y;
+    const int parts = a.parts, part = warp % parts, group = blockIdx.x * (kParWarps / parts) + warp / parts;
+    const ParView v = a.view[it];
+    const int nd = min(a.W, a.nc);   // detectors with k + centre >= nc are skipped (prj/parPrj.c:170)
+    const int kk = group * 31 + lane, k = kk - a.pC;
+    double *yr = y + (size_t)it * a.W;
+    double S = 0.0, X = 0.0;
+    if (v.edges) {
+        const bool rows = fabs(v.s) < fabs(v.c);
+        const int lines = rows ? a.nr : a.nc, lmid = rows ? a.yC : a.xC;
+        int l0 = (int)((long long)lines * part / parts), l1 = (int)((long long)lines * (part + 1) / parts);
+        clip_lines((double)k, rows ? v.c : v.s, rows ? v.s : v.c, max(a.xC, a.yC) + 1, lines, lmid, l0, l1);
+        if (group * 31 < nd) {
+            if (rows) edge_lines<true>(a, v, k, l0, l1, ximgT, S, X);
+            else edge_lines<false>(a, v, k, l0, l1, ximg, S, X);
         }
     }
-    y[e] = acc / a.bw;
+    if (parts > 1) {
+        sums[warp][0][lane] = S;
+        sums[warp][1][lane] = X;
+        __syncthreads();
+        if (part != 0) return;
+        for (int q = 1; q < parts; ++q) {
+            S += sums[warp + q][0][lane];
+            X += sums[warp + q][1][lane];
+        }
+    }
+    const double Sn = __shfl_down_sync(0xffffffffu, S, 1);
+    if (lane < 31 && kk < nd) {
+        double r = yr[kk] + fma(2.0 * v.half, X, Sn - S);
+        // no edge form at this angle; or a value that is not finite, whose
+        // neighbours' sums it must not reach
+        if (!v.edges || !isfinite(r)) r = par_gather(a, v, (double)k, ximg, ximgT, yr[kk]);
+        yr[kk] = r / a.bw;
+    }
+    if (group == 0)   // the detectors that are skipped
+        for (int e = nd + lane; e < a.W; e += 32) yr[e] /= a.bw;
+}
+
+// x = (x + sum of w * y) / bw over angles and detectors.  In the edge form a
+// footprint is cut by the edges e1 and e2 of at most three detectors k0 .. k0 + 2
+// (2 b2 + 1 <= 2.42); the outer edges lie outside it but for 1e-8.
+__device__ __forceinline__ double par_back_angle(const ParArgs &a, const ParView &v, const double *__restrict__ row,
+                                                 int px, int py, double acc)
+{
+    const double dist = par_dist(v, px, py);
+    const double ub = floor(dist + v.b2 + a.bw / 2 - kParEps);
+    const double lb = ceil(dist - v.b2 - a.bw / 2 + kParEps);
+    for (int k = (int)lb; k <= ub; ++k) {
+        if (k < -a.pC || k + a.pC >= a.nc || k + a.pC >= a.W) continue;
+        const double w = par_overlap(v, dist, (double)k, a.bw);
+        if (w != 0.0) acc += row[k + a.pC] * w;
+    }
+    return acc;
 }
 
 __global__ void __launch_bounds__(kParThreads)
 k_par_backward(const ParArgs a, const double *__restrict__ y, const double *__restrict__ mask,
                long long npix, double *__restrict__ x)
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npix) return;
-    const int m = (int)mask[i];
+    __shared__ double part[kParThreads];
+    const int parts = a.parts, per = kParThreads / parts;
+    const int p = threadIdx.x / per, t = threadIdx.x % per;
+    const long long i = (long long)blockIdx.x * per + t;
+    const bool live = i < npix;
+    const int m = live ? (int)mask[i] : 0;
     const int px = m / a.nr - a.xC, py = m % a.nr - a.yC;
-    double acc = x[i];
-    for (int it = 0; it < a.np; ++it) {
+    const unsigned nd = (unsigned)min(a.W, a.nc);
+    const int it0 = (int)((long long)a.np * p / parts), it1 = (int)((long long)a.np * (p + 1) / parts);
+    double acc = live && p == 0 ? x[i] : 0.0;
+    for (int it = it0; it < it1; ++it) {
         const ParView &v = a.view[it];
-        const double dist = par_dist(v, px, py);
-        const double ub = floor(dist + v.b2 + a.bw / 2 - kParEps);
-        const double lb = ceil(dist - v.b2 - a.bw / 2 + kParEps);
-        const double *rowp = y + (size_t)it * a.W;
-        for (int k = (int)lb; k <= ub; ++k) {
-            if (k < -a.pC || k + a.pC >= a.nc || k + a.pC >= a.W) continue;
-            const double w = par_overlap(v, dist, (double)k, a.bw);
-            if (w != 0.0) acc += rowp[k + a.pC] * w;
+        const double *row = y + (size_t)it * a.W;
+        if (!v.edges) {
+            if (live) acc = par_back_angle(a, v, row, px, py, acc);
+            continue;
         }
+        const double dist = par_dist(v, px, py);
+        const double k0 = ceil(dist - v.b2 - 0.5 + kParEps);
+        const int d0 = (int)k0 + a.pC;
+        const double F1 = par_area(v, k0 + 0.5 - dist), F2 = par_area(v, k0 + 1.5 - dist);
+        const double w0 = F1 + v.half, w1 = F2 - F1, w2 = v.half - F2;
+        if ((unsigned)d0 < nd && w0 != 0.0) acc = fma(w0, __ldg(row + d0), acc);
+        if ((unsigned)(d0 + 1) < nd && w1 != 0.0) acc = fma(w1, __ldg(row + d0 + 1), acc);
+        if ((unsigned)(d0 + 2) < nd && w2 != 0.0) acc = fma(w2, __ldg(row + d0 + 2), acc);
     }
-    x[i] = acc / a.bw;
+    if (parts > 1) {
+        part[threadIdx.x] = acc;
+        __syncthreads();
+        if (p != 0) return;
+        for (int q = 1; q < parts; ++q) acc += part[q * per + t];
+    }
+    if (live) x[i] = acc / a.bw;
 }
 
 static int par_validate(const ctprj_par_conf *c, long long npix)
@@ -242,7 +394,7 @@ static ParArgs par_args(const ctprj_par_conf *c, const ParView *view)
 static int par_table(const ctprj_par_conf *c, const double *theta, ParView **d_view, cudaStream_t s)
 {
     std::vector<ParView> tab((size_t)(c->np > 0 ? c->np : 1));
-    for (int it = 0; it < c->np; ++it) tab[it] = par_view(theta[it]);
+    for (int it = 0; it < c->np; ++it) tab[it] = par_view(theta[it], c->bw);
     int st = cuda_error(cudaMallocAsync((void **)d_view, sizeof(ParView) * tab.size(), s),
                         "parPrj view table");
     if (st) return st;
@@ -276,7 +428,7 @@ extern "C" int ctprj_par_forward(const ctprj_par_conf *conf, const double *theta
     ParView *d_view = nullptr;
     double *d_img = nullptr;
     if ((st = par_table(conf, theta_host, &d_view, s))) return st;
-    const ParArgs a = par_args(conf, d_view);
+    ParArgs a = par_args(conf, d_view);
     const size_t img_elems = (size_t)conf->nc * (size_t)conf->nr, img_bytes = 2 * sizeof(double) * img_elems;
     if (!(st = cuda_error(cudaMallocAsync((void **)&d_img, img_bytes, s), "parPrj dense image")) &&
         !(st = cuda_error(cudaMemsetAsync(d_img, 0, img_bytes, s), "parPrj dense image"))) {
@@ -287,10 +439,19 @@ extern "C" int ctprj_par_forward(const ctprj_par_conf *conf, const double *theta
             st = cuda_error(cudaGetLastError(), "parPrj scatter");
         }
         if (!st) {
-            const long long ny = (long long)conf->np * conf->prjWidth;
-            k_par_forward<<<(int)((ny + kParThreads - 1) / kParThreads), kParThreads, 0, s>>>(
-                a, d_img, d_img + img_elems, d_y);
-            st = cuda_error(cudaGetLastError(), "parPrj forward");
+            // a warp per 31 detectors and angle; few of them share each one's
+            // lines among four warps (64^2, 64 angles: 192 warps)
+            const int nd = conf->prjWidth < conf->nc ? conf->prjWidth : conf->nc, groups = (nd + 30) / 31;
+            a.parts = (long long)groups * conf->np < 24LL * sm_count() ? kParWarps : 1;
+            const int per = kParWarps / a.parts;
+            for (int it0 = 0; it0 < conf->np && !st; it0 += 65535) {
+                ParArgs b = a;
+                b.view += it0;
+                b.np = conf->np - it0 < 65535 ? conf->np - it0 : 65535;
+                k_par_forward<<<dim3((groups + per - 1) / per, b.np), 32 * kParWarps, 0, s>>>(
+                    b, d_img, d_img + img_elems, d_y + (size_t)it0 * conf->prjWidth);
+                st = cuda_error(cudaGetLastError(), "parPrj forward");
+            }
         }
     }
     if (d_img) cudaFreeAsync(d_img, s);
@@ -310,8 +471,10 @@ extern "C" int ctprj_par_backward(const ctprj_par_conf *conf, const double *thet
     cudaStream_t s = (cudaStream_t)stream;
     ParView *d_view = nullptr;
     if ((st = par_table(conf, theta_host, &d_view, s))) return st;
-    const ParArgs a = par_args(conf, d_view);
-    const int blocks = (int)((npix + kParThreads - 1) / kParThreads);
+    ParArgs a = par_args(conf, d_view);
+    // few pixels share each one's angles among eight threads
+    a.parts = npix < 384LL * sm_count() ? 8 : 1;
+    const int per = kParThreads / a.parts, blocks = (int)((npix + per - 1) / per);
     k_par_backward<<<blocks, kParThreads, 0, s>>>(a, d_y, d_mask, npix, d_x);
     st = cuda_error(cudaGetLastError(), "parPrj backward");
     cudaFreeAsync(d_view, s);
