@@ -19,8 +19,8 @@
 //            the image (rows where the angle's band is closer to the columns,
 //            else columns) are taken in turn, the pixels of a line from the
 //            copy in which they are contiguous.  With unit beams a lane owns a
-//            detector edge (edge_lines below); otherwise, and at angles whose
-//            footprint is a box, a detector whose pixels it weighs one by one.
+//            detector edge (edge_lines below); otherwise a detector whose
+//            pixels it weighs one by one.
 //            No atomics on sums: results repeat bit for bit.
 //  backward  one thread (or eight) per masked pixel, gathering over angles and
 //            detectors; no atomics.
@@ -38,9 +38,9 @@ namespace ctprj {
 struct ParView {
     double c, s, height, b1, b2, areaT, areaR;
     double inv_s, inv_c;   // 1 / s and 1 / c, 0 where zero
-    double half, iw;       // half the footprint's area; 1 / (b2 - b1)
-    int edges;             // 1: the edge form below holds (bw = 1, a footprint with ramps)
-    int pad;
+    double half, ramp;     // half the footprint's area; height / (2 (b2 - b1))
+    int edges;             // 1: the edge form below holds (bw = 1, 1/2 <= b2, b1 < b2)
+    int box;               // 1: and the footprint has next to no ramps
 };
 
 struct ParArgs {
@@ -69,9 +69,11 @@ static ParView par_view(double theta, double bw)
     v.inv_s = v.s != 0.0 ? 1.0 / v.s : 0.0;
     v.inv_c = v.c != 0.0 ? 1.0 / v.c : 0.0;
     v.half = v.areaT + 0.5 * v.areaR;
-    v.iw = 1.0 / (v.b2 - v.b1);
-    v.edges = bw == 1.0 && v.b2 - v.b1 > 1e-6;
-    v.pad = 0;
+    v.ramp = 0.5 * v.height / (v.b2 - v.b1);
+    // (negative angles get footprints with b2 < b1 from the truncated angle:
+    // those keep the reference's piecewise formula)
+    v.edges = bw == 1.0 && v.b2 > v.b1 && v.b2 >= 0.5;
+    v.box = v.edges && v.b2 - v.b1 < 1e-6;
     return v;
 }
 
@@ -136,16 +138,18 @@ __global__ void k_par_scatter(const double *__restrict__ x, const double *__rest
 // wider than the footprint (2 b2 >= 1), so the reference's overlap is the
 // footprint's area between the beam's two edges, and neighbouring detectors
 // share an edge.  par_area(u): that area from the footprint's centre to u, odd
-// in u, without branches: with z = |u| it is half the area less the falling
-// ramp's rest and the plateau's.  The reference also leaves out a detector
-// whose beam reaches less than 1e-8 into a footprint (prj/parPrj.c:124-125);
-// that sliver weighs below 1e-14 unless the footprint has no ramps (angles that
-// are multiples of 90 degrees), and those angles keep the pixel-by-pixel form.
+// in u, without branches: with z = |u|, half the area less what lies beyond z,
+// which is quadratic on the falling ramp and linear on the plateau.  The
+// reference also leaves out a detector whose beam reaches less than 1e-8 into a
+// footprint (prj/parPrj.c:124-125).  That sliver weighs below 1e-14 unless the
+// footprint is a box (angles that are multiples of 90 degrees); there the edge of
+// a beam that is left out counts as outside the footprint.
 __device__ __forceinline__ double par_area(const ParView &v, double u)
 {
-    const double z = fabs(u);
-    const double p = fmin(fmax((v.b2 - z) * v.iw, 0.0), 1.0), m = fmax(v.b1 - z, 0.0);
-    return copysign(fma(-v.height, m, fma(-v.areaT * p, p, v.half)), u);
+    const double z = fabs(u), q = v.b2 - z;
+    const double r = q < 0.0 ? 0.0 : q;
+    const double rest = z < v.b1 ? fma(v.height, v.b1 - z, v.areaT) : v.ramp * r * r;
+    return copysign(v.half - rest, u);
 }
 
 // sum of w * x over the pixels that reach detector kk, added to acc: the
@@ -211,9 +215,14 @@ __device__ __noinline__ double par_gather(const ParArgs &a, const ParView &v, do
 // is 2 half X + S(k + 1) - S(k), X the pixels between the two edges' q0 (one or
 // two, at hand).  Summed over the lines before the lanes meet, so a pixel costs
 // one area instead of two per detector that it might reach (3.3 on average).
-template <bool ROWS>
+// Bound by the FP64 pipe and the selects around it (51 % and 44 % busy): 1.57 ->
+// 0.51 ms at 512^2, 360 angles; the backward, whose samples come from L2, 1.11 ->
+// 0.31 ms.  64^2, 40 angles: 116 -> 27 and 71 -> 19 us.
+// S: of the edge as a beam's left one; Sr: as the right one, which differs at box
+// angles only.
+template <bool ROWS, bool BOX>
 __device__ __forceinline__ void edge_lines(const ParArgs &a, const ParView &v, int k, int l0, int l1,
-                                           const double *__restrict__ img, double &S, double &X)
+                                           const double *__restrict__ img, double &S, double &Sr, double &X)
 {
     // along a line: step per pixel (> 0 in q), offset per line
     const double along = ROWS ? v.c : v.s, across = ROWS ? v.s : v.c, inv = fabs(ROWS ? v.inv_c : v.inv_s);
@@ -222,6 +231,7 @@ __device__ __forceinline__ void edge_lines(const ParArgs &a, const ParView &v, i
     // first pixel with dist > edge - b2: floor(t) + 1, t = (edge - b2 - offset) / step,
     // by the same arithmetic for an edge in every lane
     auto first = [&](int kk, double ps) { return (((double)kk - 0.5) - ps - v.b2) * inv - 0.5 + kMagic; };
+#pragma unroll 2
     for (int l = l0; l < l1; ++l) {
         const double ps = (double)(l - lmid) * across;
         const double m = first(k, ps), mn = first(k + 1, ps);
@@ -236,8 +246,11 @@ __device__ __forceinline__ void edge_lines(const ParArgs &a, const ParView &v, i
         }
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            const double w = par_area(v, fma(-step, (double)j, u)) + v.half;
-            if (w != 0.0) S = fma(w, x[j], S);
+            // (an infinite pixel turns the sums of the edges near it into NaN:
+            // the caller takes those detectors pixel by pixel)
+            const double uj = fma(-step, (double)j, u), f = par_area(v, uj) + v.half;
+            S = fma(BOX && uj > v.b2 - kParEps ? 2.0 * v.half : f, x[j], S);
+            if (BOX) Sr = fma(uj < -v.b2 + kParEps ? 0.0 : f, x[j], Sr);
         }
         X += two > 1 ? x[0] + x[1] : (two == 1 ? x[0] : 0.0);
     }
@@ -268,39 +281,47 @@ __global__ void __launch_bounds__(32 * kParWarps)
 k_par_forward(const ParArgs a, const double *__restrict__ ximg, const double *__restrict__ ximgT,
               double *__restrict__ y)
 {
-    __shared__ double sums[kParWarps][2][32];
+    __shared__ double sums[kParWarps][3][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, it = blockIdx.y;
     const int parts = a.parts, part = warp % parts, group = blockIdx.x * (kParWarps / parts) + warp / parts;
     const ParView v = a.view[it];
     const int nd = min(a.W, a.nc);   // detectors with k + centre >= nc are skipped (prj/parPrj.c:170)
     const int kk = group * 31 + lane, k = kk - a.pC;
     double *yr = y + (size_t)it * a.W;
-    double S = 0.0, X = 0.0;
+    double S = 0.0, Sr = 0.0, X = 0.0;
     if (v.edges) {
         const bool rows = fabs(v.s) < fabs(v.c);
         const int lines = rows ? a.nr : a.nc, lmid = rows ? a.yC : a.xC;
         int l0 = (int)((long long)lines * part / parts), l1 = (int)((long long)lines * (part + 1) / parts);
         clip_lines((double)k, rows ? v.c : v.s, rows ? v.s : v.c, max(a.xC, a.yC) + 1, lines, lmid, l0, l1);
         if (group * 31 < nd) {
-            if (rows) edge_lines<true>(a, v, k, l0, l1, ximgT, S, X);
-            else edge_lines<false>(a, v, k, l0, l1, ximg, S, X);
+            if (v.box) {
+                if (rows) edge_lines<true, true>(a, v, k, l0, l1, ximgT, S, Sr, X);
+                else edge_lines<false, true>(a, v, k, l0, l1, ximg, S, Sr, X);
+            } else {
+                if (rows) edge_lines<true, false>(a, v, k, l0, l1, ximgT, S, Sr, X);
+                else edge_lines<false, false>(a, v, k, l0, l1, ximg, S, Sr, X);
+                Sr = S;
+            }
         }
     }
     if (parts > 1) {
         sums[warp][0][lane] = S;
         sums[warp][1][lane] = X;
+        sums[warp][2][lane] = Sr;
         __syncthreads();
         if (part != 0) return;
         for (int q = 1; q < parts; ++q) {
             S += sums[warp + q][0][lane];
             X += sums[warp + q][1][lane];
+            Sr += sums[warp + q][2][lane];
         }
     }
-    const double Sn = __shfl_down_sync(0xffffffffu, S, 1);
+    const double Sn = __shfl_down_sync(0xffffffffu, Sr, 1);
     if (lane < 31 && kk < nd) {
         double r = yr[kk] + fma(2.0 * v.half, X, Sn - S);
-        // no edge form at this angle; or a value that is not finite, whose
-        // neighbours' sums it must not reach
+        // no edge form with this beam; or a value that is not finite, which
+        // must not reach the neighbours' sums
         if (!v.edges || !isfinite(r)) r = par_gather(a, v, (double)k, ximg, ximgT, yr[kk]);
         yr[kk] = r / a.bw;
     }
@@ -311,7 +332,7 @@ k_par_forward(const ParArgs a, const double *__restrict__ ximg, const double *__
 // x = (x + sum of w * y) / bw over angles and detectors.  In the edge form a
 // footprint is cut by the edges e1 and e2 of at most three detectors k0 .. k0 + 2
 // (2 b2 + 1 <= 2.42); the outer edges lie outside it but for 1e-8.
-__device__ __forceinline__ double par_back_angle(const ParArgs &a, const ParView &v, const double *__restrict__ row,
+__device__ __noinline__ double par_back_angle(const ParArgs &a, const ParView &v, const double *__restrict__ row,
                                                  int px, int py, double acc)
 {
     const double dist = par_dist(v, px, py);
@@ -325,11 +346,14 @@ __device__ __forceinline__ double par_back_angle(const ParArgs &a, const ParView
     return acc;
 }
 
+constexpr int kParViews = 64;
+
 __global__ void __launch_bounds__(kParThreads)
 k_par_backward(const ParArgs a, const double *__restrict__ y, const double *__restrict__ mask,
                long long npix, double *__restrict__ x)
 {
     __shared__ double part[kParThreads];
+    __shared__ ParView views[kParViews];
     const int parts = a.parts, per = kParThreads / parts;
     const int p = threadIdx.x / per, t = threadIdx.x % per;
     const long long i = (long long)blockIdx.x * per + t;
@@ -337,23 +361,45 @@ k_par_backward(const ParArgs a, const double *__restrict__ y, const double *__re
     const int m = live ? (int)mask[i] : 0;
     const int px = m / a.nr - a.xC, py = m % a.nr - a.yC;
     const unsigned nd = (unsigned)min(a.W, a.nc);
-    const int it0 = (int)((long long)a.np * p / parts), it1 = (int)((long long)a.np * (p + 1) / parts);
     double acc = live && p == 0 ? x[i] : 0.0;
-    for (int it = it0; it < it1; ++it) {
-        const ParView &v = a.view[it];
-        const double *row = y + (size_t)it * a.W;
-        if (!v.edges) {
-            if (live) acc = par_back_angle(a, v, row, px, py, acc);
-            continue;
+    // the views in turns of kParViews through shared memory, of which each part
+    // takes a run
+    for (int base = 0; base < a.np; base += kParViews) {
+        const int n = min(kParViews, a.np - base);
+        __syncthreads();
+        const double *src = reinterpret_cast<const double *>(a.view + base);
+        for (int e = threadIdx.x; e < n * (int)(sizeof(ParView) / sizeof(double)); e += kParThreads)
+            reinterpret_cast<double *>(views)[e] = src[e];
+        __syncthreads();
+        const int q0 = n * p / parts, q1 = n * (p + 1) / parts;
+        const double *row = y + (size_t)(base + q0) * a.W;
+#pragma unroll 2
+        for (int q = q0; q < q1; ++q, row += a.W) {
+            const ParView &v = views[q];
+            if (!v.edges) {
+                if (live) acc = par_back_angle(a, v, row, px, py, acc);
+                continue;
+            }
+            const double dist = par_dist(v, px, py);
+            const double k0 = ceil(dist - v.b2 - 0.5 + kParEps);
+            const int d0 = (int)k0 + a.pC;
+            const double y0 = (unsigned)d0 < nd ? __ldg(row + d0) : 0.0;
+            const double y1 = (unsigned)(d0 + 1) < nd ? __ldg(row + d0 + 1) : 0.0;
+            const double y2 = (unsigned)(d0 + 2) < nd ? __ldg(row + d0 + 2) : 0.0;
+            const double F1 = par_area(v, k0 + 0.5 - dist), F2 = par_area(v, k0 + 1.5 - dist);
+            double w0 = F1 + v.half, w1 = F2 - F1, w2 = v.half - F2;
+            if (v.box) {   // the outer edges may lie 1e-8 inside, and a sliver is left out
+                const double e0 = k0 - 0.5 - dist, ub = floor(dist + v.b2 + 0.5 - kParEps);
+                const double F0 = par_area(v, e0), F3 = par_area(v, e0 + 3.0);
+                w0 = F1 - F0;
+                if (k0 + 1.0 > ub) w1 = 0.0;
+                w2 = k0 + 2.0 > ub ? 0.0 : F3 - F2;
+                if (k0 > ub) w0 = 0.0;
+            }
+            if (w0 != 0.0) acc = fma(w0, y0, acc);
+            if (w1 != 0.0) acc = fma(w1, y1, acc);
+            if (w2 != 0.0) acc = fma(w2, y2, acc);
         }
-        const double dist = par_dist(v, px, py);
-        const double k0 = ceil(dist - v.b2 - 0.5 + kParEps);
-        const int d0 = (int)k0 + a.pC;
-        const double F1 = par_area(v, k0 + 0.5 - dist), F2 = par_area(v, k0 + 1.5 - dist);
-        const double w0 = F1 + v.half, w1 = F2 - F1, w2 = v.half - F2;
-        if ((unsigned)d0 < nd && w0 != 0.0) acc = fma(w0, __ldg(row + d0), acc);
-        if ((unsigned)(d0 + 1) < nd && w1 != 0.0) acc = fma(w1, __ldg(row + d0 + 1), acc);
-        if ((unsigned)(d0 + 2) < nd && w2 != 0.0) acc = fma(w2, __ldg(row + d0 + 2), acc);
     }
     if (parts > 1) {
         part[threadIdx.x] = acc;
