@@ -57,6 +57,32 @@ constexpr int kBwdTile = 16;   // 16 x 16 octant pixels per block
 enum { kBwdUnit = 0, kBwdNarrow = 1, kBwdRange = 2 };
 constexpr int kBwdTablePad = 80;   // zero entries beyond the detectors at each end of a table row
 
+// Each pass is two launches, a table of its input and the pass itself, of which
+// the second may start while the first runs (programmatic dependent launch): the
+// first lets it at once, the second prepares its geometry and waits for the
+// first's end where it needs the table.  The first is an ordinary launch, so
+// everything before it in the stream has ended.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_table() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+static cudaError_t launch_after_table(void (*kern)(P...), dim3 grid, int threads, int cluster, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&c, kern, args...);
+}
+
 // --------------------------------------------------------------- quad image
 
 // The forward pass reads, for each pixel (x, y) a ray crosses, the eight images
@@ -98,6 +124,7 @@ __device__ __forceinline__ void quad_tile(const float *__restrict__ img, float4 
 __global__ void __launch_bounds__(256) k_quad(const float *__restrict__ img, float4 *__restrict__ Q, int n)
 {
     __shared__ float tz[32][33], tw[32][33];
+    let_next_start();
     quad_tile(img, Q, n, blockIdx.x, tz, tw);
 }
 
@@ -486,6 +513,7 @@ __device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int b
         }
     }
     wcode = __reduce_max_sync(0xffffffffu, wcode);
+    if (R != kAllParts) wait_for_table();   // the quad image
     float S[8];
     unsigned long long nz = 0;
     auto rows_of = [&](int s) {
@@ -647,14 +675,14 @@ int forward_blocks(const ctprj_plan *pl)
 }
 
 template <bool FAN, int MODE>
-static void launch_forward_t(const FwdParams &p, dim3 grid, const float4 *quad, float *sino,
-                             unsigned long long *counter, cudaStream_t s)
+static cudaError_t launch_forward_t(const FwdParams &p, dim3 grid, const float4 *quad, float *sino,
+                                    unsigned long long *counter, cudaStream_t s)
 {
     switch (p.rsplit) {
-    case 1: k_forward<FAN, MODE, kFwdViews, 1><<<grid, kFwdThreads, 0, s>>>(p, quad, sino, counter); break;
-    case 2: k_forward<FAN, MODE, kFwdViews / 2, 2><<<grid, kFwdThreads, 0, s>>>(p, quad, sino, counter); break;
-    case 4: k_forward<FAN, MODE, 1, 4><<<grid, kFwdThreads, 0, s>>>(p, quad, sino, counter); break;
-    default: k_forward<FAN, MODE, 1, 8><<<grid, 256, 0, s>>>(p, quad, sino, counter); break;
+    case 1: return launch_after_table(k_forward<FAN, MODE, kFwdViews, 1>, grid, kFwdThreads, 1, s, p, quad, sino, counter);
+    case 2: return launch_after_table(k_forward<FAN, MODE, kFwdViews / 2, 2>, grid, kFwdThreads, 1, s, p, quad, sino, counter);
+    case 4: return launch_after_table(k_forward<FAN, MODE, 1, 4>, grid, kFwdThreads, 1, s, p, quad, sino, counter);
+    default: return launch_after_table(k_forward<FAN, MODE, 1, 8>, grid, 256, 1, s, p, quad, sino, counter);
     }
 }
 
@@ -670,8 +698,9 @@ int launch_forward(const ctprj_plan *pl, const float4 *quad, float *sino,
         else k_forward<false, kModeCount, kFwdViews, 1><<<grid, kFwdThreads, 0, s>>>(p, quad, sino, counter);
     } else {
         const dim3 grid = fwd_grid(pl, p.rsplit);
-        if (fan) launch_forward_t<true, kModePlain>(p, grid, quad, sino, counter, s);
-        else launch_forward_t<false, kModePlain>(p, grid, quad, sino, counter, s);
+        const cudaError_t e = fan ? launch_forward_t<true, kModePlain>(p, grid, quad, sino, counter, s)
+                                  : launch_forward_t<false, kModePlain>(p, grid, quad, sino, counter, s);
+        if (e != cudaSuccess) return cuda_error(e, "forward launch");
     }
     return cuda_error(cudaGetLastError(), "forward launch");
 }
@@ -682,10 +711,10 @@ int launch_forward_bhc(const ctprj_plan *pl, const float4 *quad,
     FwdParams p = fwd_params(pl);
     p.bhc = a;
     const dim3 grid = fwd_grid(pl, p.rsplit);
-    if (pl->g.fan) launch_forward_t<true, kModeBhc>(p, grid, quad, nullptr, nullptr, s);
-    else launch_forward_t<false, kModeBhc>(p, grid, quad, nullptr, nullptr, s);
+    const cudaError_t e = pl->g.fan ? launch_forward_t<true, kModeBhc>(p, grid, quad, nullptr, nullptr, s)
+                                    : launch_forward_t<false, kModeBhc>(p, grid, quad, nullptr, nullptr, s);
     if (nparts) *nparts = (int)(grid.x * grid.y);
-    return cuda_error(cudaGetLastError(), "fused polychromatic forward launch");
+    return cuda_error(e, "fused polychromatic forward launch");
 }
 
 // ---------------------------------------------------------------- backward
@@ -1035,6 +1064,10 @@ constexpr int kSampThreads = 128;
 
 __global__ void __launch_bounds__(kSampThreads) k_samples(const BwdParams p, const float *__restrict__ sino)
 {
+    // Started beside this kernel, a large backprojection's blocks crowd onto the SMs
+    // it leaves free and stay there (256^2 20.5 -> 25.6 us, 512^2 fan 68 -> 78); at
+    // one block per SM the early start is worth 2 of 12 us (64^2)
+    if (p.tiles_side * (p.tiles_side + 1) / 2 * p.split <= 128) let_next_start();
     for (int i = blockIdx.y; i < p.g.P / 4; i += gridDim.y)
         sample_row(p, sino, i, blockIdx.x * kSampThreads + threadIdx.x, gridDim.x * kSampThreads);
 }
@@ -1220,31 +1253,33 @@ __device__ __forceinline__ void pair_view(const BwdParams &p, const PairView &v,
     const float4 *s0 = seg + v.i0, *s1 = s0 + SEG + 2 * kBwdPast, *fp = s1 + SEG + 2 * kBwdPast;
     const float hb = 0.5f * p.g.effRate;
     const float fA = fbp_weight<FAN, FBP>(p, v.GA), fB = fbp_weight<FAN, FBP>(p, v.GB);
-    // left edges of the first detectors; parallel beam: the areas up to them
-    float eA = fmaf(v.cb + ((float)OA - hb), v.GA, -v.EA), eB = fmaf(v.cb + ((float)OB - hb), v.GB, -v.EB);
+    // left edges of the first detectors (a window's edges are a few pitches from
+    // them); parallel beam: the areas up to them
+    const float aA = fmaf(v.cb + ((float)OA - hb), v.GA, -v.EA), aB = fmaf(v.cb + ((float)OB - hb), v.GB, -v.EB);
+    float eA = aA, eB = aB;
     if (!FAN && UNIT) {
         eA = edge_area(eA, fpar);
         eB = edge_area(eB, fpar);
     }
-    // weight of slot j: its right edge becomes the next slot's left one
-    auto weight = [&](float &e, int j, float G, float E, float4 f) {
-        const float r = fmaf(v.cb + ((float)j + hb), G, -E), l = e;
+    // weight of the window's j-th detector: its right edge becomes the next one's left
+    auto weight = [&](float &e, int j, float G, float a, float4 f) {
+        const float r = fmaf((float)j + (UNIT ? 1.0f : p.g.effRate), G, a), l = e;
         if (!FAN && UNIT) {
             e = edge_area(r, f);
             return e - l;
         }
-        e = UNIT ? r : fmaf(v.cb + ((float)(j + 1) - hb), G, -E);
+        e = UNIT ? r : fmaf((float)(j + 1), G, a);
         return edge_weight(l, r, f);
     };
 #pragma unroll
     for (int j = 0; j < U; ++j) {
         const float4 f = FAN ? fp[j] : fpar, p0 = s0[j], p1 = s1[j];
         if (j >= OA && j < OA + N) {
-            const float w = weight(eA, j, v.GA, v.EA, f);
+            const float w = weight(eA, j - OA, v.GA, aA, f);
             add_samples(A, FBP && FAN ? w * fA : w, p0, p1);
         }
         if (j >= OB && j < OB + N) {
-            const float w = weight(eB, j, v.GB, v.EB, f);
+            const float w = weight(eB, j - OB, v.GB, aB, f);
             add_samples(B, FBP && FAN ? w * fB : w, p0, p1);
         }
     }
@@ -1387,6 +1422,7 @@ __device__ __forceinline__ void quarter_sums(const BwdParams &p, int tx, int ty,
     };
     const int nbatch = (v1 - v0 + VB - 1) / VB;
     prepare(0);
+    wait_for_table();   // the sample image (nothing to wait for but in the first quarter)
     stage(0);
     for (int b = 0; b < nbatch; ++b) {
         const bool more = b + 1 < nbatch;
@@ -1652,17 +1688,8 @@ static void launch_samples(const BwdParams &p, const float *sino, cudaStream_t s
 template <bool FAN, bool FBP, int SEG, int VB, int MODE>
 static cudaError_t launch_tiled_t(const BwdParams &p, int tiles, float *img, cudaStream_t s)
 {
-    cudaLaunchConfig_t c = {};
-    c.gridDim = dim3(tiles * p.split);
-    c.blockDim = dim3(kBwdThreads);
-    c.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = p.split;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    c.attrs = at;
-    c.numAttrs = p.split > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&c, k_backward_tiled<FAN, FBP, SEG, VB, MODE>, p, img);
+    return launch_after_table(k_backward_tiled<FAN, FBP, SEG, VB, MODE>, dim3(tiles * p.split), kBwdThreads, p.split, s,
+                              p, img);
 }
 
 template <bool FAN, bool FBP, int SEG, int VB>
