@@ -28,7 +28,7 @@ struct BatchConfig {
     int fwd_views = 4;     // 2, 4, 8
     int fwd_occ = 1;       // 1 full residency, 2 half
     int fwd_order = 1;     // 1 largest slice first, 0 as given
-    int bwd_vb = 16;       // views in a tile's two staging buffers (16 only with 32-detector staging)
+    int bwd_vb = 8;        // views in a tile's two staging buffers (16 only with 32-detector staging)
     int bwd_occ = 1;
     int bwd_order = 1;
 };
