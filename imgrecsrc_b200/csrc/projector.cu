@@ -417,12 +417,12 @@ __device__ __forceinline__ void march_rows(const Geo &g, const FwdRay &ray, int 
     }
 }
 
-// rows [top, bottom] of part s of R, of the image's 2 half + 1
-__device__ __forceinline__ void part_rows(int half, int s, int R, int &top, int &bottom)
+// part s of R of the rows top, top - 1, ..., bottom (none if top < bottom)
+__device__ __forceinline__ void part_rows(int s, int R, int &top, int &bottom)
 {
-    const int M = 2 * half + 1;
-    top = half - (int)((long long)M * s / R);
-    bottom = half - (int)((long long)M * (s + 1) / R) + 1;
+    const int M = max(top - bottom + 1, 0), t = top;
+    top = t - (int)((long long)M * s / R);
+    bottom = t - (int)((long long)M * (s + 1) / R) + 1;
 }
 
 // Narrows [top, bottom] to the rows in which a ray of the warp can meet the
@@ -516,10 +516,11 @@ __device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int b
     if (R != kAllParts) wait_for_table();   // the quad image
     float S[8];
     unsigned long long nz = 0;
+    int rtop = g.half, rbottom = -g.half;
+    if (wcode != 5) clip_rows(ray, live, g.half, rtop, rbottom);
     auto rows_of = [&](int s) {
-        int top, bottom;
-        part_rows(g.half, s, p.rsplit, top, bottom);
-        if (wcode != 5) clip_rows(ray, live, g.half, top, bottom);
+        int top = rtop, bottom = rbottom;
+        part_rows(s, p.rsplit, top, bottom);
 #pragma unroll
         for (int j = 0; j < 8; ++j) S[j] = 0.0f;
         if (live && top >= bottom) march_rows<FAN, MODE>(g, ray, wcode, top, bottom, quad, S, nz);
@@ -626,13 +627,18 @@ k_forward(const FwdParams p, const float4 *__restrict__ quad, float *__restrict_
     }
 }
 
-// Parts a plan's image rows are summed in, one warp each.  The base rays alone
-// fill only part of the GPU below 1024^2 (276 warps at 256^2, where it holds
-// 2960), and up to three and a half waves of warps a split still evens out the
-// rays' uneven ways through the image.  Measured, 1 / 2 / 4 / 8 parts: 64^2 fan 28.7 / 20.5 /
-// 14.4 / 10.3 us, 256^2 parallel 84 / 51 / 31 / 21, 512^2 fan (1024 detectors)
-// 176 / 143 / 128 / 114, parallel 164 / 107 / 104 / 102, 1001^2 parallel 559 /
-// 553 / 531 / 600, 2048^2 fan 3538 / 3530 / 3561 / 3774; 16 parts gain nothing.
+// Parts a plan's image rows are summed in, one warp each: the rows between the
+// first and the last that its rays meet, so that a short chord's parts are as
+// even as a long one's (equal parts of the image's rows leave the outer ones
+// empty towards the detectors' ends; 512^2 fan 112 us, parallel 101, 1001^2
+// 523).  The base rays alone fill only part of the GPU below 1024^2 (276 warps
+// at 256^2, where it holds 2960), and up to three and a half waves of warps a
+// split still evens out the rays' uneven ways through the image.  Measured,
+// 1 / 2 / 4 / 8 parts: 64^2 fan 28.7 / 18.5 / 12.4 / 10.3 us, 256^2 parallel 84
+// / 49 / 29 / 21, 512^2 fan (1024 detectors) 178 / 144 / 118 / 101, parallel 165
+// / 107 / 85 / 86, 1001^2 parallel 590 / 522 / 476 / 497, 1024^2 fan (1536
+// views) 561 / 576 / 547 / 549, 2048^2 fan 3522 / 3442 / 3413 / 3546: the long
+// sums of 2048^2 stay in one part.
 static int forward_split(const ctprj_plan *pl)
 {
     int sms = 148;
