@@ -11,8 +11,19 @@
 // Partials are double buffered by the round's parity: a block can write round
 // r + 2 only after every block has read round r.
 //
-// A wait gives up after two seconds, or as soon as another block's has; the
-// caller then leaves its loop and the host reports the failure.
+// A meeting is a chain of latencies (the fence, the count, the partials), about
+// 4000 cycles, so it comes in steps between which a loop puts the work that does
+// not wait for the sums:
+//   sums_fold    the threads' sums to one per warp
+//   __syncthreads
+//   sums_post    the block's sums stored (warp 0)
+//   __syncthreads, when more than the partials is to be visible to the others
+//   sums_arrive  the block counted in
+//   sums_wait    every block's sums and earlier writes visible (read them past L1)
+//   sums_load    this thread's share of all blocks' sums
+//   sums_fold, __syncthreads, sums_of_block   the sums over all blocks
+// Rounds are 1, 2, ...  A wait gives up after two seconds, or as soon as another
+// block's has; the caller then leaves its loop and the host reports the failure.
 #pragma once
 
 namespace ctprj {
@@ -28,40 +39,72 @@ struct GridMeet {
 template <int K, int THREADS>
 struct GridSumsSmem {
     double red[K][THREADS / 32];
-    double sum[K];
     int ok;
 };
 
-// v: this thread's share of the K sums (K even) of round `round` = 1, 2, ...;
-// returns false when the meeting failed, else the sums over all blocks in v.
-// Every thread of the block takes part; what the block wrote to global memory
-// before is visible to the others after (read it past L1).
+// K = 2 or 4 sums per thread to one per warp: each halving of the lanes also
+// halves the sums a lane carries on (6 exchanges for four sums, not 20); sum k in
+// lanes k * 32 / K on
 template <int K, int THREADS>
-__device__ __forceinline__ bool grid_sums(const GridMeet &m, unsigned round, unsigned block, unsigned nblocks,
-                                          double (&v)[K], GridSumsSmem<K, THREADS> &S)
+__device__ __forceinline__ void sums_fold(const double (&v)[K], GridSumsSmem<K, THREADS> &S)
 {
-    const int t = threadIdx.x;
-    auto block_sums = [&]() {   // the warps' sums of v in S.red
+    static_assert(K == 2 || K == 4, "two or four sums");
+    const int lane = threadIdx.x & 31;
+    const bool hi = lane & 16;
+    double w;
+    if constexpr (K == 4) {
+        const double a = (hi ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 16);
+        const double b = (hi ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], 16);
+        const bool h8 = lane & 8;
+        w = (h8 ? b : a) + __shfl_xor_sync(0xffffffffu, h8 ? a : b, 8);
+    } else {
+        w = (hi ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[1], 16);
+        w += __shfl_xor_sync(0xffffffffu, w, 8);
+    }
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
+    for (int o = 4; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    if (lane % (32 / K) == 0) S.red[lane / (32 / K)][threadIdx.x >> 5] = w;
+}
+
+// the sum over the warps of what they left in S.red: sum k in lanes k * 32 / K on
+// (by all lanes of a warp)
+template <int K, int THREADS>
+__device__ __forceinline__ double sums_of_warps(const GridSumsSmem<K, THREADS> &S)
+{
+    constexpr int L = 32 / K;   // lanes per sum
+    const int lane = threadIdx.x & 31;
+    double w = 0.0;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-            if ((t & 31) == 0) S.red[k][t >> 5] = v[k];
-        }
-        __syncthreads();
-    };
-    block_sums();
-    double *part = m.part + (size_t)K * nblocks * (round & 1);
-    if (t == 0) {
+    for (int q = 0; q < THREADS / 32; q += L)
+        if (q + lane % L < THREADS / 32) w += S.red[lane / L][q + lane % L];
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            double w = 0.0;
-#pragma unroll
-            for (int q = 0; q < THREADS / 32; ++q) w += S.red[k][q];
-            __stcg(part + (size_t)K * block + k, w);
-        }
-        __threadfence();
-        atomicAdd(m.count, 1u);
+    for (int o = L / 2; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    return w;
+}
+
+template <int K, int THREADS>
+__device__ __forceinline__ void sums_post(const GridMeet &m, unsigned round, unsigned block, unsigned nblocks,
+                                          const GridSumsSmem<K, THREADS> &S)
+{
+    if (threadIdx.x >= 32) return;
+    const double w = sums_of_warps(S);
+    if (threadIdx.x % (32 / K) == 0)
+        __stcg(m.part + K * ((size_t)nblocks * (round & 1) + block) + threadIdx.x / (32 / K), w);
+    __syncwarp();
+}
+
+__device__ __forceinline__ void sums_arrive(const GridMeet &m)
+{
+    if (threadIdx.x == 0)
+        asm volatile("fence.acq_rel.gpu;\n\tred.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(m.count) : "memory");
+}
+
+// false when the meeting failed (the same in every thread of the block)
+template <int K, int THREADS>
+__device__ __forceinline__ bool sums_wait(const GridMeet &m, unsigned round, unsigned nblocks,
+                                          GridSumsSmem<K, THREADS> &S)
+{
+    if (threadIdx.x == 0) {
         const unsigned want = round * nblocks;
         unsigned long long t0 = 0, now;
         int ok = 1;
@@ -81,27 +124,32 @@ __device__ __forceinline__ bool grid_sums(const GridMeet &m, unsigned round, uns
         S.ok = ok;
     }
     __syncthreads();
-    if (!S.ok) return false;
+    return S.ok;
+}
+
+// this thread's share of every block's sums
+template <int K>
+__device__ __forceinline__ void sums_load(const GridMeet &m, unsigned round, unsigned nblocks, double (&v)[K])
+{
+    const double *part = m.part + (size_t)K * nblocks * (round & 1);
 #pragma unroll
     for (int k = 0; k < K; ++k) v[k] = 0.0;
-    for (unsigned b = t; b < nblocks; b += THREADS)
+    for (unsigned b = threadIdx.x; b < nblocks; b += blockDim.x)
 #pragma unroll
         for (int k = 0; k < K; k += 2) {
             const double2 u = __ldcg(reinterpret_cast<const double2 *>(part + (size_t)K * b + k));
             v[k] += u.x;
             v[k + 1] += u.y;
         }
-    block_sums();
-    if (t < K) {
-        double w = 0.0;
+}
+
+// the sums of the warps' folded ones, after a __syncthreads
+template <int K, int THREADS>
+__device__ __forceinline__ void sums_of_block(double (&v)[K], const GridSumsSmem<K, THREADS> &S)
+{
+    const double w = sums_of_warps(S);
 #pragma unroll
-        for (int q = 0; q < THREADS / 32; ++q) w += S.red[t][q];
-        S.sum[t] = w;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < K; ++k) v[k] = S.sum[k];
-    return true;
+    for (int k = 0; k < K; ++k) v[k] = __shfl_sync(0xffffffffu, w, k * (32 / K));
 }
 
 }  // namespace ctprj

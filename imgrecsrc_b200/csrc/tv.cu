@@ -92,13 +92,19 @@ __device__ __forceinline__ void block_sum4(double a[4], double *out)
 
 // The iteration's scalars from the summed partials: stopping count, restart,
 // t, momentum coefficient, done.
-__device__ void tv_advance(TvState *st, const double s[4], int max_iter, double eps)
+// t_{k+1}, and in c the step of R = P + (t_k - 1) / t_{k+1} (P - P_old)
+__device__ double tv_next_t(double tk, double &c)
+{
+    const double tkp1 = 0.5 * (1.0 + sqrt(1.0 + 4.0 * tk * tk));
+    c = (tk - 1.0) / tkp1;
+    return tkp1;
+}
+
+__device__ void tv_advance(TvState *st, const double s[4], int max_iter, double eps, double tkp1)
 {
     const double re = sqrt(s[0]) / sqrt(s[1]);   // NaN for D = 0: not a small change
     st->count = re < eps ? st->count + 1 : 0;
     const double fval = s[3] - s[2];
-    const double tk = st->tk, tkp1 = 0.5 * (1.0 + sqrt(1.0 + 4.0 * tk * tk));
-    st->c = (tk - 1.0) / tkp1;                 // R = P + (t_k - 1) / t_{k+1} (P - P_old)
     st->tk = fval > st->fold ? 1.0 : tkp1;     // restart when the dual objective rises
     st->fold = fval;
     st->iter += 1;
@@ -328,7 +334,8 @@ __global__ void __launch_bounds__(kTvThreads) k_tv_iter(const TvArgs a, int tile
     }
     if (t == 0) {
         const double tot[4] = {red[0][0], red[1][0], red[2][0], red[3][0]};
-        tv_advance(st, tot, a.max_iter, a.eps);
+        const double tkp1 = tv_next_t(st->tk, st->c);
+        tv_advance(st, tot, a.max_iter, a.eps, tkp1);
         st->arrived = 0;
     }
 }
@@ -352,28 +359,37 @@ __global__ void k_tv_start(TvState *st, int done)
 // P and writes the edge of its new P.  The blocks meet once per iteration, at the
 // sums of the stopping rule (grid_sums.cuh), after which every block advances its
 // own copy of the scalars: no host check, no second launch.  What bounds an
-// iteration is the chain of latencies (halo from L2, three phases in shared
-// memory, the meeting).
-constexpr int kTvpW = 64, kTvpH = 32, kTvpRows = 4;   // tile, thread rows
-constexpr int kTvpPer = kTvpH / kTvpRows;             // pixels per thread
+// iteration is a chain of latencies, of which the meeting (fence, count, partials
+// and halo from L2) is half; so a thread takes eight rows of one column, whose
+// neighbours above and below are mostly its own, reads shared memory four pixels
+// ahead of their use, posts its sums before the projection, works t out while
+// it waits, and begins the next iteration's R before it takes the sums.  Per
+// iteration, a launch each / this loop in the sums' order / as it stands: 512^2
+// 12.7 / 6.1 / 3.9 us, 768^2 - / 7.6 / 4.9, 1024^2 21 / 10.3 / 10.3.
+constexpr int kTvpW = 64, kTvpPer = 8;                // tile columns, pixels per thread
+constexpr int tvp_threads(int H) { return H * kTvpW / kTvpPer; }
 
+template <int H>
 struct TvpSmem {
-    float R1[kTvpH + 2][kTvpW + 1];   // rows i0-1 .. i0+H, columns j0 .. j0+W
-    float R2[kTvpH + 1][kTvpW + 2];   // rows i0 .. i0+H, columns j0-1 .. j0+W
-    float D[kTvpH + 1][kTvpW + 1];    // rows i0 .. i0+H, columns j0 .. j0+W
-    float X[kTvpH + 1][kTvpW + 1];
-    GridSumsSmem<4, kTvThreads> sums;
+    float R1[H + 2][kTvpW + 1];   // rows i0-1 .. i0+H, columns j0 .. j0+W
+    float R2[H + 1][kTvpW + 2];   // rows i0 .. i0+H, columns j0-1 .. j0+W
+    float D[H + 1][kTvpW + 1];    // rows i0 .. i0+H, columns j0 .. j0+W
+    float X[H + 1][kTvpW + 1];
+    GridSumsSmem<4, tvp_threads(H)> sums, taken;
 };
 
-__global__ void __launch_bounds__(kTvThreads, 4)
+template <bool ISO, int H, int PER_SM>
+__global__ void __launch_bounds__(tvp_threads(H), PER_SM)
 k_tv_loop(const TvArgs a, const GridMeet meet, float *__restrict__ out, int tiles_x)
 {
-    __shared__ TvpSmem S;
-    const int t = threadIdx.x, tx = t % kTvpW, ty = t / kTvpW;
-    const int i0 = (blockIdx.x / tiles_x) * kTvpH, j0 = (blockIdx.x % tiles_x) * kTvpW;
+    extern __shared__ __align__(16) unsigned char tv_smem[];
+    TvpSmem<H> &S = *reinterpret_cast<TvpSmem<H> *>(tv_smem);
+    constexpr int B = 4;   // pixels whose shared-memory reads are on their way together
+    const int t = threadIdx.x, tx = t % kTvpW, r0 = t / kTvpW * kTvpPer;   // the thread's pixels: (r0 + k, tx)
+    const int i0 = (blockIdx.x / tiles_x) * H, j0 = (blockIdx.x % tiles_x) * kTvpW;
     const int m = a.m, n = a.n, j = j0 + tx;
     const float lam = a.lam, lb = a.lb, ub = a.ub, inv8l = 1.0f / (8.0f * lam);
-    for (int e = t; e < (kTvpH + 1) * (kTvpW + 1); e += kTvThreads) {
+    for (int e = t; e < (H + 1) * (kTvpW + 1); e += tvp_threads(H)) {
         const int r = e / (kTvpW + 1), c = e % (kTvpW + 1);
         S.X[r][c] = i0 + r < m && j0 + c < n ? a.xobs[(size_t)(i0 + r) * n + j0 + c] : 0.0f;
         S.D[r][c] = 0.0f;
@@ -389,21 +405,21 @@ k_tv_loop(const TvArgs a, const GridMeet meet, float *__restrict__ out, int tile
         hr = -1;
         hc = t;
     } else if (t <= 2 * kTvpW) {
-        hr = kTvpH;
+        hr = H;
         hc = t - kTvpW - 1;
-    } else if (t <= 2 * kTvpW + 1 + kTvpH) {
+    } else if (t <= 2 * kTvpW + 1 + H) {
         hr = t - 2 * kTvpW - 1;
         hc = -1;
-    } else if (t <= 2 * kTvpW + 1 + 2 * kTvpH) {
-        hr = t - 2 * kTvpW - 2 - kTvpH;
+    } else if (t <= 2 * kTvpW + 1 + 2 * H) {
+        hr = t - 2 * kTvpW - 2 - H;
         hc = kTvpW;
     } else {
         halo = false;
     }
     const int hi = i0 + hr, hj = j0 + hc;
     const bool inside = halo && hi >= 0 && hi < m && hj >= 0 && hj < n;
-    const size_t hq = inside ? (size_t)hi * n + hj : 0;
-    float2 hp = make_float2(0.0f, 0.0f);   // the halo cell's P of the last iteration
+    const size_t hx = inside ? (size_t)hi * n + hj : 0;
+    float2 hp = make_float2(0.0f, 0.0f), hq = hp;   // the halo cell's P and P of the iteration before
     TvState st;
     st.tk = 1.0;
     st.c = 0.0;
@@ -412,83 +428,117 @@ k_tv_loop(const TvArgs a, const GridMeet meet, float *__restrict__ out, int tile
     st.done = a.max_iter <= 0;
     bool ok = true;
     __syncthreads();
-    while (!st.done) {
+    double s[4], tkp1 = 1.0;
+    for (unsigned round = 1; !st.done; ++round) {
+        // c, which the sums of the last iteration do not decide (a restart tells
+        // one iteration later), starts this one before they are taken
         const float c = (float)st.c;
+        if (round > 1) sums_load(meet, round - 1, gridDim.x, s);
+#pragma unroll
+        for (int k = 0; k < kTvpPer; ++k) {   // Q: R until P is renewed
+            Q[k].x = fmaf(c, P[k].x - Q[k].x, P[k].x);
+            Q[k].y = fmaf(c, P[k].y - Q[k].y, P[k].y);
+            S.R2[r0 + k][tx + 1] = Q[k].y;
+        }
+        S.R1[r0 + kTvpPer][tx] = Q[kTvpPer - 1].x;
         if (halo) {   // R on the halo
-            float2 p = hp;
-            if (inside && st.iter > 0) p = __ldcg(tv_p(a.buf, a.px, st.iter & 1) + hq);
-            const float2 q = hp;
-            hp = p;
-            const float r1 = fmaf(c, p.x - q.x, p.x), r2 = fmaf(c, p.y - q.y, p.y);
+            const float r1 = fmaf(c, hp.x - hq.x, hp.x), r2 = fmaf(c, hp.y - hq.y, hp.y);
             if (hc >= 0) S.R1[hr + 1][hc] = r1;
             if (hr >= 0) S.R2[hr][hc + 1] = r2;
         }
-#pragma unroll
-        for (int k = 0; k < kTvpPer; ++k) {
-            const int r = ty + kTvpRows * k;
-            S.R1[r + 1][tx] = fmaf(c, P[k].x - Q[k].x, P[k].x);
-            S.R2[r][tx + 1] = fmaf(c, P[k].y - Q[k].y, P[k].y);
-        }
+        if (round > 1) sums_fold(s, S.taken);
         __syncthreads();
+        if (round > 1) {
+            sums_of_block(s, S.taken);
+            tv_advance(&st, s, a.max_iter, a.eps, tkp1);
+            if (st.done) break;
+        }
         // C = Xobs - lambda L(R), D = clamp(C) on the tile (partials) and its halo
-        double s[4] = {0.0, 0.0, 0.0, 0.0};
+        s[0] = s[1] = s[2] = s[3] = 0.0;
+        float up = S.R1[r0][tx];
 #pragma unroll
-        for (int k = 0; k < kTvpPer; ++k) {
-            const int r = ty + kTvpRows * k;
-            if (i0 + r < m && j < n) {
-                const float L = (S.R1[r + 1][tx] - S.R1[r][tx]) + (S.R2[r][tx + 1] - S.R2[r][tx]);
-                const float C = fmaf(-lam, L, S.X[r][tx]);
-                const float Dv = fminf(fmaxf(C, lb), ub);
-                const double dd = (double)Dv - (double)S.D[r][tx], cd = (double)C - (double)Dv;
-                S.D[r][tx] = Dv;
+        for (int k0 = 0; k0 < kTvpPer; k0 += B) {
+            float left[B], X[B], D[B];
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                left[k] = S.R2[r0 + k0 + k][tx];
+                X[k] = S.X[r0 + k0 + k][tx];
+                D[k] = S.D[r0 + k0 + k][tx];
+            }
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const float2 R = Q[k0 + k];
+                const bool in = i0 + r0 + k0 + k < m && j < n;
+                const float C = in ? fmaf(-lam, (R.x - up) + (R.y - left[k]), X[k]) : 0.0f;
+                up = R.x;
+                const float Dv = in ? fminf(fmaxf(C, lb), ub) : 0.0f;
+                S.D[r0 + k0 + k][tx] = Dv;
+                const double dv = (double)Dv, dc = (double)C, dd = dv - (double)D[k], cd = dc - dv;
                 s[0] = fma(dd, dd, s[0]);
-                s[1] = fma((double)Dv, (double)Dv, s[1]);
+                s[1] = fma(dv, dv, s[1]);
                 s[2] = fma(cd, cd, s[2]);
-                s[3] = fma((double)C, (double)C, s[3]);
+                s[3] = fma(dc, dc, s[3]);
             }
         }
-        if (t < kTvpW + kTvpH) {   // the bottom row and the right column
-            const int r = t < kTvpW ? kTvpH : t - kTvpW, cc = t < kTvpW ? t : kTvpW;
+        if (t < kTvpW + H) {   // the bottom row and the right column
+            const int r = t < kTvpW ? H : t - kTvpW, cc = t < kTvpW ? t : kTvpW;
             if (i0 + r < m && j0 + cc < n) {
                 const float L = (S.R1[r + 1][cc] - S.R1[r][cc]) + (S.R2[r][cc + 1] - S.R2[r][cc]);
                 S.D[r][cc] = fminf(fmaxf(fmaf(-lam, L, S.X[r][cc]), lb), ub);
             }
         }
+        sums_fold(s, S.sums);
         __syncthreads();
+        sums_post(meet, round, blockIdx.x, gridDim.x, S.sums);
         // P_new = proj(R + Ltrans(D) / (8 lambda)) on the tile
-        float2 *N = tv_p(a.buf, a.px, (st.iter + 1) & 1);
+        float2 *N = tv_p(a.buf, a.px, round & 1);
+        float d = S.D[r0][tx];
 #pragma unroll
-        for (int k = 0; k < kTvpPer; ++k) {
-            const int r = ty + kTvpRows * k, i = i0 + r;
-            Q[k] = P[k];
-            if (i < m && j < n) {
-                const float d = S.D[r][tx];
-                float p1 = i < m - 1 ? fmaf(d - S.D[r + 1][tx], inv8l, S.R1[r + 1][tx]) : 0.0f;
-                float p2 = j < n - 1 ? fmaf(d - S.D[r][tx + 1], inv8l, S.R2[r][tx + 1]) : 0.0f;
-                if (a.iso) {   // P / max(1, |P|): scaled only outside the unit ball
-                    const float q2 = fmaf(p1, p1, p2 * p2);
-                    if (q2 > 1.0f) {
-                        const float rs = rsqrtf(q2);
-                        p1 *= rs;
-                        p2 *= rs;
-                    }
+        for (int k0 = 0; k0 < kTvpPer; k0 += B) {
+            float right[B], down[B];
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                right[k] = S.D[r0 + k0 + k][tx + 1];
+                down[k] = S.D[r0 + k0 + k + 1][tx];
+            }
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const int i = i0 + r0 + k0 + k;
+                const float2 R = Q[k0 + k];
+                float p1 = i < m - 1 && j < n ? fmaf(d - down[k], inv8l, R.x) : 0.0f;
+                float p2 = i < m && j < n - 1 ? fmaf(d - right[k], inv8l, R.y) : 0.0f;
+                d = down[k];
+                if (ISO) {   // P / max(1, |P|): scaled only outside the unit ball
+                    const float q2 = fmaf(p1, p1, p2 * p2), rs = rsqrtf(fmaxf(q2, 1.0f));
+                    p1 = q2 > 1.0f ? p1 * rs : p1;
+                    p2 = q2 > 1.0f ? p2 * rs : p2;
                 } else {
                     p1 = fminf(fmaxf(p1, -1.0f), 1.0f);
                     p2 = fminf(fmaxf(p2, -1.0f), 1.0f);
                 }
-                P[k] = make_float2(p1, p2);
-                // only the tile's edge is another block's halo
-                if (r == 0 || r == kTvpH - 1 || tx == 0 || tx == kTvpW - 1) __stcg(N + (size_t)i * n + j, P[k]);
+                Q[k0 + k] = P[k0 + k];
+                P[k0 + k] = make_float2(p1, p2);
             }
         }
-        ok = grid_sums(meet, st.iter + 1, blockIdx.x, gridDim.x, s, S.sums);
-        if (!ok) break;
-        tv_advance(&st, s, a.max_iter, a.eps);
+        // only the tile's edge is another block's halo
+        const bool side = tx == 0 || tx == kTvpW - 1;
+#pragma unroll
+        for (int k = 0; k < kTvpPer; ++k) {
+            const int r = r0 + k, i = i0 + r;
+            if (i < m && j < n && (side || (k == 0 && r == 0) || (k == kTvpPer - 1 && r == H - 1)))
+                __stcg(N + (size_t)i * n + j, P[k]);
+        }
+        __syncthreads();
+        sums_arrive(meet);
+        tkp1 = tv_next_t(st.tk, st.c);
+        if (!(ok = sums_wait(meet, round, gridDim.x, S.sums))) break;
+        hq = hp;
+        if (inside) hp = __ldcg(N + hx);
     }
     if (!ok) return;
 #pragma unroll
     for (int k = 0; k < kTvpPer; ++k) {
-        const int r = ty + kTvpRows * k, i = i0 + r;
+        const int r = r0 + k, i = i0 + r;
         if (i < m && j < n) out[(size_t)i * n + j] = S.D[r][tx];
     }
     if (blockIdx.x == 0 && t == 0) {
@@ -521,9 +571,9 @@ __global__ void k_tv_sum(const double *__restrict__ part, int nblocks, double *_
     sum_partials(part, nblocks, 1, 1, out);
 }
 
-static int tv_loop_tiles(int m, int n)
+static int tv_loop_tiles(int m, int n, int H = 32)
 {
-    return ((n + kTvpW - 1) / kTvpW) * ((m + kTvpH - 1) / kTvpH);
+    return ((n + kTvpW - 1) / kTvpW) * ((m + H - 1) / H);
 }
 
 // the state, and the one-launch loop's failure word and count
@@ -562,6 +612,31 @@ void TvWorkspace::release(cudaStream_t s)
     rows = cols = 0;
 }
 
+// The loop's variant for an image.  Up to two 32-row tiles per SM a thread may
+// take 128 registers; beyond, two blocks per SM of twice the rows meet a little
+// sooner than four (1024^2: 10.3 us per iteration against 11.2, 1056^2 10.6
+// against 12.0), and those four are left for the sizes whose 64-row tiles would
+// not all fit.
+struct TvLoop {
+    const void *kernel;
+    int tiles, threads;
+    size_t smem;
+};
+
+template <int H, int PER_SM>
+static TvLoop tv_loop_variant(int m, int n, int iso)
+{
+    const void *kernel = iso ? (const void *)k_tv_loop<true, H, PER_SM> : (const void *)k_tv_loop<false, H, PER_SM>;
+    return {kernel, tv_loop_tiles(m, n, H), tvp_threads(H), sizeof(TvpSmem<H>)};
+}
+
+static TvLoop tv_loop_of(int m, int n, int iso, int sms)
+{
+    if (tv_loop_tiles(m, n, 32) <= 2 * sms) return tv_loop_variant<32, 2>(m, n, iso);
+    if (tv_loop_tiles(m, n, 64) <= 2 * sms) return tv_loop_variant<64, 2>(m, n, iso);
+    return tv_loop_variant<32, 4>(m, n, iso);
+}
+
 int tv_denoise(TvWorkspace &ws, const float *xobs, int m, int n, double lambda, double lb, double ub,
                int iso, int max_iter, double eps, float *out, int *iterations, cudaStream_t s)
 {
@@ -586,13 +661,13 @@ int tv_denoise(TvWorkspace &ws, const float *xobs, int m, int n, double lambda, 
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // every tile a block of its own on the GPU at once: the loop in one launch
-    // (12.7 -> 6.1 us per iteration at 512^2, 21 -> 10 at 1024^2, where launches
-    // and the loads' latency took most of it; a round's chain of latencies, 5 us,
-    // is what is left).  Larger images stream through the persistent blocks below.
-    if ((st = cuda_error(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tv_loop, kTvThreads, 0),
+    const TvLoop loop = tv_loop_of(m, n, iso, sms);
+    if ((st = cuda_error(cudaFuncSetAttribute(loop.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)loop.smem),
+                         "TV shared memory")) ||
+        (st = cuda_error(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, loop.kernel, loop.threads, loop.smem),
                          "TV occupancy")))
         return st;
-    if (tv_loop_tiles(m, n) <= sms * per_sm) {
+    if (loop.tiles <= sms * per_sm) {
         struct {
             TvState st;
             int failed;
@@ -600,11 +675,11 @@ int tv_denoise(TvWorkspace &ws, const float *xobs, int m, int n, double lambda, 
         // after the state: the failure word and the count of the meetings
         int *failed = (int *)(a.st + 1);
         GridMeet meet = {(unsigned *)(failed + 1), failed, ws.part};
-        const int ntiles = tv_loop_tiles(m, n);
         int tx = (n + kTvpW - 1) / kTvpW;
         void *args[] = {&a, &meet, &out, &tx};
         if ((st = cuda_error(cudaMemsetAsync(a.st, 0, kTvStateBytes, s), "TV start")) ||
-            (st = cuda_error(cudaLaunchCooperativeKernel((void *)k_tv_loop, dim3(ntiles), dim3(kTvThreads), args, 0, s),
+            (st = cuda_error(cudaLaunchCooperativeKernel(loop.kernel, dim3(loop.tiles), dim3(loop.threads), args,
+                                                         loop.smem, s),
                              "TV loop")) ||
             (st = cuda_error(cudaMemcpyAsync(&h, a.st, sizeof h, cudaMemcpyDeviceToHost, s), "TV state")) ||
             (st = cuda_error(cudaStreamSynchronize(s), "TV state")))

@@ -752,8 +752,15 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
                 nu[e] = s[e] = 0.0f;
             }
         }
-        ok = grid_sums(p.meet, st.iter + 1, block, nblocks, ps, sums);
-        if (!ok) break;
+        sums_fold(ps, sums);
+        __syncthreads();
+        sums_post(p.meet, st.iter + 1, block, nblocks, sums);
+        sums_arrive(p.meet);
+        if (!(ok = sums_wait(p.meet, st.iter + 1, nblocks, sums))) break;
+        sums_load(p.meet, st.iter + 1, nblocks, ps);
+        sums_fold(ps, sums);
+        __syncthreads();
+        sums_of_block(ps, sums);
         admm_advance(&st, ps[0], ps[1]);
     }
     if (!ok) return;
