@@ -527,12 +527,17 @@ __global__ void __launch_bounds__(kHaarThreads) k_admm_haar(const HaarArgs a)
 // touch, so where every tile has a block of its own on the GPU (k_admm_loop's
 // callers check) s, nu and a never leave the block: a thread keeps a 4 x 4
 // pixel block -- its fifteen coefficients of levels 1 and 2 and one cell of the
-// tile's 16 x 16 coarse array -- in registers, does levels 1 and 2 there, and
-// one warp does the coarser levels on the 16 x 16 array in shared memory.  Per
-// iteration the blocks exchange nothing but the two sums of the stopping rule
-// (grid_sums.cuh), after which every block advances its own copy of the
-// scalars.  The arithmetic is the level kernels' operation for
-// operation; what bounds an iteration is the chain of latencies.
+// tile's 16 x 16 coarse array -- in registers.  Levels 3 and 4 join 2 x 2 lanes of
+// half a warp; the sixteen cells of level 4 go through shared memory, and levels 5
+// and 6 are worked out by every half warp alike, so that the way back needs no
+// exchange between warps.  Per iteration the blocks exchange nothing but the two
+// sums of the stopping rule (grid_sums.cuh), after which every block advances its
+// own copy of the scalars.  The arithmetic is the level kernels' operation for
+// operation.  What bounds an iteration is the chain of latencies: the meeting is
+// half of it, and of the rest the soft threshold's branches (they are selects now)
+// and the coarse levels by one warp in shared memory took most.  Per iteration, a
+// launch each / this loop with those / as it stands: 64^2 - / 5.5 / 4.0 us, 512^2
+// - / 5.8 / 4.1, 1024^2 23 / 7.0 / 5.6.
 constexpr int kLoopTile = 64, kLoopSide = kLoopTile / 4;   // tile, 4 x 4 blocks along its side
 constexpr int kLoopThreads = kLoopSide * kLoopSide;
 
@@ -586,81 +591,52 @@ __device__ __forceinline__ void haar_join(const HaarArgs &a, float ll, float lh,
     x11 = fmaf(a.h1, ulo, fmaf(a.g1, uhi, 0.0f));
 }
 
-// levels 3 .. levels of the tile's 16 x 16 array, in place, by one warp
-__device__ __forceinline__ void coarse_split(const HaarArgs &a, float (*W)[kLoopSide + 1], int levels)
+// One level of the transform over lanes: lanes 2 x 2 by lane bits dx and dy (this
+// one in column `col` and row `row` of the four) give their values and take one of
+// the cell's results each, operation for operation haar_split's and haar_join's.
+__device__ __forceinline__ float lane_split(const HaarArgs &a, float x, int dx, int dy, bool col, bool row)
 {
-    const int lane = threadIdx.x & 31;
-    for (int l = 3; l <= levels; ++l) {
-        const int g = 6 - l, T = 1 << g;
-        float v[2][4];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int q = lane + 32 * u, k = q >> g, c = q & (T - 1);
-            if (q < T * T)
-                haar_split(a, W[2 * k][2 * c], W[2 * k][2 * c + 1], W[2 * k + 1][2 * c], W[2 * k + 1][2 * c + 1], v[u][0],
-                           v[u][1], v[u][2], v[u][3]);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int q = lane + 32 * u, k = q >> g, c = q & (T - 1);
-            if (q < T * T) {
-                W[k][c] = v[u][0];
-                W[k][c + T] = v[u][1];
-                W[k + T][c] = v[u][2];
-                W[k + T][c + T] = v[u][3];
-            }
-        }
-        __syncwarp();
-    }
+    float o = __shfl_xor_sync(0xffffffffu, x, dx);
+    x = fmaf(col ? a.g1 : a.h1, col ? x : o, fmaf(col ? a.g0 : a.h0, col ? o : x, 0.0f));
+    o = __shfl_xor_sync(0xffffffffu, x, dy);
+    return fmaf(row ? a.g1 : a.h1, row ? x : o, fmaf(row ? a.g0 : a.h0, row ? o : x, 0.0f));
 }
-__device__ __forceinline__ void coarse_join(const HaarArgs &a, float (*W)[kLoopSide + 1], int levels)
+__device__ __forceinline__ float lane_join(const HaarArgs &a, float x, int dx, int dy, bool col, bool row)
 {
-    const int lane = threadIdx.x & 31;
-    for (int l = levels; l >= 3; --l) {
-        const int g = 6 - l, T = 1 << g;
-        float x[2][4];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int q = lane + 32 * u, k = q >> g, c = q & (T - 1);
-            if (q < T * T)
-                haar_join(a, W[k][c], W[k][c + T], W[k + T][c], W[k + T][c + T], x[u][0], x[u][1], x[u][2], x[u][3]);
-        }
-        __syncwarp();
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int q = lane + 32 * u, k = q >> g, c = q & (T - 1);
-            if (q < T * T) {
-                W[2 * k][2 * c] = x[u][0];
-                W[2 * k][2 * c + 1] = x[u][1];
-                W[2 * k + 1][2 * c] = x[u][2];
-                W[2 * k + 1][2 * c + 1] = x[u][3];
-            }
-        }
-        __syncwarp();
-    }
+    float o = __shfl_xor_sync(0xffffffffu, x, dy);
+    x = fmaf(row ? a.h1 : a.h0, row ? o : x, fmaf(row ? a.g1 : a.g0, row ? x : o, 0.0f));
+    o = __shfl_xor_sync(0xffffffffu, x, dx);
+    return fmaf(col ? a.h1 : a.h0, col ? o : x, fmaf(col ? a.g1 : a.g0, col ? x : o, 0.0f));
 }
 
 __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArgs p)
 {
     const HaarArgs &a = p.h;
-    __shared__ float W[kLoopSide][kLoopSide + 1];
     __shared__ float A[16][kLoopThreads];     // a at this thread's pixels
+    __shared__ float cells[16];               // the tile's cells of level 4
     __shared__ GridSumsSmem<2, kLoopThreads> sums;
-    const int t = threadIdx.x, by = t / kLoopSide, bx = t % kLoopSide, ti = blockIdx.y, tj = blockIdx.x;
+    // half a warp has the 4 x 4 coarse cells of one cell of level 4, l this
+    // thread's among them
+    const int t = threadIdx.x, ti = blockIdx.y, tj = blockIdx.x;
+    const int l = t & 15, cell4 = t >> 4, by = (cell4 & ~3) + (l >> 2), bx = 4 * (cell4 & 3) + (l & 3);
+    const bool up4 = (l & 5) == 0;   // a cell of level 3 is this lane's to pass on
     const unsigned nblocks = gridDim.x * gridDim.y, block = blockIdx.y * gridDim.x + blockIdx.x;
     const size_t pix = (size_t)(ti * kLoopTile + 4 * by) * a.cols + tj * kLoopTile + 4 * bx;
     const double ss = *p.ss;
     const int levels = p.levels;
-    // coefficients of this thread: 0 its coarse cell; 1..3 (LH, HL, HH) of level
-    // 2; 4 + 3 q .. of level 1, q its 2 x 2 cell
-    unsigned pm = 0xffffu, cm = 0xffffu;
+    // coefficients of this thread: 0 what levels 3 and 4 left in its lane; 1..3
+    // (LH, HL, HH) of level 2; 4 + 3 q .. of level 1, q its 2 x 2 cell; and one of
+    // levels 5 and 6 ("top"), which every half warp works out for itself
+    const int p3 = (l >> 1 & 2) | (l & 1), p4 = (l >> 2 & 2) | (l >> 1 & 1);
+    const bool tops = levels >= 5;
+    unsigned pm = 0xffffu, cm = tops && l == 0 ? 0xfffeu : 0xffffu;
+    bool topm = tops;
     if (a.pmask) {
         pm = 0;
         for (int e = 0; e < 16; ++e) pm |= (unsigned)(a.pmask[pix + (size_t)(e >> 2) * a.cols + (e & 3)] != 0) << e;
     }
     if (a.cmask) {
-        cm = 0;
+        auto coef = [&](int r, int c) { return a.cmask[loop_coef_index(r, c, ti, tj, levels, a.rows, a.cols)] != 0; };
         for (int e = 0; e < 16; ++e) {
             int r = by, c = bx;
             if (e >= 4) {
@@ -670,20 +646,41 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
             } else if (e > 0) {
                 r += (e >> 1) * 16;
                 c += (e & 1) * 16;
+            } else if (levels >= 4 && up4) {
+                r = (by >> 2) + (p4 >> 1) * 4;
+                c = (bx >> 2) + (p4 & 1) * 4;
+            } else if (levels >= 3) {
+                r = (by >> 1) + (p3 >> 1) * 8;
+                c = (bx >> 1) + (p3 & 1) * 8;
             }
-            cm |= (unsigned)(a.cmask[loop_coef_index(r, c, ti, tj, levels, a.rows, a.cols)] != 0) << e;
+            if (!coef(r, c)) cm &= ~(1u << e);
         }
+        if (tops)
+            topm = levels >= 6 && up4 ? coef(p4 >> 1, p4 & 1) : coef((l >> 3) + (p3 & 2), (l >> 1 & 1) + 2 * (p3 & 1));
     }
-    float s[16], nu[16], x[16];
-    // levels 1 and 2 of x into v, the coarse cells into W
-    auto split = [&](float (&v)[16]) {
+    float s[16], nu[16], x[16], stop = 0.0f, nutop = 0.0f;
+    // the transform of x into v and top
+    auto split = [&](float (&v)[16], float &top) {
         float l1[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int e = (q >> 1) * 8 + (q & 1) * 2;
             haar_split(a, x[e], x[e + 1], x[e + 4], x[e + 5], l1[q], v[4 + 3 * q], v[5 + 3 * q], v[6 + 3 * q]);
         }
-        haar_split(a, l1[0], l1[1], l1[2], l1[3], W[by][bx], v[1], v[2], v[3]);
+        haar_split(a, l1[0], l1[1], l1[2], l1[3], v[0], v[1], v[2], v[3]);
+        if (levels >= 3) v[0] = lane_split(a, v[0], 1, 4, l & 1, l & 4);
+        if (levels >= 4) {
+            const float u = lane_split(a, v[0], 2, 8, l & 2, l & 8);
+            if (up4) v[0] = u;
+        }
+        if (!tops) return;
+        if (l == 0) cells[cell4] = v[0];
+        __syncthreads();
+        top = lane_split(a, cells[l], 1, 4, l & 1, l & 4);
+        if (levels >= 6) {
+            const float u = lane_split(a, top, 2, 8, l & 2, l & 8);
+            if (up4) top = u;
+        }
     };
 #pragma unroll
     for (int e = 0; e < 16; ++e) {
@@ -692,14 +689,12 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
         x[e] = p.init[q];
         nu[e] = 0.0f;
     }
-    split(s);
-    __syncthreads();
-    if (t < 32) coarse_split(a, W, levels);
-    __syncthreads();
-    s[0] = W[by][bx];
+    split(s, stop);
+    __syncthreads();   // cells are read
 #pragma unroll
     for (int e = 0; e < 16; ++e)
         if (!((cm >> e) & 1)) s[e] = 0.0f;
+    if (!topm) stop = 0.0f;
     AdmmState st;
     st.rho = st.nu_mul = 1.0;
     st.tol = fmin(1e-3, p.rel_tol) * sqrt(ss);
@@ -711,13 +706,23 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
     for (;;) {
         const float mul = (float)st.nu_mul, rho = (float)st.rho, thr = (float)(a.u / st.rho);
         // x = Psi(s + nu), then alpha = max((a + rho x) / (1 + rho), 0)
-        __syncthreads();
-        W[by][bx] = fmaf(mul, nu[0], s[0]);
-        __syncthreads();
-        if (t < 32) coarse_join(a, W, levels);
-        __syncthreads();
+        float w0 = fmaf(mul, nu[0], s[0]);
+        if (tops) {
+            float top = fmaf(mul, nutop, stop);
+            if (levels >= 6) {
+                const float u = lane_join(a, top, 2, 8, l & 2, l & 8);
+                if (up4) top = u;
+            }
+            top = __shfl_sync(0xffffffffu, lane_join(a, top, 1, 4, l & 1, l & 4), cell4);
+            if (l == 0) w0 = top;
+        }
+        if (levels >= 4) {
+            const float u = lane_join(a, w0, 2, 8, l & 2, l & 8);
+            if (up4) w0 = u;
+        }
+        if (levels >= 3) w0 = lane_join(a, w0, 1, 4, l & 1, l & 4);
         float l1[4];
-        haar_join(a, W[by][bx], fmaf(mul, nu[1], s[1]), fmaf(mul, nu[2], s[2]), fmaf(mul, nu[3], s[3]), l1[0], l1[1],
+        haar_join(a, w0, fmaf(mul, nu[1], s[1]), fmaf(mul, nu[2], s[2]), fmaf(mul, nu[3], s[3]), l1[0], l1[1],
                   l1[2], l1[3]);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -725,33 +730,65 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
             haar_join(a, l1[q], fmaf(mul, nu[4 + 3 * q], s[4 + 3 * q]), fmaf(mul, nu[5 + 3 * q], s[5 + 3 * q]),
                       fmaf(mul, nu[6 + 3 * q], s[6 + 3 * q]), x[e], x[e + 1], x[e + 4], x[e + 5]);
         }
-#pragma unroll
-        for (int e = 0; e < 16; ++e)
-            x[e] = (pm >> e) & 1 ? fmaxf(fmaf(rho, x[e], A[e][t]) / (1.0f + rho), 0.0f) : 0.0f;
-        if (st.done) break;
-        float v[16];
-        split(v);   // (W is read by its own thread only since the join)
-        __syncthreads();
-        if (t < 32) coarse_split(a, W, levels);
-        __syncthreads();
-        v[0] = W[by][bx];
-        // s = soft(v - nu, u / rho), nu = nu + s - v
-        double ps[2] = {0.0, 0.0};
+        // The quotients by 1 + rho through its FP64 reciprocal: a quotient of two
+        // 24-bit numbers is no nearer than 2^-49 of itself to a number halfway
+        // between two of FP32 (the numerator less that times the divisor is a
+        // whole multiple of their last places), the product 2^-52 off at most, so
+        // it rounds to the quotient's FP32 (sixteen divisions took 2600 cycles).
+        const double inv = 1.0 / (double)(1.0f + rho);
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-            const float nue = mul * nu[e];
-            const float w = v[e] - nue;
-            const float sn = w > thr ? w - thr : (w < -thr ? w + thr : 0.0f);
-            if ((cm >> e) & 1) {
-                nu[e] = nue + sn - v[e];
-                const double d = (double)sn - (double)s[e], r = (double)sn - (double)v[e];
-                s[e] = sn;
-                ps[0] = fma(d, d, ps[0]);
-                ps[1] = fma(r, r, ps[1]);
-            } else {   // not a coefficient of the masked transform
-                nu[e] = s[e] = 0.0f;
+            const float q = (float)((double)fmaf(rho, x[e], A[e][t]) * inv);
+            x[e] = (pm >> e) & 1 ? fmaxf(q, 0.0f) : 0.0f;
+        }
+        if (st.done) break;
+        float v[16], vtop = 0.0f;
+        split(v, vtop);
+        // s = soft(v - nu, u / rho), nu = nu + s - v; zero where the masked
+        // transform has no coefficient
+        double ps[2] = {0.0, 0.0}, pt[2] = {0.0, 0.0};
+        auto shrink = [&](float &nue, float &ve, bool coef) {
+            const float m = mul * nue, w = ve - m;
+            const float above = w - thr, below = w + thr;
+            float sn = w > thr ? above : 0.0f;
+            sn = w < -thr ? below : sn;
+            sn = coef ? sn : 0.0f;
+            ve = coef ? ve : 0.0f;
+            nue = coef ? m + sn - ve : 0.0f;
+            return sn;
+        };
+#pragma unroll
+        for (int e0 = 0; e0 < 16; e0 += 4) {   // four chains of FP64 latencies side by side
+            float sn[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) sn[q] = shrink(nu[e0 + q], v[e0 + q], (cm >> (e0 + q)) & 1);
+            double d[4], r[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const double ds = (double)sn[q];
+                d[q] = ds - (double)s[e0 + q];
+                r[q] = ds - (double)v[e0 + q];
+                s[e0 + q] = sn[q];
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q += 2) {
+                ps[0] = fma(d[q], d[q], ps[0]);
+                ps[1] = fma(r[q], r[q], ps[1]);
+                pt[0] = fma(d[q + 1], d[q + 1], pt[0]);
+                pt[1] = fma(r[q + 1], r[q + 1], pt[1]);
             }
         }
+        if (tops) {
+            const float sn = shrink(nutop, vtop, topm);
+            if (t < 16) {
+                const double ds = (double)sn, d = ds - (double)stop, r = ds - (double)vtop;
+                ps[0] = fma(d, d, ps[0]);
+                ps[1] = fma(r, r, ps[1]);
+            }
+            stop = sn;
+        }
+        ps[0] += pt[0];
+        ps[1] += pt[1];
         sums_fold(ps, sums);
         __syncthreads();
         sums_post(p.meet, st.iter + 1, block, nblocks, sums);
@@ -1028,8 +1065,8 @@ int wvlt_admm(WvltProx &ws, const float *a, int rows, int cols, const double *h,
     ha.cmask = cmask;
     AdmmState h_st{};
     // whole 64 x 64 tiles, each with a block of its own on the GPU at once: the
-    // loop in one launch (23 -> 7.2 us per iteration at 1024^2: s, nu and a no
-    // longer pass through L2, and 12 block-wide barriers became 7).  Other sizes
+    // loop in one launch (23 -> 5.6 us per iteration at 1024^2: s, nu and a no
+    // longer pass through L2, and 12 block-wide barriers became 4).  Other sizes
     // take a launch per iteration, in tiles of 2^levels.
     if (fused && levels >= 2 && rows % kLoopTile == 0 && cols % kLoopTile == 0) {
         int dev = 0, sms = 148, per_sm = 0;
