@@ -72,7 +72,8 @@ static ParView par_view(double theta, double bw)
     v.ramp = 0.5 * v.height / (v.b2 - v.b1);
     // (negative angles get footprints with b2 < b1 from the truncated angle:
     // those keep the reference's piecewise formula)
-    v.edges = bw == 1.0 && v.b2 > v.b1 && v.b2 >= 0.5;
+    // (the pixels of a line are at least b2 <= sqrt(1/2) apart, as edge_lines counts on)
+    v.edges = bw == 1.0 && v.b2 > v.b1 && v.b2 >= 0.5 && fmax(fabs(v.c), fabs(v.s)) >= v.b2 - 1e-12;
     v.box = v.edges && v.b2 - v.b1 < 1e-6;
     return v;
 }
@@ -208,16 +209,20 @@ __device__ __noinline__ double par_gather(const ParArgs &a, const ParView &v, do
 // One warp of the forward: 32 detector edges kk0 - 1/2 + lane of angle v over
 // the lines [l0, l1) of the image (rows where the band is closer to the columns,
 // else columns), 31 detectors.  Per line, with q the pixel index along it in the
-// direction of growing distance, lane e's edge has the pixels q0 .. q0 + 2 whose
-// footprints it cuts (2 b2 / max(|c|, |s|) <= 2 apart); everything before q0
-// lies left of it.  The mass left of the edge is that of the pixels before q0
-// plus S = sum x (area(edge - dist) + half), so detector k's share of the line
-// is 2 half X + S(k + 1) - S(k), X the pixels between the two edges' q0 (one or
-// two, at hand).  Summed over the lines before the lanes meet, so a pixel costs
-// one area instead of two per detector that it might reach (3.3 on average).
-// Bound by the FP64 pipe and the selects around it (51 % and 44 % busy): 1.57 ->
-// 0.51 ms at 512^2, 360 angles; the backward, whose samples come from L2, 1.11 ->
-// 0.31 ms.  64^2, 40 angles: 116 -> 27 and 71 -> 19 us.
+// direction of growing distance, q0 is the first pixel whose footprint's far end
+// lies beyond lane e's edge: everything before it lies left of the edge.  Pixels
+// are max(|c|, |s|) >= b2 apart (sqrt(1/2) lies between the two), so the edge cuts
+// q0 and q0 + 1 at most, the latter left of its centre.  The mass left of the edge
+// is that of the pixels before q0 plus S = sum x (area(edge - dist) + half), so
+// detector k's share of the line is 2 half X + S(k + 1) - S(k), X the pixels
+// between the two edges' q0 (one or two, at hand).  Summed over the lines before
+// the lanes meet, so a pixel costs one area instead of two per detector that it
+// might reach (3.3 on average).  Rounding may move q0 by one pixel; what that puts
+// on the other side of the edge weighs the square of a rounding.
+// Bound by the latency of the lines' loads (four lines on their way) and the FP64
+// pipe: 512^2, 360 angles: pixel by pixel 1.57 ms, three areas a line 0.51, two
+// 0.37; the backward, whose samples come from L2, 1.11 -> 0.31 ms.  64^2, 40
+// angles: 116 -> 27 and 71 -> 17 us.
 // S: of the edge as a beam's left one; Sr: as the right one, which differs at box
 // angles only.
 template <bool ROWS, bool BOX>
@@ -230,29 +235,36 @@ __device__ __forceinline__ void edge_lines(const ParArgs &a, const ParView &v, i
     const double step = fabs(along), kMagic = 6755399441055744.0;   // 1.5 * 2^52: rounds to an integer
     // first pixel with dist > edge - b2: floor(t) + 1, t = (edge - b2 - offset) / step,
     // by the same arithmetic for an edge in every lane
-    auto first = [&](int kk, double ps) { return (((double)kk - 0.5) - ps - v.b2) * inv - 0.5 + kMagic; };
-#pragma unroll 2
+    const double edge = (double)k - 0.5, full = 2.0 * v.half;
+#pragma unroll 4
     for (int l = l0; l < l1; ++l) {
-        const double ps = (double)(l - lmid) * across;
-        const double m = first(k, ps), mn = first(k + 1, ps);
-        const int q0 = __double2loint(m) + 1, two = __double2loint(mn) - __double2loint(m);
-        const double u = (((double)k - 0.5) - ps) - step * ((m - kMagic) + 1.0);
+        const double e = fma(-(double)(l - lmid), across, edge);
+        // floor(t) + 1, t = (e - b2) / step
+        const double m = fma(e - v.b2, inv, -0.5) + kMagic;
+        const int q0 = __double2loint(m) + 1, two = __shfl_down_sync(0xffffffffu, q0, 1) - q0;
+        const double u0 = fma(-step, m - kMagic, e) - step, z1 = step - u0;   // u1 = -z1
         const double *line = img + (size_t)l * len;
-        double x[3];
+        double x[2];
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
+        for (int j = 0; j < 2; ++j) {
             const int i = mid + sg * (q0 + j);
             x[j] = (unsigned)i < (unsigned)len ? __ldg(line + i) : 0.0;
         }
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            // (an infinite pixel turns the sums of the edges near it into NaN:
-            // the caller takes those detectors pixel by pixel)
-            const double uj = fma(-step, (double)j, u), f = par_area(v, uj) + v.half;
-            S = fma(BOX && uj > v.b2 - kParEps ? 2.0 * v.half : f, x[j], S);
-            if (BOX) Sr = fma(uj < -v.b2 + kParEps ? 0.0 : f, x[j], Sr);
+        // (an infinite pixel turns the sums of the edges near it into NaN:
+        // the caller takes those detectors pixel by pixel)
+        // par_area + half: |u0| <= b2 but for rounding, and u1 <= 0
+        const double z0 = fabs(u0), r0 = v.b2 - z0, rest = z0 < v.b1 ? fma(v.height, v.b1 - z0, v.areaT) : v.ramp * r0 * r0;
+        const double f0 = __double2hiint(u0) < 0 ? rest : full - rest;
+        const double r1 = __double2hiint(v.b2 - z1) < 0 ? 0.0 : v.b2 - z1;
+        const double f1 = z1 < v.b1 ? fma(v.height, v.b1 - z1, v.areaT) : v.ramp * r1 * r1;
+        S = fma(BOX && u0 > v.b2 - kParEps ? full : f0, x[0], S);
+        S = fma(f1, x[1], S);
+        if (BOX) {
+            Sr = fma(u0 < -v.b2 + kParEps ? 0.0 : f0, x[0], Sr);
+            Sr = fma(-z1 < -v.b2 + kParEps ? 0.0 : f1, x[1], Sr);
         }
-        X += two > 1 ? x[0] + x[1] : (two == 1 ? x[0] : 0.0);
+        X += two > 0 ? x[0] : 0.0;
+        X += two > 1 ? x[1] : 0.0;
     }
 }
 
@@ -277,7 +289,7 @@ constexpr int kParWarps = 4;
 // y[it, kk] = (y[it, kk] + sum of w * x) / bw.  Block: 4 warps that take the
 // detectors (a.parts = 1) or the lines (4: their sums meet in shared memory, in
 // order) of one angle.
-__global__ void __launch_bounds__(32 * kParWarps)
+__global__ void __launch_bounds__(32 * kParWarps, 6)
 k_par_forward(const ParArgs a, const double *__restrict__ ximg, const double *__restrict__ ximgT,
               double *__restrict__ y)
 {
