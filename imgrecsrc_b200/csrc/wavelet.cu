@@ -538,6 +538,9 @@ __global__ void __launch_bounds__(kHaarThreads) k_admm_haar(const HaarArgs a)
 // and the coarse levels by one warp in shared memory took most.  Per iteration, a
 // launch each / this loop with those / as it stands: 64^2 - / 5.5 / 4.0 us, 512^2
 // - / 5.8 / 4.1, 1024^2 23 / 7.0 / 5.6.
+// The registers hold everything but a and "top" with nothing to spare, and nothing
+// may spill: with 16 bytes of local memory the first pass after a program's other
+// kernels took 25 to 33 ms (1024^2, whole pass), without 0.8.
 constexpr int kLoopTile = 64, kLoopSide = kLoopTile / 4;   // tile, 4 x 4 blocks along its side
 constexpr int kLoopThreads = kLoopSide * kLoopSide;
 
@@ -613,6 +616,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
 {
     const HaarArgs &a = p.h;
     __shared__ float A[16][kLoopThreads];     // a at this thread's pixels
+    __shared__ float stops[kLoopThreads], nutops[kLoopThreads];   // s and nu of "top"
     __shared__ float cells[16];               // the tile's cells of level 4
     __shared__ GridSumsSmem<2, kLoopThreads> sums;
     // half a warp has the 4 x 4 coarse cells of one cell of level 4, l this
@@ -658,7 +662,8 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
         if (tops)
             topm = levels >= 6 && up4 ? coef(p4 >> 1, p4 & 1) : coef((l >> 3) + (p3 & 2), (l >> 1 & 1) + 2 * (p3 & 1));
     }
-    float s[16], nu[16], x[16], stop = 0.0f, nutop = 0.0f;
+    float s[16], nu[16], x[16];
+    nutops[t] = 0.0f;
     // the transform of x into v and top
     auto split = [&](float (&v)[16], float &top) {
         float l1[4];
@@ -689,12 +694,15 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
         x[e] = p.init[q];
         nu[e] = 0.0f;
     }
-    split(s, stop);
+    {
+        float top = 0.0f;
+        split(s, top);
+        stops[t] = topm ? top : 0.0f;
+    }
     __syncthreads();   // cells are read
 #pragma unroll
     for (int e = 0; e < 16; ++e)
         if (!((cm >> e) & 1)) s[e] = 0.0f;
-    if (!topm) stop = 0.0f;
     AdmmState st;
     st.rho = st.nu_mul = 1.0;
     st.tol = fmin(1e-3, p.rel_tol) * sqrt(ss);
@@ -708,7 +716,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
         // x = Psi(s + nu), then alpha = max((a + rho x) / (1 + rho), 0)
         float w0 = fmaf(mul, nu[0], s[0]);
         if (tops) {
-            float top = fmaf(mul, nutop, stop);
+            float top = fmaf(mul, nutops[t], stops[t]);
             if (levels >= 6) {
                 const float u = lane_join(a, top, 2, 8, l & 2, l & 8);
                 if (up4) top = u;
@@ -779,13 +787,15 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
             }
         }
         if (tops) {
+            float nutop = nutops[t];
             const float sn = shrink(nutop, vtop, topm);
+            nutops[t] = nutop;
             if (t < 16) {
-                const double ds = (double)sn, d = ds - (double)stop, r = ds - (double)vtop;
+                const double ds = (double)sn, d = ds - (double)stops[t], r = ds - (double)vtop;
                 ps[0] = fma(d, d, ps[0]);
                 ps[1] = fma(r, r, ps[1]);
             }
-            stop = sn;
+            stops[t] = sn;
         }
         ps[0] += pt[0];
         ps[1] += pt[1];
