@@ -23,7 +23,6 @@
 // of O(n)); that keeps the projections within 1e-7..1e-6 of the FP64 oracle,
 // where the reference's own FP32 build is 1.5e-5 off on signed inputs.
 // The footprint itself is branch-free (footprint.cuh).
-#include <climits>
 #include <cstdio>
 #include <type_traits>
 
@@ -31,6 +30,7 @@
 
 #include "ctprj_internal.h"
 #include "footprint.cuh"
+#include "row_parts.h"
 #include "bhc_spline.cuh"
 
 namespace ctprj {
@@ -417,33 +417,12 @@ __device__ __forceinline__ void march_rows(const Geo &g, const FwdRay &ray, int 
     }
 }
 
-// part s of R of the rows top, top - 1, ..., bottom (none if top < bottom)
-__device__ __forceinline__ void part_rows(int s, int R, int &top, int &bottom)
+// The rows that the rays of a warp can meet (row_parts.h).  Every lane of the
+// warp takes part, lanes without a ray with no rows.
+__device__ __forceinline__ RowRange warp_rows(const FwdRay &ray, bool live, int half)
 {
-    const int M = max(top - bottom + 1, 0), t = top;
-    top = t - (int)((long long)M * s / R);
-    bottom = t - (int)((long long)M * (s + 1) / R) + 1;
-}
-
-// Narrows [top, bottom] to the rows in which a ray of the warp can meet the
-// image: its crossing xc = Ac - y Sc is affine in y, and rows with |xc| > half
-// + 2 are skipped anyway; two rows of margin cover the division's rounding.
-// Every lane of the warp takes part, lanes without a ray with no rows.
-__device__ __forceinline__ void clip_rows(const FwdRay &ray, bool live, int half, int &top, int &bottom)
-{
-    const float A = 0.5f * (ray.Al + ray.Ar), S = 0.5f * (ray.Sl + ray.Sr), lim = (float)half + 2.0f;
-    float lo = (float)-half, hi = (float)half;
-    if (fabsf(S) > 1e-6f) {
-        const float a = __fdividef(A - lim, S), b = __fdividef(A + lim, S);
-        lo = fmaxf(lo, fminf(a, b) - 2.0f);
-        hi = fminf(hi, fmaxf(a, b) + 2.0f);
-    } else if (fabsf(A) > lim + 1.0f) {
-        lo = 1.0f;
-        hi = 0.0f;
-    }
-    const int ylo = live && lo <= hi ? __float2int_rd(lo) : INT_MAX, yhi = live && lo <= hi ? __float2int_ru(hi) : INT_MIN;
-    bottom = max(bottom, __reduce_min_sync(0xffffffffu, ylo));
-    top = min(top, __reduce_max_sync(0xffffffffu, yhi));
+    const RowRange r = live ? ray_rows(0.5f * (ray.Al + ray.Ar), 0.5f * (ray.Sl + ray.Sr), half) : no_rows(half);
+    return {__reduce_min_sync(0xffffffffu, r.bottom), __reduce_max_sync(0xffffffffu, r.top)};
 }
 
 // Stores image j's sum of ray (view b, detector k), scaled, or takes it through
@@ -516,14 +495,13 @@ __device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int b
     if (R != kAllParts) wait_for_table();   // the quad image
     float S[8];
     unsigned long long nz = 0;
-    int rtop = g.half, rbottom = -g.half;
-    if (wcode != 5) clip_rows(ray, live, g.half, rtop, rbottom);
+    RowRange all = {-g.half, g.half};
+    if (wcode != 5) all = warp_rows(ray, live, g.half);
     auto rows_of = [&](int s) {
-        int top = rtop, bottom = rbottom;
-        part_rows(s, p.rsplit, top, bottom);
+        const RowRange r = part_rows(all, s, p.rsplit);
 #pragma unroll
         for (int j = 0; j < 8; ++j) S[j] = 0.0f;
-        if (live && top >= bottom) march_rows<FAN, MODE>(g, ray, wcode, top, bottom, quad, S, nz);
+        if (live && r.top >= r.bottom) march_rows<FAN, MODE>(g, ray, wcode, r.top, r.bottom, quad, S, nz);
     };
     if constexpr (R > 1) {
         // a part of the rows per warp; each warp then takes its share of the images
