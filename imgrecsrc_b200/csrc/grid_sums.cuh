@@ -22,6 +22,10 @@
 //   sums_wait    every block's sums and earlier writes visible (read them past L1)
 //   sums_load    this thread's share of all blocks' sums
 //   sums_fold, __syncthreads, sums_of_block   the sums over all blocks
+// Every warp reads what was folded, so a buffer may be folded into again only
+// after a barrier that follows the sums_post or sums_of_block that read it: the
+// two folds of a round have a buffer each, and the other one's barriers lie
+// between a buffer's uses.
 // Rounds are 1, 2, ...  A wait gives up after two seconds, or as soon as another
 // block's has; the caller then leaves its loop and the host reports the failure.
 #pragma once

@@ -618,7 +618,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
     __shared__ float A[16][kLoopThreads];     // a at this thread's pixels
     __shared__ float stops[kLoopThreads], nutops[kLoopThreads];   // s and nu of "top"
     __shared__ float cells[16];               // the tile's cells of level 4
-    __shared__ GridSumsSmem<2, kLoopThreads> sums;
+    __shared__ GridSumsSmem<2, kLoopThreads> sums[2];   // the block's sums, all blocks' sums
     // half a warp has the 4 x 4 coarse cells of one cell of level 4, l this
     // thread's among them
     const int t = threadIdx.x, ti = blockIdx.y, tj = blockIdx.x;
@@ -633,11 +633,12 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
     // levels 5 and 6 ("top"), which every half warp works out for itself
     const int p3 = (l >> 1 & 2) | (l & 1), p4 = (l >> 2 & 2) | (l >> 1 & 1);
     const bool tops = levels >= 5;
-    unsigned pm = 0xffffu, cm = tops && l == 0 ? 0xfffeu : 0xffffu;
+    // bit e: coefficient e is one of the transform's; bit 16 + e: pixel e may be nonzero
+    unsigned keep = tops && l == 0 ? 0xfffffffeu : 0xffffffffu;
     bool topm = tops;
     if (a.pmask) {
-        pm = 0;
-        for (int e = 0; e < 16; ++e) pm |= (unsigned)(a.pmask[pix + (size_t)(e >> 2) * a.cols + (e & 3)] != 0) << e;
+        for (int e = 0; e < 16; ++e)
+            if (!a.pmask[pix + (size_t)(e >> 2) * a.cols + (e & 3)]) keep &= ~(0x10000u << e);
     }
     if (a.cmask) {
         auto coef = [&](int r, int c) { return a.cmask[loop_coef_index(r, c, ti, tj, levels, a.rows, a.cols)] != 0; };
@@ -657,7 +658,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
                 r = (by >> 1) + (p3 >> 1) * 8;
                 c = (bx >> 1) + (p3 & 1) * 8;
             }
-            if (!coef(r, c)) cm &= ~(1u << e);
+            if (!coef(r, c)) keep &= ~(1u << e);
         }
         if (tops)
             topm = levels >= 6 && up4 ? coef(p4 >> 1, p4 & 1) : coef((l >> 3) + (p3 & 2), (l >> 1 & 1) + 2 * (p3 & 1));
@@ -702,7 +703,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
     __syncthreads();   // cells are read
 #pragma unroll
     for (int e = 0; e < 16; ++e)
-        if (!((cm >> e) & 1)) s[e] = 0.0f;
+        if (!((keep >> e) & 1)) s[e] = 0.0f;
     AdmmState st;
     st.rho = st.nu_mul = 1.0;
     st.tol = fmin(1e-3, p.rel_tol) * sqrt(ss);
@@ -747,7 +748,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
             const float q = (float)((double)fmaf(rho, x[e], A[e][t]) * inv);
-            x[e] = (pm >> e) & 1 ? fmaxf(q, 0.0f) : 0.0f;
+            x[e] = (keep >> (16 + e)) & 1 ? fmaxf(q, 0.0f) : 0.0f;
         }
         if (st.done) break;
         float v[16], vtop = 0.0f;
@@ -769,7 +770,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
         for (int e0 = 0; e0 < 16; e0 += 4) {   // four chains of FP64 latencies side by side
             float sn[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) sn[q] = shrink(nu[e0 + q], v[e0 + q], (cm >> (e0 + q)) & 1);
+            for (int q = 0; q < 4; ++q) sn[q] = shrink(nu[e0 + q], v[e0 + q], (keep >> (e0 + q)) & 1);
             double d[4], r[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -799,15 +800,15 @@ __global__ void __launch_bounds__(kLoopThreads, 2) k_admm_loop(const AdmmLoopArg
         }
         ps[0] += pt[0];
         ps[1] += pt[1];
-        sums_fold(ps, sums);
+        sums_fold(ps, sums[0]);
         __syncthreads();
-        sums_post(p.meet, st.iter + 1, block, nblocks, sums);
+        sums_post(p.meet, st.iter + 1, block, nblocks, sums[0]);
         sums_arrive(p.meet);
-        if (!(ok = sums_wait(p.meet, st.iter + 1, nblocks, sums))) break;
+        if (!(ok = sums_wait(p.meet, st.iter + 1, nblocks, sums[0]))) break;
         sums_load(p.meet, st.iter + 1, nblocks, ps);
-        sums_fold(ps, sums);
+        sums_fold(ps, sums[1]);
         __syncthreads();
-        sums_of_block(ps, sums);
+        sums_of_block(ps, sums[1]);
         admm_advance(&st, ps[0], ps[1]);
     }
     if (!ok) return;

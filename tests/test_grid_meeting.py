@@ -1,0 +1,43 @@
+"""The shared-memory rule of the one-launch loops' meetings (grid_sums.cuh): a
+buffer that every warp of a block reads (sums_post, sums_of_block) is not folded
+into again before a barrier.  Checked on the source of each loop, its body taken
+twice in a row so that the step from one iteration to the next is covered;
+barriers that only some plans reach (inside a lambda) do not count."""
+import os
+import re
+
+import pytest
+
+from imgrecsrc_b200 import build
+
+STEP = re.compile(r"(sums_fold|sums_post|sums_wait|sums_of_block|__syncthreads)\(((?:[^()]|\([^()]*\))*)\)")
+
+
+def loop_body(source, kernel):
+    """Text of the iteration loop (`for` with round or without a condition) of a kernel."""
+    text = open(os.path.join(build.CSRC, source)).read()
+    at = text.index("\n" + kernel) if "\n" + kernel in text else text.index(kernel)
+    at = re.compile(r"for \((unsigned round = 1; !st\.done; \+\+round|;;)\) \{").search(text, at).end()
+    depth, end = 1, at
+    while depth:
+        depth += {"{": 1, "}": -1}.get(text[end], 0)
+        end += 1
+    return re.sub(r"//[^\n]*", "", text[at:end - 1])
+
+
+@pytest.mark.parametrize("source, kernel", [("tv.cu", "k_tv_loop(const TvArgs"), ("wavelet.cu", "k_admm_loop(const AdmmLoopArgs")])
+def test_no_fold_into_a_buffer_that_is_being_read(source, kernel):
+    steps = [(m.group(1), m.group(2).split(",")[-1].strip()) for m in STEP.finditer(loop_body(source, kernel))]
+    names = [s for s, _ in steps]
+    assert names.count("sums_fold") == 2 and names.count("sums_post") == names.count("sums_of_block") == 1
+    reading, folded = set(), set()
+    for step, buf in steps + steps:
+        if step in ("__syncthreads", "sums_wait"):   # sums_wait ends with a barrier
+            reading.clear()
+            folded.clear()
+        elif step == "sums_fold":
+            assert buf not in reading, "%s folds into %s while it is being read" % (kernel, buf)
+            folded.add(buf)
+        else:
+            assert buf not in folded, "%s reads %s before a barrier" % (kernel, buf)
+            reading.add(buf)
