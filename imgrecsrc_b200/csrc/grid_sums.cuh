@@ -27,7 +27,13 @@
 // two folds of a round have a buffer each, and the other one's barriers lie
 // between a buffer's uses.
 // Rounds are 1, 2, ...  A wait gives up after two seconds, or as soon as another
-// block's has; the caller then leaves its loop and the host reports the failure.
+// block's has; the block then leaves its loop without a result.  In the last round
+// one block may give up while the others meet, so the host goes by the failure
+// word as well as by the state that block 0 leaves (loop_met), and then takes the
+// launch-per-iteration kernels, which wait for nothing.  A cooperative launch
+// starts once there is room for all its blocks (beside a kernel that held half the
+// GPU for four seconds the loops started when it ended, and met), so a wait runs
+// out only where the whole GPU is taken from the program for that long.
 #pragma once
 
 namespace ctprj {
@@ -39,6 +45,20 @@ struct GridMeet {
     int *failed;       // zero before the launch
     double *part;      // 2 * K * blocks doubles, 16-byte aligned
 };
+
+// whether a loop's result stands
+inline bool loop_met(int done, int failed) { return done && !failed; }
+
+// Launches a loop's blocks, all of them to be on the GPU at once.  started: false
+// where the device has no room for that; the launch-per-iteration kernels need none.
+inline int launch_loop(const void *kernel, dim3 grid, int threads, size_t smem, void **args, cudaStream_t s, bool *started)
+{
+    const cudaError_t e = cudaLaunchCooperativeKernel(kernel, grid, dim3(threads), args, smem, s);
+    *started = e == cudaSuccess;
+    if (e != cudaErrorCooperativeLaunchTooLarge) return cuda_error(e, "one-launch loop");
+    cudaGetLastError();
+    return CTPRJ_OK;
+}
 
 template <int K, int THREADS>
 struct GridSumsSmem {

@@ -677,16 +677,16 @@ int tv_denoise(TvWorkspace &ws, const float *xobs, int m, int n, double lambda, 
         GridMeet meet = {(unsigned *)(failed + 1), failed, ws.part};
         int tx = (n + kTvpW - 1) / kTvpW;
         void *args[] = {&a, &meet, &out, &tx};
+        bool started = false;
         if ((st = cuda_error(cudaMemsetAsync(a.st, 0, kTvStateBytes, s), "TV start")) ||
-            (st = cuda_error(cudaLaunchCooperativeKernel(loop.kernel, dim3(loop.tiles), dim3(loop.threads), args,
-                                                         loop.smem, s),
-                             "TV loop")) ||
+            (st = launch_loop(loop.kernel, dim3(loop.tiles), loop.threads, loop.smem, args, s, &started)) ||
             (st = cuda_error(cudaMemcpyAsync(&h, a.st, sizeof h, cudaMemcpyDeviceToHost, s), "TV state")) ||
             (st = cuda_error(cudaStreamSynchronize(s), "TV state")))
             return st;
-        if (!h.st.done) return set_error(CTPRJ_ETIMEOUT, "the TV loop's blocks did not meet");
-        if (iterations) *iterations = h.st.iter;
-        return CTPRJ_OK;
+        if (started && loop_met(h.st.done, h.failed)) {
+            if (iterations) *iterations = h.st.iter;
+            return CTPRJ_OK;
+        }
     }
     const int tiles_x = (n + kTvTile - 1) / kTvTile, ntiles = tiles_x * ((m + kTvTile - 1) / kTvTile);
     const dim3 block(32, kTvThreads / 32);

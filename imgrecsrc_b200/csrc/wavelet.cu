@@ -1104,15 +1104,16 @@ int wvlt_admm(WvltProx &ws, const float *a, int rows, int cols, const double *h,
             la.max_itr = max_itr;
             la.levels = levels;
             void *args[] = {&la};
+            bool started = false;
             if ((st = cuda_error(cudaMemsetAsync(dst, 0, kAdmmStateBytes, s), "ADMM start")) ||
-                (st = cuda_error(cudaLaunchCooperativeKernel((void *)k_admm_loop, grid, dim3(kLoopThreads), args, 0, s),
-                                 "ADMM loop")) ||
+                (st = launch_loop((const void *)k_admm_loop, grid, kLoopThreads, 0, args, s, &started)) ||
                 (st = cuda_error(cudaMemcpyAsync(&h, dst, sizeof h, cudaMemcpyDeviceToHost, s), "ADMM state")) ||
                 (st = cuda_error(cudaStreamSynchronize(s), "ADMM state")))
                 return st;
-            if (!h.st.done) return set_error(CTPRJ_ETIMEOUT, "the ADMM loop's blocks did not meet");
-            if (iterations) *iterations = h.st.iter;
-            return CTPRJ_OK;
+            if (started && loop_met(h.st.done, h.failed)) {
+                if (iterations) *iterations = h.st.iter;
+                return CTPRJ_OK;
+            }
         }
     }
     double ss = 0.0;

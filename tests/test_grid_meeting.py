@@ -5,6 +5,7 @@ twice in a row so that the step from one iteration to the next is covered;
 barriers that only some plans reach (inside a lambda) do not count."""
 import os
 import re
+import subprocess
 
 import pytest
 
@@ -41,3 +42,18 @@ def test_no_fold_into_a_buffer_that_is_being_read(source, kernel):
         else:
             assert buf not in folded, "%s reads %s before a barrier" % (kernel, buf)
             reading.add(buf)
+
+
+def test_a_block_that_gave_up_voids_the_result(tmp_path):
+    """Block 0 may finish the last round while another block gives up: the state
+    then says done, and only the failure word tells.  The rule (loop_met) run on
+    the host, and that both loops' hosts go by it."""
+    (tmp_path / "met.cu").write_text('#include "ctprj_internal.h"\n#include "grid_sums.cuh"\nusing namespace ctprj;\n'
+                                     "int main() { return loop_met(1, 0) && !loop_met(1, 1) && !loop_met(0, 0) && "
+                                     "!loop_met(0, 1) ? 0 : 1; }\n")
+    subprocess.run([build.nvcc(), "-std=c++17", "-I", build.CSRC, str(tmp_path / "met.cu"), "-o",
+                    str(tmp_path / "met")] + build.ARCH, check=True)
+    assert subprocess.run([str(tmp_path / "met")]).returncode == 0
+    for source in ("tv.cu", "wavelet.cu"):
+        text = open(os.path.join(build.CSRC, source)).read()
+        assert len(re.findall(r"started && loop_met\(h\.st\.done, h\.failed\)", text)) == 1
