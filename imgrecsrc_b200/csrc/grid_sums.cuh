@@ -46,6 +46,11 @@ struct GridMeet {
     double *part;      // 2 * K * blocks doubles, 16-byte aligned
 };
 
+// Whether `count` arrivals, counted modulo 2^32, are the `want` = round * blocks of
+// a round.  No block is more than one round ahead of another, so the two are less
+// than 2^31 apart; their product passes 2^32 after some 7 million rounds.
+__host__ __device__ inline bool all_in(unsigned count, unsigned want) { return (int)(count - want) >= 0; }
+
 // whether a loop's result stands
 inline bool loop_met(int done, int failed) { return done && !failed; }
 
@@ -135,7 +140,7 @@ __device__ __forceinline__ bool sums_wait(const GridMeet &m, unsigned round, uns
         for (unsigned n = 0;; ++n) {
             unsigned r;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(r) : "l"(m.count) : "memory");
-            if (r >= want) break;
+            if (all_in(r, want)) break;
             if ((n & 255) != 255) continue;   // a long wait: look at the clock
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
             if (t0 == 0) t0 = now;

@@ -57,3 +57,30 @@ def test_a_block_that_gave_up_voids_the_result(tmp_path):
     for source in ("tv.cu", "wavelet.cu"):
         text = open(os.path.join(build.CSRC, source)).read()
         assert len(re.findall(r"started && loop_met\(h\.st\.done, h\.failed\)", text)) == 1
+
+
+def test_the_count_of_arrivals_may_wrap(tmp_path):
+    """Arrivals are counted in 32 bits: in the rounds around 2^32 / blocks a wait
+    still ends when the round's last block is in, and not before."""
+    (tmp_path / "count.cu").write_text(r"""
+#include "ctprj_internal.h"
+#include "grid_sums.cuh"
+using namespace ctprj;
+int main()
+{
+    for (unsigned blocks : {1u, 148u, 592u}) {
+        const unsigned long long wrap = (1ull << 32) / blocks;
+        for (unsigned long long round = 1; round < wrap + 3; round = round == 3 ? wrap - 3 : round + 1) {
+            const unsigned want = (unsigned)round * blocks;
+            for (unsigned long long in = (round - 1) * blocks; in < (round + 1) * blocks; ++in)
+                if (all_in((unsigned)in, want) != (in >= round * blocks)) return 1;
+        }
+    }
+    return 0;
+}
+""")
+    subprocess.run([build.nvcc(), "-std=c++17", "-I", build.CSRC, str(tmp_path / "count.cu"), "-o",
+                    str(tmp_path / "count")] + build.ARCH, check=True)
+    assert subprocess.run([str(tmp_path / "count")]).returncode == 0
+    text = open(os.path.join(build.CSRC, "grid_sums.cuh")).read()
+    assert re.search(r"const unsigned want = round \* nblocks;", text) and "if (all_in(r, want)) break;" in text
