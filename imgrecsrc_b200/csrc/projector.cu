@@ -1869,9 +1869,13 @@ __device__ __forceinline__ int wait_for(const volatile int *word, int want, int 
     }
 }
 
-// Items of slice i: its sample rows, then its tiles.  A sample row waits for
-// the host's flag, a tile for the slice's rows, which blocks that are running
-// have taken before it (items are handed out in order).
+// Items of slice i: its sample rows, then its tiles.  Both wait for the host's
+// flag, a tile then also for the slice's rows, which blocks that are running have
+// taken before it (items are handed out in order).  The host's limit is for the
+// publication alone: the rows, which take microseconds once the flag is up, have
+// at least kRowsNs.
+constexpr unsigned long long kRowsNs = 2000000000ull;
+
 template <int SEG, int VB>
 __global__ void __launch_bounds__(kBwdThreads, CTPRJ_BWD_MINBLOCKS)
 k_backward_stream(const BatchArgs a, const volatile int *__restrict__ ready, int *__restrict__ rows_done,
@@ -1896,9 +1900,8 @@ k_backward_stream(const BatchArgs a, const volatile int *__restrict__ ready, int
         const int local = (int)(item - a.prefix[i] - a.oprefix[i]), rows = (int)(a.oprefix[i + 1] - a.oprefix[i]);
         const bool sample = local < rows;
         if (threadIdx.x == 0)
-            go = ((volatile int *)status)[s] == 0 &&
-                 (sample || rows == 0 ? wait_for(ready + s, 1, status + s, timeout_ns)
-                                      : wait_for(rows_done + s, rows, status + s, timeout_ns));
+            go = ((volatile int *)status)[s] == 0 && wait_for(ready + s, 1, status + s, timeout_ns) &&
+                 (sample || wait_for(rows_done + s, rows, status + s, timeout_ns > kRowsNs ? timeout_ns : kRowsNs));
         __syncthreads();
         if (!go) continue;
         __threadfence();   // the sinogram was published before the flag, the rows before their count
