@@ -462,16 +462,6 @@ __device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int b
     const int b = bx * V + warp % V, seg = warp / V;
     const int r = by * 32 + lane;
     double fsum = 0.0;            // polychromatic mode: this thread's likelihood terms
-    // detector 0 of an even-width sinogram: no ray, zero projection
-    if (MODE != kModeCount && p.zero_col0 && bx == 0 && by == 0)
-        for (int v = threadIdx.x; v < g.np; v += blockDim.x) {
-            if constexpr (MODE == kModeBhc) {
-                fsum += bhc_entry(p.bhc, tab, Ie, 0.0f, (size_t)v * g.W);
-                if (p.bhc.proj_out) p.bhc.proj_out[(size_t)v * g.W] = 0.0f;
-            } else {
-                sino[(size_t)v * g.W] = 0.0f;
-            }
-        }
 
     // The window a warp marches with is the widest any of its rays needs: xr -
     // xl is affine in y, so a ray's widest run is at the first or the last row.
@@ -492,7 +482,19 @@ __device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int b
         }
     }
     wcode = __reduce_max_sync(0xffffffffu, wcode);
-    if (R != kAllParts) wait_for_table();   // the quad image
+    // The quad image.  Until it is there the sinogram is not touched: it may lie
+    // on the image that the first kernel reads.
+    if (R != kAllParts) wait_for_table();
+    // detector 0 of an even-width sinogram: no ray, zero projection
+    if (MODE != kModeCount && p.zero_col0 && bx == 0 && by == 0)
+        for (int v = threadIdx.x; v < g.np; v += blockDim.x) {
+            if constexpr (MODE == kModeBhc) {
+                fsum += bhc_entry(p.bhc, tab, Ie, 0.0f, (size_t)v * g.W);
+                if (p.bhc.proj_out) p.bhc.proj_out[(size_t)v * g.W] = 0.0f;
+            } else {
+                sino[(size_t)v * g.W] = 0.0f;
+            }
+        }
     float S[8];
     unsigned long long nz = 0;
     RowRange all = {-g.half, g.half};
