@@ -245,6 +245,16 @@ __device__ __forceinline__ FwdRay fwd_ray(const FwdParams &p, int b, int k)
 // polychromatic mode.
 constexpr int kAllParts = -1;
 
+// A quad image's entry.  NC: through the read-only path, which holds for data
+// that nothing writes while the kernel runs; a kernel that starts beside the one
+// that builds the image takes an ordinary load.
+template <bool NC>
+__device__ __forceinline__ float4 load_quad(const float4 *q)
+{
+    if constexpr (NC) return __ldg(q);
+    else return *q;
+}
+
 // The rows of one part for one ray: S += the eight images' sums.  Row y reads
 // the quad row |y|:
 //   q[x] = {I(x, |y|), I(x, -|y|), I(|y|, x), I(-|y|, x)},
@@ -253,9 +263,9 @@ constexpr int kAllParts = -1;
 //   S5 += I(y, x), S3 += I(y, -x), S1 += I(-y, x), S7 += I(-y, -x)
 // from q[x] and q[-x]; for y < 0 the pairs of components swap.
 // wcode: 3 / 4: window of 3 / 4 pixels; 5: bounded range loop (one for the warp).
-template <bool FAN, int MODE>
+template <bool FAN, int MODE, bool NC>
 __device__ __forceinline__ void march_rows(const Geo &g, const FwdRay &ray, int wcode, int ytop, int ybot,
-                                           const float4 *__restrict__ quad, float (&S)[8], unsigned long long &nz)
+                                           const float4 *quad, float (&S)[8], unsigned long long &nz)
 {
     const double cR = ray.cR, sR = ray.sR, off = ray.off;
     const float Alf = ray.Al, Slf = ray.Sl, Arf = ray.Ar, Srf = ray.Sr;
@@ -264,7 +274,7 @@ __device__ __forceinline__ void march_rows(const Geo &g, const FwdRay &ray, int 
     const float cRw = ray.cRw, dhbw = ray.dhbw;
     const int half = g.half;
     const int QW = 2 * half + 1;
-    auto march_row = [&](const int y, const float4 *__restrict__ q, auto neg) {
+    auto march_row = [&](const int y, const float4 *q, auto neg) {
         constexpr bool NEG = decltype(neg)::value;
         const float yf = (float)y;
         const float xl = fmaf(-yf, Slf, Alf), xr = fmaf(-yf, Srf, Arf);
@@ -322,15 +332,15 @@ __device__ __forceinline__ void march_rows(const Geo &g, const FwdRay &ray, int 
                 if (p1) nz += (footprint_weight_v(D1, H1, fp) != 0.0f);
                 if (p2) nz += (footprint_weight_v(D2, H2, fp) != 0.0f);
             } else {
-                const float4 pp0 = __ldg(q + x0), pm0 = __ldg(q - x0);
+                const float4 pp0 = load_quad<NC>(q + x0), pm0 = load_quad<NC>(q - x0);
                 float4 pp1 = {}, pm1 = {}, pp2 = {}, pm2 = {};
                 if (p1) {
-                    pp1 = __ldg(q + x0 + 1);
-                    pm1 = __ldg(q - x0 - 1);
+                    pp1 = load_quad<NC>(q + x0 + 1);
+                    pm1 = load_quad<NC>(q - x0 - 1);
                 }
                 if (p2) {
-                    pp2 = __ldg(q + x0 + 2);
-                    pm2 = __ldg(q - x0 - 2);
+                    pp2 = load_quad<NC>(q + x0 + 2);
+                    pm2 = load_quad<NC>(q - x0 - 2);
                 }
                 accumulate(footprint_weight_v(D0, H0, fp), pp0, pm0);
                 if (p1) accumulate(footprint_weight_v(D1, H1, fp), pp1, pm1);
@@ -344,7 +354,7 @@ __device__ __forceinline__ void march_rows(const Geo &g, const FwdRay &ray, int 
                 nz += (footprint_weight_v(D, H, fp) != 0.0f);
                 continue;
             }
-            accumulate(footprint_weight_v(D, H, fp), __ldg(q + x), __ldg(q - x));
+            accumulate(footprint_weight_v(D, H, fp), load_quad<NC>(q + x), load_quad<NC>(q - x));
         }
     };
     // The fixed-window march (plain and polychromatic modes).  Where a
@@ -357,7 +367,7 @@ __device__ __forceinline__ void march_rows(const Geo &g, const FwdRay &ray, int 
     // beam edges differ).  The window is chosen per warp (the widest any
     // of its rays needs), so the warp stays converged.
     const float Acf = 0.5f * (Alf + Arf), Scf = 0.5f * (Slf + Srf);
-    auto march_win = [&](const int y, const float4 *__restrict__ q, auto neg, auto wn) {
+    auto march_win = [&](const int y, const float4 *q, auto neg, auto wn) {
         constexpr bool NEG = decltype(neg)::value;
         constexpr int WN = decltype(wn)::value;
         const float yf = (float)y;
@@ -372,8 +382,8 @@ __device__ __forceinline__ void march_rows(const Geo &g, const FwdRay &ray, int 
         float4 pp[WN], pm[WN];
 #pragma unroll
         for (int j = 0; j < WN; ++j) {
-            pp[j] = __ldg(q + xs + j);
-            pm[j] = __ldg(q - xs - j);
+            pp[j] = load_quad<NC>(q + xs + j);
+            pm[j] = load_quad<NC>(q - xs - j);
         }
 #pragma unroll
         for (int j = 0; j < WN; ++j) {
@@ -453,7 +463,7 @@ __device__ __forceinline__ double put_image(const FwdParams &p, int b, int k, in
 }
 
 template <bool FAN, int MODE, int V, int R>
-__device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int by, const float4 *__restrict__ quad,
+__device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int by, const float4 *quad,
                                                float *__restrict__ sino, unsigned long long *__restrict__ counter,
                                                const double *tab, const double *Ie, float *parts)
 {
@@ -503,7 +513,7 @@ __device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int b
         const RowRange r = part_rows(all, s, p.rsplit);
 #pragma unroll
         for (int j = 0; j < 8; ++j) S[j] = 0.0f;
-        if (live && r.top >= r.bottom) march_rows<FAN, MODE>(g, ray, wcode, r.top, r.bottom, quad, S, nz);
+        if (live && r.top >= r.bottom) march_rows<FAN, MODE, R == kAllParts>(g, ray, wcode, r.top, r.bottom, quad, S, nz);
     };
     if constexpr (R > 1) {
         // a part of the rows per warp; each warp then takes its share of the images
@@ -585,7 +595,7 @@ __host__ __device__ constexpr int fwd_part_floats(int warps) { return warps * 8 
 
 template <bool FAN, int MODE, int V, int R>
 __global__ void __launch_bounds__(32 * V * R, V * R <= 4 ? CTPRJ_FWD_MINBLOCKS : 2)
-k_forward(const FwdParams p, const float4 *__restrict__ quad, float *__restrict__ sino,
+k_forward(const FwdParams p, const float4 *quad, float *__restrict__ sino,
           unsigned long long *__restrict__ counter)
 {
     const double *tab = nullptr, *Ie = nullptr;
