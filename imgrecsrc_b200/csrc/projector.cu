@@ -731,12 +731,27 @@ __device__ __forceinline__ void image_of(int j, int x, int y, int &gx, int &gy)
     }
 }
 
+// A sinogram sample.  LIVE: of a launch during which sinograms arrive (the
+// streaming backprojection): past L1, whose 32-byte sectors may hold the first
+// samples of a slice as they were when its neighbour in memory was read.
+template <bool LIVE>
+__device__ __forceinline__ float load_sample(const float *p)
+{
+    if constexpr (LIVE) {
+        float v;
+        asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+        return v;
+    } else {
+        return __ldg(p);
+    }
+}
+
 // One base view of the pixel-driven backprojection for octant pixel (x, y):
 // the detectors under the pixel's shadow, one footprint weight each, serving
 // the eight symmetric images (prj/cpuPrj.c:213-300).  Everything is read from
 // global memory (L1); used by k_backward_direct and, for views whose tile
 // shadow exceeds the staging capacity, by k_backward_tiled.
-template <bool FAN, bool COUNT, bool FBP>
+template <bool FAN, bool COUNT, bool FBP, bool LIVE = false>
 __device__ __forceinline__ void bwd_view_direct(const BwdParams &p, const float *__restrict__ sino,
                                                 int i, int x, int y, int nimg, float (&S)[8],
                                                 unsigned long long &nz)
@@ -801,10 +816,10 @@ __device__ __forceinline__ void bwd_view_direct(const BwdParams &p, const float 
         for (int j = 0; j < 8; ++j) {
             const int sg = j < 4 ? dt : -dt;
             const int row = bv.row[j];
-            if (row >= 0) S[j] = fmaf(w, __ldg(sino + row + pC + sg), S[j]);
+            if (row >= 0) S[j] = fmaf(w, load_sample<LIVE>(sino + row + pC + sg), S[j]);
             if (!FAN) {
                 const int row2 = bv.row2[j];
-                if (row2 >= 0) S[j] = fmaf(w, __ldg(sino + row2 + pC - sg), S[j]);
+                if (row2 >= 0) S[j] = fmaf(w, load_sample<LIVE>(sino + row2 + pC - sg), S[j]);
             }
         }
     }
@@ -834,7 +849,7 @@ __device__ __forceinline__ void write_octant(const BwdParams &p, float *__restri
 }
 
 // one tile of the unstaged backprojection (plain mode), for persistent use
-template <bool FAN>
+template <bool FAN, bool LIVE>
 __device__ __forceinline__ void backward_tile_direct(const BwdParams &p, int tile,
                                                      const float *__restrict__ sino,
                                                      float *__restrict__ img)
@@ -855,7 +870,7 @@ __device__ __forceinline__ void backward_tile_direct(const BwdParams &p, int til
 #pragma unroll
         for (int j = 0; j < 8; ++j) S[j] = 0.0f;
         unsigned long long nz = 0;
-        for (int i = 0; i < p.nv; ++i) bwd_view_direct<FAN, false, false>(p, sino, i, x, y, nimg, S, nz);
+        for (int i = 0; i < p.nv; ++i) bwd_view_direct<FAN, false, false, LIVE>(p, sino, i, x, y, nimg, S, nz);
         write_octant(p, img, x, y, nimg, S);
     }
 }
@@ -1025,6 +1040,7 @@ __global__ void __launch_bounds__(256) k_footprints(const BwdParams p, float4 *_
 
 // Row i of the sample image (a block's threads along the detectors); the
 // entries beyond the detectors stay zero.
+template <bool LIVE>
 __device__ __forceinline__ void sample_row(const BwdParams &p, const float *__restrict__ sino, int i,
                                            int k0, int step)
 {
@@ -1046,11 +1062,11 @@ __device__ __forceinline__ void sample_row(const BwdParams &p, const float *__re
     for (int k = k0 - dmax; k <= dmax; k += step) {
         float v[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = src[j] ? __ldg(src[j] + (j < 4 ? k : -k)) : 0.0f;
+        for (int j = 0; j < 8; ++j) v[j] = src[j] ? load_sample<LIVE>(src[j] + (j < 4 ? k : -k)) : 0.0f;
         if (!g.fan)
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-                if (src2[j]) v[j] += __ldg(src2[j] - (j < 4 ? k : -k));
+                if (src2[j]) v[j] += load_sample<LIVE>(src2[j] - (j < 4 ? k : -k));
         dst[k] = make_float4(v[0], v[1], v[2], v[3]);
         dst[p.Wp + k] = make_float4(v[4], v[5], v[6], v[7]);
     }
@@ -1065,7 +1081,7 @@ __global__ void __launch_bounds__(kSampThreads) k_samples(const BwdParams p, con
     // one block per SM the early start is worth 2 of 12 us (64^2)
     if (p.tiles_side * (p.tiles_side + 1) / 2 * p.split <= 128) let_next_start();
     for (int i = blockIdx.y; i < p.g.P / 4; i += gridDim.y)
-        sample_row(p, sino, i, blockIdx.x * kSampThreads + threadIdx.x, gridDim.x * kSampThreads);
+        sample_row<false>(p, sino, i, blockIdx.x * kSampThreads + threadIdx.x, gridDim.x * kSampThreads);
 }
 
 constexpr int kBwdThreads = kBwdTile * kBwdTile / 2;   // two pixels per thread
@@ -1798,7 +1814,7 @@ __global__ void __launch_bounds__(kSampThreads) k_samples_batch(const BatchArgs 
     for (long long e = blockIdx.x; e < a.stotal; e += gridDim.x) {
         const int i = find_slot(a.sprefix, a.nslices, e);
         const BatchSlice &sl = a.slices[i];
-        sample_row(sl.bp, sl.bsino, (int)(e - a.sprefix[i]), threadIdx.x, kSampThreads);
+        sample_row<false>(sl.bp, sl.bsino, (int)(e - a.sprefix[i]), threadIdx.x, kSampThreads);
     }
 }
 
@@ -1813,13 +1829,13 @@ struct BatchSmem {
 };
 
 // one tile of a batch slice
-template <int SEG, int VB>
+template <int SEG, int VB, bool LIVE>
 __device__ __forceinline__ void batch_tile(const BatchSlice &sl, int tile, BatchSmem<SEG, VB> &sm)
 {
     const BwdParams &p = sl.bp;
     if (!sl.tiled) {
-        if (p.g.fan) backward_tile_direct<true>(p, tile, sl.bsino, sl.bimg);
-        else backward_tile_direct<false>(p, tile, sl.bsino, sl.bimg);
+        if (p.g.fan) backward_tile_direct<true, LIVE>(p, tile, sl.bsino, sl.bimg);
+        else backward_tile_direct<false, LIVE>(p, tile, sl.bsino, sl.bimg);
     } else if (p.g.fan) {
         if (p.mode == kBwdUnit) backward_tile<true, false, SEG, VB, kBwdUnit>(p, tile, sl.bimg, sm.st.fan, sm.sums);
         else if (p.mode == kBwdNarrow) backward_tile<true, false, SEG, VB, kBwdNarrow>(p, tile, sl.bimg, sm.st.fan, sm.sums);
@@ -1843,7 +1859,7 @@ __global__ void __launch_bounds__(kBwdThreads, CTPRJ_BWD_MINBLOCKS) k_backward_b
         const int i = find_slot(a.prefix, a.nslices, item);
         const BatchSlice &sl = a.slices[a.order[i]];
         const int tile = (int)(item - a.prefix[i]);
-        batch_tile<SEG, VB>(sl, tile, sm);
+        batch_tile<SEG, VB, false>(sl, tile, sm);
     }
 }
 
@@ -1918,12 +1934,12 @@ k_backward_stream(const BatchArgs a, const volatile int *__restrict__ ready, int
         if (!go) continue;
         __threadfence();   // the sinogram was published before the flag, the rows before their count
         if (sample) {
-            sample_row(sl.bp, sl.bsino, local, threadIdx.x, kBwdThreads);
+            sample_row<true>(sl.bp, sl.bsino, local, threadIdx.x, kBwdThreads);
             __threadfence();
             __syncthreads();
             if (threadIdx.x == 0) atomicAdd(&rows_done[s], 1);
         } else {
-            batch_tile<SEG, VB>(sl, local - rows, sm);
+            batch_tile<SEG, VB, true>(sl, local - rows, sm);
         }
     }
 }
