@@ -156,13 +156,15 @@ __device__ __forceinline__ bool sums_wait(const GridMeet &m, unsigned round, uns
     return S.ok;
 }
 
-// this thread's share of every block's sums
+// this thread's share of every block's sums (one to three turns; unrolled, they
+// would take more registers than the loops have left)
 template <int K>
 __device__ __forceinline__ void sums_load(const GridMeet &m, unsigned round, unsigned nblocks, double (&v)[K])
 {
     const double *part = m.part + (size_t)K * nblocks * (round & 1);
 #pragma unroll
     for (int k = 0; k < K; ++k) v[k] = 0.0;
+#pragma unroll 1
     for (unsigned b = threadIdx.x; b < nblocks; b += blockDim.x)
 #pragma unroll
         for (int k = 0; k < K; k += 2) {

@@ -354,8 +354,8 @@ __global__ void k_tv_start(TvState *st, int done)
 // ---- images that fit the GPU's registers and shared memory: one launch ----
 // Up to about 1.2 million pixels every tile of the image has a block of its own
 // on the GPU, so the whole iteration loop is one cooperative launch: a thread
-// keeps the dual P and P_prev of its eight pixels in registers, the tile's Xobs
-// and D stay in shared memory, and per iteration a block reads only its halo of
+// keeps the dual P of its eight pixels in registers (and P_prev, or in shared
+// memory), the tile's Xobs and D stay in shared memory, and per iteration a block reads only its halo of
 // P and writes the edge of its new P.  The blocks meet once per iteration, at the
 // sums of the stopping rule (grid_sums.cuh), after which every block advances its
 // own copy of the scalars: no host check, no second launch.  What bounds an
@@ -363,9 +363,13 @@ __global__ void k_tv_start(TvState *st, int done)
 // and halo from L2) is half; so a thread takes eight rows of one column, whose
 // neighbours above and below are mostly its own, reads shared memory four pixels
 // ahead of their use, posts its sums before the projection, works t out while
-// it waits, and begins the next iteration's R before it takes the sums.  Per
-// iteration, a launch each / this loop in the sums' order / as it stands: 512^2
-// 12.7 / 6.1 / 3.9 us, 768^2 - / 7.6 / 4.9, 1024^2 21 / 10.3 / 10.3.
+// it waits, and begins the next iteration's R before it takes the sums.  Nothing
+// lies in local memory: what a thread keeps between iterations is its P, a word of
+// bits that say where its pixels lie and a few indices.  (With the predicates and
+// addresses kept as well the kernels had stack frames of 32 to 168 bytes.)  Per
+// iteration, a launch each / this loop in the sums' order / with those frames / as
+// it stands: 512^2 12.7 / 6.1 / 3.8 / 3.5 us, 768^2 - / 7.6 / 4.95 / 4.7, 1024^2
+// 21 / 10.3 / 10.4 / 7.3.
 constexpr int kTvpW = 64, kTvpPer = 8;                // tile columns, pixels per thread
 constexpr int tvp_threads(int H) { return H * kTvpW / kTvpPer; }
 
@@ -376,6 +380,9 @@ struct TvpSmem {
     float D[H + 1][kTvpW + 1];    // rows i0 .. i0+H, columns j0 .. j0+W
     float X[H + 1][kTvpW + 1];
     GridSumsSmem<4, tvp_threads(H)> sums, taken;
+    float2 hp[tvp_threads(H)], hq[tvp_threads(H)];   // each thread's halo cell: P and P of the iteration before
+    TvState st[tvp_threads(H) / 32];                 // the scalars, a copy per warp
+    double tkp1[tvp_threads(H) / 32];
 };
 
 template <bool ISO, int H, int PER_SM>
@@ -385,18 +392,46 @@ k_tv_loop(const TvArgs a, const GridMeet meet, float *__restrict__ out, int tile
     extern __shared__ __align__(16) unsigned char tv_smem[];
     TvpSmem<H> &S = *reinterpret_cast<TvpSmem<H> *>(tv_smem);
     constexpr int B = 4;   // pixels whose shared-memory reads are on their way together
-    const int t = threadIdx.x, tx = t % kTvpW, r0 = t / kTvpW * kTvpPer;   // the thread's pixels: (r0 + k, tx)
+    int t = threadIdx.x, tx = t % kTvpW, r0 = t / kTvpW * kTvpPer;   // the thread's pixels: (r0 + k, tx)
     const int i0 = (blockIdx.x / tiles_x) * H, j0 = (blockIdx.x % tiles_x) * kTvpW;
     const int m = a.m, n = a.n, j = j0 + tx;
+    // bits of pixel k: k it lies in the image, 8 + k and not in its last row, 16 + k and
+    // not in its last column, 24 + k and on the tile's edge, another block's halo
+    unsigned at = 0;
+    for (int k = 0; k < kTvpPer; ++k) {
+        const int r = r0 + k, i = i0 + r;
+        const bool in = i < m && j < n, edge = tx == 0 || tx == kTvpW - 1 || r == 0 || r == H - 1;
+        at |= (in ? 1u << k : 0) | (in && i < m - 1 ? 0x100u << k : 0) | (in && j < n - 1 ? 0x10000u << k : 0) |
+              (in && edge ? 0x1000000u << k : 0);
+    }
     const float lam = a.lam, lb = a.lb, ub = a.ub, inv8l = 1.0f / (8.0f * lam);
     for (int e = t; e < (H + 1) * (kTvpW + 1); e += tvp_threads(H)) {
         const int r = e / (kTvpW + 1), c = e % (kTvpW + 1);
         S.X[r][c] = i0 + r < m && j0 + c < n ? a.xobs[(size_t)(i0 + r) * n + j0 + c] : 0.0f;
         S.D[r][c] = 0.0f;
     }
-    float2 P[kTvpPer], Q[kTvpPer];
+    // P of the thread's pixels, and Q: R until P is renewed, then the P before it.  Where
+    // a thread has 64 registers, Q lies in the pixels' own places of R1 and R2, which no
+    // other thread reads between the renewal and the next R.
+    constexpr bool KEEP = PER_SM * tvp_threads(H) <= 512;
+    float2 P[kTvpPer], Q[KEEP ? kTvpPer : 1];
+    auto get_q = [&](int k) {
+        if constexpr (KEEP) return Q[k];
+        else return make_float2(S.R1[r0 + k + 1][tx], S.R2[r0 + k][tx + 1]);
+    };
+    auto set_q = [&](int k, float2 q) {
+        if constexpr (KEEP) {
+            Q[k] = q;
+        } else {
+            S.R1[r0 + k + 1][tx] = q.x;
+            S.R2[r0 + k][tx + 1] = q.y;
+        }
+    };
 #pragma unroll
-    for (int k = 0; k < kTvpPer; ++k) P[k] = Q[k] = make_float2(0.0f, 0.0f);
+    for (int k = 0; k < kTvpPer; ++k) {
+        P[k] = make_float2(0.0f, 0.0f);
+        set_q(k, P[k]);
+    }
     // this thread's halo cell: the row above with the right corner, the row
     // below, the left column with the bottom corner, the right column
     int hr = 0, hc = 0;
@@ -416,42 +451,50 @@ k_tv_loop(const TvArgs a, const GridMeet meet, float *__restrict__ out, int tile
     } else {
         halo = false;
     }
+    // its place in R1 (low half) and R2, 0xffff for none, and the pixel's in the image, -1
     const int hi = i0 + hr, hj = j0 + hc;
-    const bool inside = halo && hi >= 0 && hi < m && hj >= 0 && hj < n;
-    const size_t hx = inside ? (size_t)hi * n + hj : 0;
-    float2 hp = make_float2(0.0f, 0.0f), hq = hp;   // the halo cell's P and P of the iteration before
-    TvState st;
-    st.tk = 1.0;
-    st.c = 0.0;
-    st.fold = INFINITY;
-    st.count = st.iter = 0;
-    st.done = a.max_iter <= 0;
+    unsigned hs = (halo && hc >= 0 ? (hr + 1) * (kTvpW + 1) + hc : 0xffff) |
+                  (halo && hr >= 0 ? hr * (kTvpW + 2) + hc + 1 : 0xffff) << 16;
+    int hx = halo && hi >= 0 && hi < m && hj >= 0 && hj < n ? hi * n + hj : -1, x0 = (i0 + r0) * n + j;
+    S.hp[t] = S.hq[t] = make_float2(0.0f, 0.0f);
+    const TvState &st = S.st[0];   // (every warp's copy says the same)
+    if ((t & 31) == 0) {
+        S.st[t >> 5] = {1.0, 0.0, INFINITY, 0, 0, a.max_iter <= 0, 0u};
+        S.tkp1[t >> 5] = 1.0;
+    }
     bool ok = true;
     __syncthreads();
-    double s[4], tkp1 = 1.0;
+    double s[4];
     for (unsigned round = 1; !st.done; ++round) {
+        // what a thread keeps between rounds, not the predicates and addresses that follow
+        // from these, which do not fit the registers
+        asm volatile("" : "+r"(at), "+r"(hs), "+r"(hx), "+r"(x0), "+r"(t), "+r"(tx), "+r"(r0));
+        TvState &own = S.st[t >> 5];
+        double &tkp1 = S.tkp1[t >> 5];
         // c, which the sums of the last iteration do not decide (a restart tells
         // one iteration later), starts this one before they are taken
-        const float c = (float)st.c;
+        const float c = (float)own.c;
         if (round > 1) sums_load(meet, round - 1, gridDim.x, s);
 #pragma unroll
-        for (int k = 0; k < kTvpPer; ++k) {   // Q: R until P is renewed
-            Q[k].x = fmaf(c, P[k].x - Q[k].x, P[k].x);
-            Q[k].y = fmaf(c, P[k].y - Q[k].y, P[k].y);
-            S.R2[r0 + k][tx + 1] = Q[k].y;
+        for (int k = 0; k < kTvpPer; ++k) {
+            float2 q = get_q(k);
+            q.x = fmaf(c, P[k].x - q.x, P[k].x);
+            q.y = fmaf(c, P[k].y - q.y, P[k].y);
+            set_q(k, q);
+            S.R2[r0 + k][tx + 1] = q.y;
+            if (k == kTvpPer - 1) S.R1[r0 + k + 1][tx] = q.x;
         }
-        S.R1[r0 + kTvpPer][tx] = Q[kTvpPer - 1].x;
-        if (halo) {   // R on the halo
-            const float r1 = fmaf(c, hp.x - hq.x, hp.x), r2 = fmaf(c, hp.y - hq.y, hp.y);
-            if (hc >= 0) S.R1[hr + 1][hc] = r1;
-            if (hr >= 0) S.R2[hr][hc + 1] = r2;
-        }
+        // R on the halo
+        const float2 hp = S.hp[t], hq = S.hq[t];
+        if ((hs & 0xffff) != 0xffff) S.R1[0][hs & 0xffff] = fmaf(c, hp.x - hq.x, hp.x);
+        if (hs >> 16 != 0xffff) S.R2[0][hs >> 16] = fmaf(c, hp.y - hq.y, hp.y);
         if (round > 1) sums_fold(s, S.taken);
         __syncthreads();
         if (round > 1) {
             sums_of_block(s, S.taken);
-            tv_advance(&st, s, a.max_iter, a.eps, tkp1);
-            if (st.done) break;
+            if ((t & 31) == 0) tv_advance(&own, s, a.max_iter, a.eps, tkp1);
+            __syncwarp();
+            if (own.done) break;
         }
         // C = Xobs - lambda L(R), D = clamp(C) on the tile (partials) and its halo
         s[0] = s[1] = s[2] = s[3] = 0.0;
@@ -467,8 +510,8 @@ k_tv_loop(const TvArgs a, const GridMeet meet, float *__restrict__ out, int tile
             }
 #pragma unroll
             for (int k = 0; k < B; ++k) {
-                const float2 R = Q[k0 + k];
-                const bool in = i0 + r0 + k0 + k < m && j < n;
+                const float2 R = get_q(k0 + k);
+                const bool in = at >> (k0 + k) & 1;
                 const float C = in ? fmaf(-lam, (R.x - up) + (R.y - left[k]), X[k]) : 0.0f;
                 up = R.x;
                 const float Dv = in ? fminf(fmaxf(C, lb), ub) : 0.0f;
@@ -503,10 +546,9 @@ k_tv_loop(const TvArgs a, const GridMeet meet, float *__restrict__ out, int tile
             }
 #pragma unroll
             for (int k = 0; k < B; ++k) {
-                const int i = i0 + r0 + k0 + k;
-                const float2 R = Q[k0 + k];
-                float p1 = i < m - 1 && j < n ? fmaf(d - down[k], inv8l, R.x) : 0.0f;
-                float p2 = i < m && j < n - 1 ? fmaf(d - right[k], inv8l, R.y) : 0.0f;
+                const float2 R = get_q(k0 + k);
+                float p1 = at >> (8 + k0 + k) & 1 ? fmaf(d - down[k], inv8l, R.x) : 0.0f;
+                float p2 = at >> (16 + k0 + k) & 1 ? fmaf(d - right[k], inv8l, R.y) : 0.0f;
                 d = down[k];
                 if (ISO) {   // P / max(1, |P|): scaled only outside the unit ball
                     const float q2 = fmaf(p1, p1, p2 * p2), rs = rsqrtf(fmaxf(q2, 1.0f));
@@ -516,31 +558,23 @@ k_tv_loop(const TvArgs a, const GridMeet meet, float *__restrict__ out, int tile
                     p1 = fminf(fmaxf(p1, -1.0f), 1.0f);
                     p2 = fminf(fmaxf(p2, -1.0f), 1.0f);
                 }
-                Q[k0 + k] = P[k0 + k];
+                set_q(k0 + k, P[k0 + k]);
                 P[k0 + k] = make_float2(p1, p2);
+                // only the tile's edge is another block's halo
+                if (at >> (24 + k0 + k) & 1) __stcg(N + x0 + (k0 + k) * n, P[k0 + k]);
             }
-        }
-        // only the tile's edge is another block's halo
-        const bool side = tx == 0 || tx == kTvpW - 1;
-#pragma unroll
-        for (int k = 0; k < kTvpPer; ++k) {
-            const int r = r0 + k, i = i0 + r;
-            if (i < m && j < n && (side || (k == 0 && r == 0) || (k == kTvpPer - 1 && r == H - 1)))
-                __stcg(N + (size_t)i * n + j, P[k]);
         }
         __syncthreads();
         sums_arrive(meet);
-        tkp1 = tv_next_t(st.tk, st.c);
+        if ((t & 31) == 0) tkp1 = tv_next_t(own.tk, own.c);
         if (!(ok = sums_wait(meet, round, gridDim.x, S.sums))) break;
-        hq = hp;
-        if (inside) hp = __ldcg(N + hx);
+        S.hq[t] = S.hp[t];
+        if (hx >= 0) S.hp[t] = __ldcg(N + hx);
     }
     if (!ok) return;
 #pragma unroll
-    for (int k = 0; k < kTvpPer; ++k) {
-        const int r = r0 + k, i = i0 + r;
-        if (i < m && j < n) out[(size_t)i * n + j] = S.D[r][tx];
-    }
+    for (int k = 0; k < kTvpPer; ++k)
+        if (at >> k & 1) out[x0 + k * n] = S.D[r0 + k][tx];
     if (blockIdx.x == 0 && t == 0) {
         a.st->iter = st.iter;
         a.st->done = 1;
@@ -613,10 +647,9 @@ void TvWorkspace::release(cudaStream_t s)
 }
 
 // The loop's variant for an image.  Up to two 32-row tiles per SM a thread may
-// take 128 registers; beyond, two blocks per SM of twice the rows meet a little
-// sooner than four (1024^2: 10.3 us per iteration against 11.2, 1056^2 10.6
-// against 12.0), and those four are left for the sizes whose 64-row tiles would
-// not all fit.
+// take 128 registers; beyond, two blocks per SM of twice the rows meet sooner
+// than four (1024^2: 7.3 us per iteration against 8.3, 1056^2 7.5 against 8.7),
+// and those four are left for the sizes whose 64-row tiles would not all fit.
 struct TvLoop {
     const void *kernel;
     int tiles, threads;
