@@ -154,54 +154,35 @@ __device__ __forceinline__ double par_area(const ParView &v, double u)
 }
 
 // sum of w * x over the pixels that reach detector kk, added to acc: the
-// pixel's own range test (prj/parPrj.c:124-125) and weight (:133-168).  The
-// rows a column can contribute are bracketed from |dist - k| <= b2 + bw/2 with
-// a margin.
-__device__ __noinline__ double par_gather(const ParArgs &a, const ParView &v, double k, const double *__restrict__ ximg,
-                                          const double *__restrict__ ximgT, double acc)
+// pixel's own range test (prj/parPrj.c:124-125) and weight (:133-168).  Lines as
+// the edge form takes them; the pixels of one that can reach the detector are
+// bracketed from |dist - k| <= b2 + bw/2 with a margin.
+__device__ __forceinline__ double par_gather(const ParArgs &a, const ParView &v, double k, const double *__restrict__ ximg,
+                                             const double *__restrict__ ximgT, double acc)
 {
+    const bool rows = fabs(v.s) < fabs(v.c);   // the band is closer to the columns
     const double hw = v.b2 + a.bw / 2 + 1e-6;
-    const double ylo = (double)-a.yC, yhi = (double)(a.nr - 1 - a.yC);
-    const double xlo = (double)-a.xC, xhi = (double)(a.nc - 1 - a.xC);
-    auto add = [&](int px, int py, double xv) {
-        if (xv == 0.0) return;
-        const double dist = par_dist(v, px, py);
-        const double ub = floor(dist + v.b2 + a.bw / 2 - kParEps);
-        const double lb = ceil(dist - v.b2 - a.bw / 2 + kParEps);
-        if (k < lb || k > ub) return;
-        const double w = par_overlap(v, dist, k, a.bw);
-        if (w != 0.0) acc += w * xv;
-    };
-    if (fabs(v.s) < fabs(v.c)) {
-        // the band is closer to the columns: row by row, a few columns each
-        for (int ry = 0; ry < a.nr; ++ry) {
-            const int py = ry - a.yC;
-            const double ps = (double)py * v.s;
-            double c0 = (k - hw - ps) * v.inv_c, c1 = (k + hw - ps) * v.inv_c;
-            if (c0 > c1) { const double t = c0; c0 = c1; c1 = t; }
-            const int px0 = (int)ceil(fmax(c0, xlo)), px1 = (int)floor(fmin(c1, xhi));
-            const double *row = ximgT + (size_t)ry * a.nc + a.xC;
-            for (int px = px0; px <= px1; ++px) add(px, py, row[px]);
+    const double across = rows ? v.s : v.c, inv = rows ? v.inv_c : v.inv_s;
+    const int lines = rows ? a.nr : a.nc, lmid = rows ? a.yC : a.xC;
+    const int len = rows ? a.nc : a.nr, mid = rows ? a.xC : a.yC;
+    const double *line = (rows ? ximgT : ximg) + mid;
+#pragma unroll 1
+    for (int l = -lmid; l < lines - lmid; ++l, line += len) {
+        const double o = (double)l * across;
+        const double r0 = (k - hw - o) * inv, r1 = (k + hw - o) * inv;
+        const int q0 = (int)ceil(fmax(fmin(r0, r1), (double)-mid));
+        const int q1 = (int)floor(fmin(fmax(r0, r1), (double)(len - 1 - mid)));
+#pragma unroll 1
+        for (int q = q0; q <= q1; ++q) {
+            const double xv = line[q];
+            if (xv == 0.0) continue;
+            const double dist = rows ? par_dist(v, q, l) : par_dist(v, l, q);
+            const double ub = floor(dist + v.b2 + a.bw / 2 - kParEps);
+            const double lb = ceil(dist - v.b2 - a.bw / 2 + kParEps);
+            if (k < lb || k > ub) continue;
+            const double w = par_overlap(v, dist, k, a.bw);
+            if (w != 0.0) acc += w * xv;
         }
-        return acc;
-    }
-    for (int cx = 0; cx < a.nc; ++cx) {
-        const int px = cx - a.xC;
-        const double pc = (double)px * v.c;
-        double r0, r1;
-        if (v.inv_s != 0.0) {
-            r0 = (k - hw - pc) * v.inv_s;
-            r1 = (k + hw - pc) * v.inv_s;
-            if (r0 > r1) { const double t = r0; r0 = r1; r1 = t; }
-        } else if (fabs(pc - k) <= hw) {
-            r0 = ylo;
-            r1 = yhi;
-        } else {
-            continue;
-        }
-        const int py0 = (int)ceil(fmax(r0, ylo)), py1 = (int)floor(fmin(r1, yhi));
-        const double *col = ximg + (size_t)cx * a.nr + a.yC;
-        for (int py = py0; py <= py1; ++py) add(px, py, col[py]);
     }
     return acc;
 }
@@ -221,7 +202,8 @@ __device__ __noinline__ double par_gather(const ParArgs &a, const ParView &v, do
 // on the other side of the edge weighs the square of a rounding.
 // Bound by the latency of the lines' loads (four lines on their way) and the FP64
 // pipe: 512^2, 360 angles: pixel by pixel 1.57 ms, three areas a line 0.51, two
-// 0.37; the backward, whose samples come from L2, 1.11 -> 0.31 ms.  64^2, 40
+// 0.37; the backward, whose samples come from L2, 1.11 -> 0.31 ms (0.30 -> 0.27
+// without local memory).  64^2, 40
 // angles: 116 -> 27 and 71 -> 17 us.
 // S: of the edge as a beam's left one; Sr: as the right one, which differs at box
 // angles only.
@@ -341,10 +323,11 @@ k_par_forward(const ParArgs a, const double *__restrict__ ximg, const double *__
         for (int e = nd + lane; e < a.W; e += 32) yr[e] /= a.bw;
 }
 
-// x = (x + sum of w * y) / bw over angles and detectors.  In the edge form a
-// footprint is cut by the edges e1 and e2 of at most three detectors k0 .. k0 + 2
+// x = (x + sum of w * y) / bw over angles and detectors.  EDGES: every angle has
+// the edge form (the kernel then holds no division, whose calls would keep
+// registers in local memory).  In the edge form a footprint is cut by the edges e1 and e2 of at most three detectors k0 .. k0 + 2
 // (2 b2 + 1 <= 2.42); the outer edges lie outside it but for 1e-8.
-__device__ __noinline__ double par_back_angle(const ParArgs &a, const ParView &v, const double *__restrict__ row,
+__device__ __forceinline__ double par_back_angle(const ParArgs &a, const ParView &v, const double *__restrict__ row,
                                                  int px, int py, double acc)
 {
     const double dist = par_dist(v, px, py);
@@ -360,7 +343,8 @@ __device__ __noinline__ double par_back_angle(const ParArgs &a, const ParView &v
 
 constexpr int kParViews = 64;
 
-__global__ void __launch_bounds__(kParThreads)
+template <bool EDGES>
+__global__ void __launch_bounds__(kParThreads, EDGES ? 0 : 3)
 k_par_backward(const ParArgs a, const double *__restrict__ y, const double *__restrict__ mask,
                long long npix, double *__restrict__ x)
 {
@@ -388,7 +372,7 @@ k_par_backward(const ParArgs a, const double *__restrict__ y, const double *__re
 #pragma unroll 2
         for (int q = q0; q < q1; ++q, row += a.W) {
             const ParView &v = views[q];
-            if (!v.edges) {
+            if (!EDGES && !v.edges) {
                 if (live) acc = par_back_angle(a, v, row, px, py, acc);
                 continue;
             }
@@ -419,7 +403,7 @@ k_par_backward(const ParArgs a, const double *__restrict__ y, const double *__re
         if (p != 0) return;
         for (int q = 1; q < parts; ++q) acc += part[q * per + t];
     }
-    if (live) x[i] = acc / a.bw;
+    if (live) x[i] = EDGES ? acc : acc / a.bw;   // (the edge form has bw = 1)
 }
 
 static int par_validate(const ctprj_par_conf *c, long long npix)
@@ -449,10 +433,15 @@ static ParArgs par_args(const ctprj_par_conf *c, const ParView *view)
 }
 
 // view table in stream-ordered device memory (released after the kernels)
-static int par_table(const ctprj_par_conf *c, const double *theta, ParView **d_view, cudaStream_t s)
+static int par_table(const ctprj_par_conf *c, const double *theta, ParView **d_view, cudaStream_t s,
+                     bool *edges = nullptr)
 {
     std::vector<ParView> tab((size_t)(c->np > 0 ? c->np : 1));
     for (int it = 0; it < c->np; ++it) tab[it] = par_view(theta[it], c->bw);
+    if (edges) {
+        *edges = true;
+        for (int it = 0; it < c->np; ++it) *edges = *edges && tab[it].edges;
+    }
     int st = cuda_error(cudaMallocAsync((void **)d_view, sizeof(ParView) * tab.size(), s),
                         "parPrj view table");
     if (st) return st;
@@ -528,12 +517,14 @@ extern "C" int ctprj_par_backward(const ctprj_par_conf *conf, const double *thet
         return set_error(CTPRJ_EINVAL, "NULL buffer");
     cudaStream_t s = (cudaStream_t)stream;
     ParView *d_view = nullptr;
-    if ((st = par_table(conf, theta_host, &d_view, s))) return st;
+    bool edges = false;
+    if ((st = par_table(conf, theta_host, &d_view, s, &edges))) return st;
     ParArgs a = par_args(conf, d_view);
     // few pixels share each one's angles among eight threads
     a.parts = npix < 384LL * sm_count() ? 8 : 1;
     const int per = kParThreads / a.parts, blocks = (int)((npix + per - 1) / per);
-    k_par_backward<<<blocks, kParThreads, 0, s>>>(a, d_y, d_mask, npix, d_x);
+    if (edges) k_par_backward<true><<<blocks, kParThreads, 0, s>>>(a, d_y, d_mask, npix, d_x);
+    else k_par_backward<false><<<blocks, kParThreads, 0, s>>>(a, d_y, d_mask, npix, d_x);
     st = cuda_error(cudaGetLastError(), "parPrj backward");
     cudaFreeAsync(d_view, s);
     return st;

@@ -11,7 +11,7 @@ import pytest
 from imgrecsrc_b200 import build
 
 
-@pytest.mark.parametrize("source, kernel", [("tv.cu", "k_tv_loop"), ("wavelet.cu", "k_admm_loop")])
+@pytest.mark.parametrize("source, kernel", [("tv.cu", "k_tv_loop"), ("wavelet.cu", "k_admm_loop"), ("parprj.cu", "k_par_")])
 def test_no_stack_frame(source, kernel, tmp_path):
     r = subprocess.run([build.nvcc()] + build.ARCH + build.FLAGS + ["-Xptxas", "-v", "-c", os.path.join(build.CSRC, source), "-o",
                         str(tmp_path / "a.o")], capture_output=True, text=True, check=True)
