@@ -149,7 +149,11 @@ void fill_det_table(const Geo &g, DetEntry *de)
 static void free_plan(ctprj_plan *p)
 {
     if (!p) return;
-    cudaFree(p->d_arena);
+    // The pool waits for nothing when memory goes back to it: what still runs on the
+    // plan ends before cudaFree of d_wait returns.  (Where that fails, as during a
+    // capture, the arena stays allocated, too.)
+    if (!p->d_wait) cudaFree(p->d_arena);
+    else if (cudaFree(p->d_wait) == cudaSuccess) cudaFreeAsync(p->d_arena, 0);
     cudaFree(p->d_ramp);
     cudaFree(p->d_fsino);
     cudaFree(p->d_mimg);
@@ -222,7 +226,11 @@ static int build_plan(const ctprj_geometry *geom, int device, ctprj_plan **out)
     if ((st = dg.status)) { delete p; return st; }
     // One allocation and one upload for the plan: the host-built tables and the
     // counter, then the quad image and the staged backprojection's tables (an
-    // allocation of its own for each took most of a plan's creation).
+    // allocation of its own for each took most of a plan's creation).  Between 1 and
+    // 32 MB it comes from the device's memory pool: cudaMalloc maps new memory for
+    // every request above 1 MB, 0.35 ms each, the pool maps 32 MB at a time, and only
+    // the first of a program's plans pays (plans that are kept, cudaMalloc / pool:
+    // 256^2 parallel 400 / 68 us, 512^2 fan 404 / 82; 64^2, 0.1 MB, 47 / 49).
     struct Part {
         size_t at, bytes;
     };
@@ -243,12 +251,23 @@ static int build_plan(const ctprj_geometry *geom, int device, ctprj_plan **out)
     memcpy(&host[pb.at], bv.data(), pb.bytes);
     memcpy(&host[pd.at], de.data(), pd.bytes);
     bool tables = true;
-    if (cudaMalloc((void **)&p->d_arena, total) != cudaSuccess) {
+    auto arena = [&](size_t bytes) {
+        if (bytes > (1u << 20) && bytes <= (32u << 20) && cudaMalloc((void **)&p->d_wait, 1) == cudaSuccess) {
+            if (cudaMallocAsync((void **)&p->d_arena, bytes, 0) == cudaSuccess) return true;
+            cudaFree(p->d_wait);   // no pool, or short of memory
+        }
+        cudaGetLastError();
+        p->d_wait = p->d_arena = nullptr;
+        if (cudaMalloc((void **)&p->d_arena, bytes) == cudaSuccess) return true;
+        p->d_arena = nullptr;
+        return false;
+    };
+    if (!arena(total)) {
         // no room for the tables: the unstaged backprojection needs none
         cudaGetLastError();
-        p->d_arena = nullptr;
         tables = false;
-        if ((st = cuda_error(cudaMalloc((void **)&p->d_arena, without), "plan allocation"))) {
+        if (!arena(without)) {
+            st = cuda_error(cudaGetLastError(), "plan allocation");
             free_plan(p);
             return st;
         }

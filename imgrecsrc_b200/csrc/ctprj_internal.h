@@ -135,7 +135,8 @@ struct ctprj_plan {
     int bwd_seg;              // staged detectors per view and tile (32, 64), 0: unstaged
     int bwd_split;            // parts the staged backprojection sums the base views in
     float4 *d_samp, *d_foot;  // staged backprojection: sample image (scratch) and footprint table
-    char *d_arena;            // the plan's one allocation, which the next pointers lead into
+    char *d_arena;            // the plan's one large allocation, which the next pointers lead into
+    char *d_wait;             // an ordinary allocation, where the arena is the memory pool's
     ctprj::FwdView *d_fview;
     ctprj::BwdView *d_bview;
     ctprj::DetEntry *d_det;
