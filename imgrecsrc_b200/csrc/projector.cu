@@ -535,17 +535,15 @@ __device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int b
     }
     rows_of(0);
     if constexpr (R == kAllParts) {
-        if (p.rsplit > 1) {
-            float *tot = parts + threadIdx.x;
-            const int step = blockDim.x;
-            for (int s = 1; s < p.rsplit; ++s) {
+        float *tot = parts + threadIdx.x;
+        const int step = blockDim.x;
+        for (int s = 1; s < p.rsplit; ++s) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) tot[j * step] = s == 1 ? S[j] : tot[j * step] + S[j];
-                rows_of(s);
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) S[j] = tot[j * step] + S[j];
+            for (int j = 0; j < 8; ++j) tot[j * step] = s == 1 ? S[j] : tot[j * step] + S[j];
+            rows_of(s);
         }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) S[j] = tot[j * step] + S[j];
     }
     if (!live) return fsum;
     if constexpr (MODE == kModeCount) {
@@ -555,34 +553,6 @@ __device__ __forceinline__ double forward_rays(const FwdParams &p, int bx, int b
             if (p.view[b].out[j] >= 0) entries += (!FAN && 2 * g.pC - det != det) ? 2 : 1;
         }
         if (nz * entries) atomicAdd(counter, nz * entries);
-    } else if constexpr (MODE == kModeBhc) {
-        // the entries this ray sum feeds, gathered first so that one copy of
-        // the FP64 epilogue serves them all
-        const int pC = g.pC;
-        float eval[16];
-        int eidx[16];
-        int ne = 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int v = p.view[b].out[j];
-            if (v < 0) continue;
-            const int det = j < 4 ? k : 2 * pC - k;
-            const int det2 = 2 * pC - det;
-            const size_t row = (size_t)v * g.W;
-            if (FAN) {
-                eval[ne] = S[j] / g.effRate; eidx[ne++] = (int)(row + det);
-            } else if (det2 != det) {
-                eval[ne] = S[j] / g.effRate; eidx[ne++] = (int)(row + det);
-                eval[ne] = S[j ^ 2] / g.effRate; eidx[ne++] = (int)(row + det2);
-            } else {
-                eval[ne] = S[j ^ 2] / g.effRate; eidx[ne++] = (int)(row + det);
-            }
-        }
-#pragma unroll 1
-        for (int e = 0; e < ne; ++e) {
-            fsum += bhc_entry(p.bhc, tab, Ie, eval[e], (size_t)eidx[e]);
-            if (p.bhc.proj_out) p.bhc.proj_out[eidx[e]] = eval[e];
-        }
     } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) put_image<FAN, MODE>(p, b, k, j, S[j], sino, tab, Ie);
@@ -622,19 +592,23 @@ k_forward(const FwdParams p, const float4 *quad, float *__restrict__ sino,
 // even as a long one's (equal parts of the image's rows leave the outer ones
 // empty towards the detectors' ends; 512^2 fan 112 us, parallel 101, 1001^2
 // 523).  The base rays alone fill only part of the GPU below 1024^2 (276 warps
-// at 256^2, where it holds 2960), and up to three and a half waves of warps a
-// split still evens out the rays' uneven ways through the image.  Measured,
-// 1 / 2 / 4 / 8 parts: 64^2 fan 28.7 / 18.5 / 12.4 / 10.3 us, 256^2 parallel 84
-// / 49 / 29 / 21, 512^2 fan (1024 detectors) 178 / 144 / 118 / 101, parallel 165
-// / 107 / 85 / 86, 1001^2 parallel 590 / 522 / 476 / 497, 1024^2 fan (1536
-// views) 561 / 576 / 547 / 549, 2048^2 fan 3522 / 3442 / 3413 / 3546: the long
-// sums of 2048^2 stay in one part.
+// at 256^2, where it holds 2960), so up to three and a half waves of warps come
+// from a split.  Beyond that it evens out the rays' uneven ways through the image:
+// two parts while those are within seven waves, four for the long sums above
+// (whose parts are still hundreds of rows).  Measured, 1 / 2 / 4 / 8 parts: 64^2
+// fan 28.7 / 18.5 / 12.4 / 10.3 us, 256^2 parallel 84 / 49 / 29 / 21, 512^2 fan
+// (1024 detectors) 172 / 142 / 117 / 100, parallel 165 / 107 / 85 / 86, 1001^2
+// parallel 582 / 521 / 474 / 494, 1024^2 fan (1536 detectors) 560 / 571 / 542 /
+// 546, 1500^2 fan 1587 / 1547 / 1538 / 1632 and with the polychromatic epilogue
+// 1752 / 1681 / 1697 / 1835, 2048^2 fan 3505 / 3442 / 3398 / 3521 and 3801 / 3706
+// / 3701 / 3900, 2048^2 parallel 3750 / 3525 / 3485 / 3668.
 static int forward_split(const ctprj_plan *pl)
 {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pl->device);
     const long long warps = (long long)pl->nb * ((pl->nk + 31) / 32), wave = 4LL * CTPRJ_FWD_MINBLOCKS * sms;
-    int R = 1;
+    if (2 * warps >= 7 * wave) return 4;
+    int R = 2;
     while (R < 8 && 2 * warps * R < 7 * wave) R *= 2;
     return R;
 }
@@ -675,7 +649,6 @@ static cudaError_t launch_forward_t(const FwdParams &p, dim3 grid, const float4 
                                     unsigned long long *counter, cudaStream_t s)
 {
     switch (p.rsplit) {
-    case 1: return launch_after_table(k_forward<FAN, MODE, kFwdViews, 1>, grid, kFwdThreads, 1, s, p, quad, sino, counter);
     case 2: return launch_after_table(k_forward<FAN, MODE, kFwdViews / 2, 2>, grid, kFwdThreads, 1, s, p, quad, sino, counter);
     case 4: return launch_after_table(k_forward<FAN, MODE, 1, 4>, grid, kFwdThreads, 1, s, p, quad, sino, counter);
     default: return launch_after_table(k_forward<FAN, MODE, 1, 8>, grid, 256, 1, s, p, quad, sino, counter);
