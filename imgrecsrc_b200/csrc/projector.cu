@@ -18,10 +18,13 @@
 //            detectors under the pair's shadow, staged in shared memory; each
 //            thread owns its sixteen output pixels, so no atomics are needed.
 //
-// Precision: the weights are FP32 but each distance from a ray is evaluated in
-// FP64 before rounding (x cos R + y sin R - offset cancels to O(1) from terms
-// of O(n)); that keeps the projections within 1e-7..1e-6 of the FP64 oracle,
-// where the reference's own FP32 build is 1.5e-5 off on signed inputs.
+// Precision: the weights are FP32, but x cos R + y sin R - offset, which cancels
+// to O(1) from terms of O(n), is formed in FP64 and then rounded: in the forward
+// per row of a ray, in the unstaged backprojection per pixel and detector, in the
+// staged one per 8 x 8 square and view, from where FP32 steps of a few units lead
+// to the square's pixels and detectors.  That keeps the projections within
+// 1e-7..1e-6 of the FP64 oracle, where the reference's own FP32 build is 1.5e-5
+// off on signed inputs.
 // The footprint itself is branch-free (footprint.cuh).
 #include <cstdio>
 #include <type_traits>
@@ -722,8 +725,9 @@ __device__ __forceinline__ float load_sample(const float *p)
 // One base view of the pixel-driven backprojection for octant pixel (x, y):
 // the detectors under the pixel's shadow, one footprint weight each, serving
 // the eight symmetric images (prj/cpuPrj.c:213-300).  Everything is read from
-// global memory (L1); used by k_backward_direct and, for views whose tile
-// shadow exceeds the staging capacity, by k_backward_tiled.
+// global memory (L1); used by k_backward and backward_tile_direct, which a plan
+// takes as a whole where any view's tile shadow exceeds the staging capacity (the
+// staged kernel counts on every span fitting its buffers).
 template <bool FAN, bool COUNT, bool FBP, bool LIVE = false>
 __device__ __forceinline__ void bwd_view_direct(const BwdParams &p, const float *__restrict__ sino,
                                                 int i, int x, int y, int nimg, float (&S)[8],

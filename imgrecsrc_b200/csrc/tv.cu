@@ -26,7 +26,8 @@
 // (count, restart, t, the momentum coefficient, done), so every decision
 // stays on the device; the host checks the done flag every eight
 // iterations, and launches after convergence change nothing.  Images that fit
-// the GPU's registers and shared memory take k_tv_loop instead.
+// the GPU's registers and shared memory take k_tv_loop instead, one launch that the
+// host waits for once.
 #include <algorithm>
 #include <cmath>
 

@@ -20,8 +20,13 @@
  * i * cols + j.  The reference's images are column-major MATLAB arrays; since
  * the iteration treats the two axes alike, passing a column-major image with
  * rows and cols swapped gives the same D up to FP32 rounding.  All calls are
- * enqueued on `stream`; ctprj_tv_denoise synchronises it every eight
- * iterations to read the stopping flag.
+ * enqueued on `stream`; ctprj_tv_denoise synchronises it.  Images of up to about
+ * 1.2 million pixels take one cooperative launch, which starts once all its
+ * blocks have room on the GPU, and one synchronisation at its end.  Its blocks
+ * meet once per iteration and wait for one another for at most two seconds;
+ * where a meeting fails, or the device has no room for all blocks at once, the
+ * call goes on as for larger images: a launch per iteration, and a
+ * synchronisation every eight to read the stopping flag.
  */
 #ifndef CTPRJ_TV_H
 #define CTPRJ_TV_H

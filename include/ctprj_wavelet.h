@@ -55,7 +55,11 @@ int ctprj_wvlt_l1(const float *d_x, int rows, int cols, const double *h, int lh,
  * units of a / ||a||, or more than max_itr iterations) and rho adaptation.
  * d_init may be NULL (init = a).  d_alpha (rows*cols floats) may not alias
  * d_a or d_init.  *iterations (may be NULL) receives iter.  Synchronises
- * `stream` once at the start and every eight iterations. */
+ * `stream`: with a 2-tap filter, 2 to 6 levels and an image in whole 64 x 64
+ * tiles that the GPU holds at once, the loop is one cooperative launch as
+ * ctprj_tv_denoise's (ctprj_tv.h), with one synchronisation at its end;
+ * otherwise, and where that launch's blocks do not meet, once at the start and
+ * every eight iterations. */
 int ctprj_wvlt_admm(const float *d_a, int rows, int cols, const double *h, int lh, int levels, double u,
                     double rel_tol, int max_itr, const float *d_init, float *d_alpha, int *iterations,
                     void *stream);
