@@ -1013,12 +1013,15 @@ int WvltProx::alloc(int m, int n, cudaStream_t s)
 int WvltProx::reserve_parts(size_t need, cudaStream_t s)
 {
     if (part_cap >= need) return CTPRJ_OK;
+    // (the smaller buffer stays until there is another: the workspace is used again
+    // after a call that found no memory)
+    double *larger = nullptr;
+    const int st = cuda_error(cudaMallocAsync((void **)&larger, sizeof(double) * need, s), "wavelet partials");
+    if (st) return st;
     if (part) cudaFreeAsync(part, s);
-    part = nullptr;
-    part_cap = 0;
-    const int st = cuda_error(cudaMallocAsync((void **)&part, sizeof(double) * need, s), "wavelet partials");
-    if (!st) part_cap = need;
-    return st;
+    part = larger;
+    part_cap = need;
+    return CTPRJ_OK;
 }
 
 void WvltProx::release(cudaStream_t s)
