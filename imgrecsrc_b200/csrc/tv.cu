@@ -355,11 +355,12 @@ __global__ void k_tv_start(TvState *st, int done)
 // ---- images that fit the GPU's registers and shared memory: one launch ----
 // Up to about 1.2 million pixels every tile of the image has a block of its own
 // on the GPU, so the whole iteration loop is one cooperative launch: a thread
-// keeps the dual P of its eight pixels in registers (and P_prev, or in shared
-// memory), the tile's Xobs and D stay in shared memory, and per iteration a block reads only its halo of
-// P and writes the edge of its new P.  The blocks meet once per iteration, at the
-// sums of the stopping rule (grid_sums.cuh), after which every block advances its
-// own copy of the scalars: no host check, no second launch.  What bounds an
+// keeps the dual P of its eight pixels in registers (P_prev, too, or in shared
+// memory), the tile's Xobs and D stay in shared memory, and per iteration a block
+// reads only its halo of P and writes the edge of its new P.  The blocks meet once
+// per iteration, at the sums of the stopping rule (grid_sums.cuh), after which every
+// warp advances its own copy of the scalars: no host check, no second launch.
+// What bounds an
 // iteration is a chain of latencies, of which the meeting (fence, count, partials
 // and halo from L2) is half; so a thread takes eight rows of one column, whose
 // neighbours above and below are mostly its own, reads shared memory four pixels
